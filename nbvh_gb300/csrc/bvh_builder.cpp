@@ -525,6 +525,52 @@ bool nodes_in_fast_div_domain(const std::vector<BVHNode> &nodes)
     return true;
 }
 
+// Boxes whose coordinates are +0 or of magnitude in [2^-40, 2^10]: they are multiples of 2^-63, so a
+// corner dilated by a factor up to 2 is a multiple of 2^-87 (extent, its half and its dilated half
+// round to at least that granule) and its difference to an origin in the fast-division domain is +0
+// or at least 2^-87 in magnitude: Markstein's division stays exact (the remainder's lowest bit, 2^-135,
+// is representable), and no dilated corner is -0.
+bool nodes_in_train_div_domain(const std::vector<BVHNode> &nodes)
+{
+    for (const BVHNode &n : nodes)
+        for (int k = 0; k < 6; k++) {
+            const float c = k < 3 ? n.min[k] : n.max[k - 3];
+            uint32_t bits;
+            std::memcpy(&bits, &c, 4);
+            const float a = std::fabs(c);
+            if (bits != 0u && !(a >= 0x1p-40f && a <= 0x1p10f))
+                return false;
+        }
+    return true;
+}
+
+// Whether every LoD has the same leaves (no leaf has children) and no leaf lies deeper than
+// max_depth; the largest leaf extent and coordinate magnitude.
+bool cut_allows_train_cull(const std::vector<BVHNode> &neural, uint32_t max_depth, float &leaf_extent,
+                           float &max_coord)
+{
+    leaf_extent = 0.f;
+    max_coord = 0.f;
+    std::vector<uint32_t> depth(neural.size(), 0u);
+    bool ok = true;
+    for (size_t i = 0; i < neural.size(); i++) { // children are allocated after their parent
+        const BVHNode &n = neural[i];
+        for (int k = 0; k < 3; k++)
+            max_coord = std::max(max_coord, std::max(std::fabs(n.min[k]), std::fabs(n.max[k])));
+        if (n.left_or_prim_offset == kNoNeuralChild) {
+            for (int k = 0; k < 3; k++)
+                leaf_extent = std::max(leaf_extent, n.max[k] - n.min[k]);
+            ok = ok && depth[i] <= max_depth;
+        } else {
+            ok = ok && n.prim_count == 0u && n.left_or_prim_offset > i && n.left_or_prim_offset + 1u < neural.size();
+            if (!ok)
+                return false;
+            depth[n.left_or_prim_offset] = depth[n.left_or_prim_offset + 1u] = depth[i] + 1u;
+        }
+    }
+    return ok;
+}
+
 // Inference copy of the neural cut: every node box dilated once by `dil` with the FP32 operations
 // of intersect_primitive_min_max / intersect_traversal_bbox (include/cuda/neural/accel/
 // neural_bvh2.cuh:80-86, 101-107; centre = min + extent * 0.5, extent * (1 + dil)), and per node the

@@ -187,34 +187,35 @@ __device__ __forceinline__ V3 div3r(V3 a, const RayDiv &r)
     return div3(a, r.d);
 }
 
-// BVH2Node::intersect, include/base/accel/bvh.h:121-133
-__device__ __forceinline__ float box_entry(V3 bmin, V3 bmax, V3 o, V3 d, float rmint, float rmaxt)
+// Entry and exit of the slabs of one box for a ray inside the fast-division domain (RayDiv::fast):
+// the quotients are finite, so hardware minima and maxima (three-input ones on this architecture)
+// give the values of the glm selects, up to the sign of a zero. Traversals choose between this form
+// and the general one once per ray instead of once per division. They are bound by instruction issue
+// at 10-14 active lanes of 32: 36 instructions fewer per node visit took the classic query from 1,056
+// to 927-960 us and the neural query (with neural_intersect_impl's order of work) from 3,233 to 3,068 us
+// per 2^22 uniform rays on GB300.
+__device__ __forceinline__ float hw_max3(float a, float b, float c)
 {
-    V3 t0 = div3(sub3(bmin, o), d);
-    V3 t1 = div3(sub3(bmax, o), d);
-    float mint = gmax(rmint, cmax3(min3(t0, t1)));
-    float maxt = gmin(rmaxt, cmin3(max3(t0, t1)));
-    return (mint <= maxt) ? mint : FLT_MAX;
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
-
-// BVH2Node::intersect with the prepared-ray division (bit-identical quotients)
-__device__ __forceinline__ float box_entry(V3 bmin, V3 bmax, V3 o, const RayDiv &rd, float rmint, float rmaxt)
+__device__ __forceinline__ float hw_min3(float a, float b, float c)
 {
-    V3 t0 = div3r(sub3(bmin, o), rd);
-    V3 t1 = div3r(sub3(bmax, o), rd);
-    float mint = gmax(rmint, cmax3(min3(t0, t1)));
-    float maxt = gmin(rmaxt, cmin3(max3(t0, t1)));
-    return (mint <= maxt) ? mint : FLT_MAX;
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
-
-// Ray3f::intersect_bbox_min_max without ray bounds, include/cuda/base/ray.cuh:111-132
-__device__ __forceinline__ bool slab_min_max(V3 bmin, V3 bmax, V3 o, V3 d, float &mint, float &maxt)
+__device__ __forceinline__ void slab_fast(V3 bmin, V3 bmax, V3 o, const RayDiv &r, float &entry, float &exit_)
 {
-    V3 t0 = div3(sub3(bmin, o), d);
-    V3 t1 = div3(sub3(bmax, o), d);
-    mint = cmax3(min3(t0, t1));
-    maxt = cmin3(max3(t0, t1));
-    return mint <= maxt;
+    const float ax = markstein_div(__fsub_rn(bmin.x, o.x), r.d.x, r.inv.x);
+    const float bx = markstein_div(__fsub_rn(bmax.x, o.x), r.d.x, r.inv.x);
+    const float ay = markstein_div(__fsub_rn(bmin.y, o.y), r.d.y, r.inv.y);
+    const float by = markstein_div(__fsub_rn(bmax.y, o.y), r.d.y, r.inv.y);
+    const float az = markstein_div(__fsub_rn(bmin.z, o.z), r.d.z, r.inv.z);
+    const float bz = markstein_div(__fsub_rn(bmax.z, o.z), r.d.z, r.inv.z);
+    entry = hw_max3(fminf(ax, bx), fminf(ay, by), fminf(az, bz));
+    exit_ = hw_min3(fmaxf(ax, bx), fmaxf(ay, by), fmaxf(az, bz));
 }
 
 // dilated neural node box: BVH2Node::bbox_center (min + extent * 0.5) and
@@ -260,19 +261,47 @@ __device__ __forceinline__ bool tri_intersect(V3 v0, V3 e1, V3 e2, V3 o, V3 d, f
     return true;
 }
 
-// CudaBVH2::intersect<ShadowRay>, include/cuda/accel/bvh2.cuh:12-88: root-first DFS, nearer child
-// first (swap when child1_mint > child2_mint), ray.maxt shrinks on every accepted hit.
-template <bool ANY_HIT>
-__device__ __forceinline__ void classic_traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, V3 o,
-                                                 V3 d, float rmint, float rmaxt, float &best_t, float &best_u,
-                                                 float &best_v, uint32_t &best_prim, uint32_t *best_rec = nullptr,
-                                                 bool scene_fast_div = false)
+// Raw slab of a box: entry = max_i min(t0_i, t1_i), exit = min_i max(t0_i, t1_i) with the
+// glm operation order of Ray3f::intersect_bbox_min_max (include/cuda/base/ray.cuh:111-132).
+__device__ __forceinline__ void slab_raw(V3 bmin, V3 bmax, V3 o, const RayDiv &rd, float &entry, float &exit_)
 {
-    best_t = FLT_MAX;
-    best_u = 0.f;
-    best_v = 0.f;
-    best_prim = 0xFFFFFFFFu;
-    const RayDiv rd = make_raydiv(o, d, scene_fast_div);
+    V3 t0 = div3r(sub3(bmin, o), rd);
+    V3 t1 = div3r(sub3(bmax, o), rd);
+    entry = cmax3(min3(t0, t1));
+    exit_ = cmin3(max3(t0, t1));
+}
+
+template <bool FAST>
+__device__ __forceinline__ void slab_any(V3 bmin, V3 bmax, V3 o, const RayDiv &rd, float &entry, float &exit_)
+{
+    if constexpr (FAST)
+        slab_fast(bmin, bmax, o, rd, entry, exit_);
+    else
+        slab_raw(bmin, bmax, o, rd, entry, exit_);
+}
+
+// BVH2Node::intersect, include/base/accel/bvh.h:121-133: where the ray enters the box within
+// [rmint, rmaxt], FLT_MAX if it does not. FAST: the fast-division domain and bounds that are not NaN.
+template <bool FAST>
+__device__ __forceinline__ float box_entry(V3 bmin, V3 bmax, V3 o, const RayDiv &rd, float rmint, float rmaxt)
+{
+    float e, x;
+    slab_any<FAST>(bmin, bmax, o, rd, e, x);
+    const float mint = FAST ? fmaxf(rmint, e) : gmax(rmint, e);
+    const float maxt = FAST ? fminf(rmaxt, x) : gmin(rmaxt, x);
+    return mint <= maxt ? mint : FLT_MAX;
+}
+
+// CudaBVH2::intersect<ShadowRay>, include/cuda/accel/bvh2.cuh:12-88: root-first DFS, nearer child
+// first (swap when child1_mint > child2_mint), ray.maxt shrinks on every accepted hit. The two pops
+// stay in their branches: one shared pop after them took 1,245 us where this form takes 960 (2^22
+// uniform rays), and an if / else over the nearer child instead of the swap 985.
+template <bool ANY_HIT, bool FAST>
+__device__ __forceinline__ void classic_traverse_impl(const float4 *__restrict__ nodes,
+                                                      const float4 *__restrict__ tris, V3 o, const RayDiv &rd,
+                                                      float rmint, float rmaxt, float &best_t, float &best_u,
+                                                      float &best_v, uint32_t &best_prim, uint32_t &best_rec)
+{
     uint32_t stack[32];
     int sp = 0;
     NodeBox node = load_node(nodes, 0);
@@ -284,15 +313,14 @@ __device__ __forceinline__ void classic_traverse(const float4 *__restrict__ node
                 float4 r1 = __ldg(tris + 3u * pid + 1u);
                 float4 r2 = __ldg(tris + 3u * pid + 2u);
                 float t, u, v;
-                if (tri_intersect(mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), mk3(r2.x, r2.y, r2.z), o, d, rmint,
+                if (tri_intersect(mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), mk3(r2.x, r2.y, r2.z), o, rd.d, rmint,
                                   rmaxt, t, u, v) &&
                     t < rmaxt) {
                     best_t = t;
                     best_u = u;
                     best_v = v;
                     best_prim = __float_as_uint(r0.w);
-                    if (best_rec)
-                        *best_rec = pid;
+                    best_rec = pid;
                     if (ANY_HIT) {
                         done = true;
                         break;
@@ -309,8 +337,8 @@ __device__ __forceinline__ void classic_traverse(const float4 *__restrict__ node
         // both children are adjacent: four 128-bit loads
         NodeBox n1 = load_node(nodes, c1);
         NodeBox n2 = load_node(nodes, c2);
-        float d1 = box_entry(n1.mn, n1.mx, o, rd, rmint, rmaxt);
-        float d2 = box_entry(n2.mn, n2.mx, o, rd, rmint, rmaxt);
+        float d1 = box_entry<FAST>(n1.mn, n1.mx, o, rd, rmint, rmaxt);
+        float d2 = box_entry<FAST>(n2.mn, n2.mx, o, rd, rmint, rmaxt);
         if (d1 > d2) {
             float td = d1;
             d1 = d2;
@@ -334,98 +362,24 @@ __device__ __forceinline__ void classic_traverse(const float4 *__restrict__ node
     }
 }
 
-// NeuralBVH2::intersect, include/cuda/neural/accel/neural_bvh2.cuh:170-292. Pops the next node
-// from `stack` and returns 1 with the next entered leaf segment, 0 when the stack runs empty,
-// -1 on a stack overflow (the reference prints and returns false), 2 when `budget` node visits
-// ran out first (call again to continue).
-template <typename Stack>
-__device__ __forceinline__ int neural_intersect(const float4 *__restrict__ nodes, uint32_t lod, V3 o, V3 d, Stack &stack,
-                                                int &sp, bool inference, float mint_eps_inf, float maxt_eps_inf,
-                                                float mint_eps_learn, float maxt_eps_learn, float current_maxt,
-                                                float dil, float &seg_mint, float &seg_maxt, uint32_t &seg_node,
-                                                int budget = 0x7FFFFFFF)
+template <bool ANY_HIT>
+__device__ __forceinline__ void classic_traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, V3 o,
+                                                 V3 d, float rmint, float rmaxt, float &best_t, float &best_u,
+                                                 float &best_v, uint32_t &best_prim, uint32_t *best_rec = nullptr,
+                                                 bool scene_fast_div = false)
 {
-    const float rmint = -FLT_MAX, rmaxt = current_maxt;
-    uint32_t node_idx = stack[--sp];
-    for (;; budget--) {
-        if (budget <= 0) {
-            // out of node visits: the current node goes back on the stack and the call reports "not
-            // finished" (2); the next call resumes exactly here (sp <= 23: a push to 24 returned -1)
-            stack[sp++] = node_idx;
-            return 2;
-        }
-        NodeBox node = load_node(nodes, node_idx);
-        if ((node.count > 0u && node.count <= 2u + lod) || node.offset == 0xFFFFFFFFu) {
-            V3 bmin, bmax;
-            float mint, maxt;
-            dilated_box(node, dil, bmin, bmax);
-            if (slab_min_max(bmin, bmax, o, d, mint, maxt)) {
-                float maxt_eps = inference ? maxt_eps_inf : maxt_eps_learn;
-                float mint_eps = inference ? mint_eps_inf : mint_eps_learn;
-                bool valid = mint < rmaxt;
-                if (mint < 0.0f)
-                    valid &= maxt > maxt_eps;
-                else
-                    valid &= mint > mint_eps;
-                if (valid) {
-                    seg_mint = mint;
-                    seg_maxt = maxt;
-                    seg_node = node_idx;
-                    return 1;
-                }
-            }
-            if (sp == 0)
-                return 0;
-            node_idx = stack[--sp];
-            continue;
-        }
-        uint32_t c1 = node.offset, c2 = node.offset + 1u;
-        NodeBox n1 = load_node(nodes, c1);
-        NodeBox n2 = load_node(nodes, c2);
-        V3 b1min, b1max, b2min, b2max;
-        dilated_box(n1, dil, b1min, b1max);
-        dilated_box(n2, dil, b2min, b2max);
-        float d1 = box_entry(b1min, b1max, o, d, rmint, rmaxt);
-        float d2 = box_entry(b2min, b2max, o, d, rmint, rmaxt);
-        if (d1 > d2) {
-            float td = d1;
-            d1 = d2;
-            d2 = td;
-            uint32_t tc = c1;
-            c1 = c2;
-            c2 = tc;
-        }
-        if (d1 == FLT_MAX) {
-            if (sp == 0)
-                return 0;
-            node_idx = stack[--sp];
-        } else {
-            node_idx = c1;
-            if (d2 != FLT_MAX) {
-                stack[sp++] = c2;
-                if (sp >= 24)
-                    return -1;
-            }
-        }
-    }
-}
-
-// Raw slab of a box: entry = max_i min(t0_i, t1_i), exit = min_i max(t0_i, t1_i) with the
-// glm operation order of Ray3f::intersect_bbox_min_max (include/cuda/base/ray.cuh:111-132).
-__device__ __forceinline__ void slab_raw(V3 bmin, V3 bmax, V3 o, V3 d, float &entry, float &exit_)
-{
-    V3 t0 = div3(sub3(bmin, o), d);
-    V3 t1 = div3(sub3(bmax, o), d);
-    entry = cmax3(min3(t0, t1));
-    exit_ = cmin3(max3(t0, t1));
-}
-
-__device__ __forceinline__ void slab_raw(V3 bmin, V3 bmax, V3 o, const RayDiv &rd, float &entry, float &exit_)
-{
-    V3 t0 = div3r(sub3(bmin, o), rd);
-    V3 t1 = div3r(sub3(bmax, o), rd);
-    entry = cmax3(min3(t0, t1));
-    exit_ = cmin3(max3(t0, t1));
+    best_t = FLT_MAX;
+    best_u = 0.f;
+    best_v = 0.f;
+    best_prim = 0xFFFFFFFFu;
+    uint32_t rec = 0;
+    const RayDiv rd = make_raydiv(o, d, scene_fast_div);
+    if (rd.fast && rmint == rmint && rmaxt == rmaxt)
+        classic_traverse_impl<ANY_HIT, true>(nodes, tris, o, rd, rmint, rmaxt, best_t, best_u, best_v, best_prim, rec);
+    else
+        classic_traverse_impl<ANY_HIT, false>(nodes, tris, o, rd, rmint, rmaxt, best_t, best_u, best_v, best_prim, rec);
+    if (best_rec)
+        *best_rec = rec;
 }
 
 // Leaf acceptance of NeuralBVH2::intersect (neural_bvh2.cuh:199-215) from the raw slab.
@@ -441,10 +395,152 @@ __device__ __forceinline__ bool leaf_accepts(float entry, float exit_, float rma
     return valid;
 }
 
+// NeuralBVH2::intersect of the training rays (include/cuda/neural/accel/neural_bvh2.cuh:170-292), every
+// box dilated by the sample's own `dil` as it is met. Pops the next node from `stack` and returns 1
+// with the next entered leaf segment, 0 when the stack runs empty, -1 on a stack overflow (the
+// reference prints and returns false), 2 when `budget` node visits ran out first (call again to
+// continue).
+//
+// `bounds` (may be NULL) skips subtrees that lie behind the origin: two float4 per node, the union
+// of the leaf boxes below it, grown by `grow` on every side so that it contains those boxes at any
+// dilation the sampler draws, rounding included. The quotients of the slab test are monotone in the
+// box bounds, so no leaf below such a node exits later than the grown union, and every accepted leaf
+// exits after min(mint_eps, maxt_eps). Leaves that are not accepted are then not pushed either. Both
+// leave out only nodes that yield nothing, so segments and their order stay; they are for cuts
+// whose stack cannot overflow, so that no overflow is skipped with them.
+struct TrainCut {
+    const float4 *nodes;
+    const float4 *bounds;
+    float grow;
+};
+
+// Measured per 2^18 samples: the search of a training step 533 -> 212 us with the fast division, the
+// culling and neural_intersect_impl's order of work.
+template <bool FAST, typename Stack>
+__device__ __forceinline__ int neural_intersect_train_impl(const TrainCut &cut, uint32_t lod, V3 o, const RayDiv &d,
+                                                           bool cull_ok, Stack &stack, int &sp, float mint_eps,
+                                                           float maxt_eps, float dil, float &seg_mint, float &seg_maxt,
+                                                           uint32_t &seg_node, int budget)
+{
+    const float cull_eps = gmin(mint_eps, maxt_eps);
+    const bool cull = cut.bounds != nullptr;
+    auto is_leaf = [lod](const NodeBox &n) {
+        return (n.count > 0u && n.count <= 2u + lod) || n.offset == 0xFFFFFFFFu;
+    };
+    auto slab = [&](const NodeBox &n, float &e, float &x) {
+        V3 bmin, bmax;
+        dilated_box(n, dil, bmin, bmax);
+        slab_any<FAST>(bmin, bmax, o, d, e, x);
+    };
+    // the segment of an accepted leaf; a zero end of a fast slab is recomputed for its sign
+    auto accept = [&](uint32_t i, float e, float x) {
+        if (FAST && (e == 0.0f || x == 0.0f)) {
+            V3 bmin, bmax;
+            dilated_box(load_node(cut.nodes, i), dil, bmin, bmax);
+            slab_raw(bmin, bmax, o, d, e, x);
+        }
+        seg_mint = e;
+        seg_maxt = x;
+        seg_node = i;
+    };
+    uint32_t idx = stack[--sp];
+    NodeBox node = load_node(cut.nodes, idx);
+    for (;; budget--) {
+        if (budget <= 0) {
+            // out of node visits: the current node goes back on the stack and the call reports "not
+            // finished" (2); the next call resumes exactly here (sp <= 23: a push to 24 returned -1)
+            stack[sp++] = idx;
+            return 2;
+        }
+        if (is_leaf(node)) {
+            float e, x;
+            slab(node, e, x);
+            if (leaf_accepts(e, x, FLT_MAX, mint_eps, maxt_eps)) {
+                accept(idx, e, x);
+                return 1;
+            }
+            if (sp == 0)
+                return 0;
+            idx = stack[--sp];
+            node = load_node(cut.nodes, idx);
+            continue;
+        }
+        const uint32_t c1 = node.offset, c2 = node.offset + 1u;
+        const NodeBox n1 = load_node(cut.nodes, c1);
+        const NodeBox n2 = load_node(cut.nodes, c2);
+        float e1, x1, e2, x2;
+        slab(n1, e1, x1);
+        slab(n2, e2, x2);
+        const float m1 = FAST ? e1 : gmax(-FLT_MAX, e1), m2 = FAST ? e2 : gmax(-FLT_MAX, e2);
+        const float d1 = (m1 <= (FAST ? x1 : gmin(FLT_MAX, x1))) ? m1 : FLT_MAX;
+        const float d2 = (m2 <= (FAST ? x2 : gmin(FLT_MAX, x2))) ? m2 : FLT_MAX;
+        auto alive = [&](float dd, const NodeBox &nb, uint32_t ci, float e, float x) -> bool {
+            if (dd == FLT_MAX)
+                return false;
+            if (!cull)
+                return true;
+            if (is_leaf(nb))
+                return leaf_accepts(e, x, FLT_MAX, mint_eps, maxt_eps);
+            if (cull_ok && x <= cull_eps) {
+                const float4 lo = __ldg(cut.bounds + 2u * ci), hi = __ldg(cut.bounds + 2u * ci + 1u);
+                float ue, ux;
+                slab_any<FAST>(adds3(mk3(lo.x, lo.y, lo.z), -cut.grow), adds3(mk3(hi.x, hi.y, hi.z), cut.grow), o, d,
+                               ue, ux);
+                return !(ux <= cull_eps);
+            }
+            return true;
+        };
+        const bool a1 = alive(d1, n1, c1, e1, x1);
+        const bool a2 = alive(d2, n2, c2, e2, x2);
+        if (a2 && (!a1 || d1 > d2)) {
+            idx = c2;
+            if (a1) {
+                stack[sp++] = c1;
+                if (sp >= 24)
+                    return -1;
+            }
+            if (cull && is_leaf(n2)) {
+                accept(idx, e2, x2);
+                return 1;
+            }
+            node = n2;
+        } else if (a1) {
+            idx = c1;
+            if (a2) {
+                stack[sp++] = c2;
+                if (sp >= 24)
+                    return -1;
+            }
+            if (cull && is_leaf(n1)) {
+                accept(idx, e1, x1);
+                return 1;
+            }
+            node = n1;
+        } else {
+            if (sp == 0)
+                return 0;
+            idx = stack[--sp];
+            node = load_node(cut.nodes, idx);
+        }
+    }
+}
+
+template <typename Stack>
+__device__ __forceinline__ int neural_intersect_train(const TrainCut &cut, uint32_t lod, V3 o, const RayDiv &d,
+                                                      bool cull_ok, Stack &stack, int &sp, float mint_eps,
+                                                      float maxt_eps, float dil, float &seg_mint, float &seg_maxt,
+                                                      uint32_t &seg_node, int budget = 0x7FFFFFFF)
+{
+    return d.fast ? neural_intersect_train_impl<true>(cut, lod, o, d, cull_ok, stack, sp, mint_eps, maxt_eps, dil,
+                                                      seg_mint, seg_maxt, seg_node, budget)
+                  : neural_intersect_train_impl<false>(cut, lod, o, d, cull_ok, stack, sp, mint_eps, maxt_eps, dil,
+                                                       seg_mint, seg_maxt, seg_node, budget);
+}
+
 // NeuralBVH2::intersect for inference on a pre-dilated copy of the cut (`nodes` boxes already
 // dilated by fixed_node_dilation with the reference's operations). Returns the same accepted leaf
 // segments in the same order as the reference; it differs only in work skipped:
-//  * the slab of the child it descends into is carried over instead of recomputed;
+//  * a leaf it descends into is accepted with the slab computed as a child;
 //  * a child is not pushed / entered when nothing below it can be accepted: a leaf that fails the
 //    acceptance test now (the bound rmaxt only shrinks later), or an interior node whose union of
 //    dilated leaf boxes (`bounds`) lies entirely at t <= min(mint_eps, maxt_eps), beyond rmaxt, or
@@ -489,6 +585,114 @@ struct SharedCut {
     }
 };
 
+// A leaf chosen among the children is returned at once (it was tested just now), one popped later
+// is tested again; the two children are not swapped but taken in an if / else: 3,068 us per 2^22-ray
+// query, against 3,130 with the swap and 3,150 with one shared pop after the branches.
+template <bool FAST, typename Src, typename Stack>
+__device__ __forceinline__ int neural_intersect_impl(const Src &src, uint32_t lod, V3 o, const RayDiv &d, bool cull_ok,
+                                                     Stack &stack, int &sp, float mint_eps, float maxt_eps,
+                                                     float rmaxt, float &seg_mint, float &seg_maxt,
+                                                     uint32_t &seg_node, int budget)
+{
+    const float cull_eps = gmin(mint_eps, maxt_eps);
+    auto is_leaf = [lod](const NodeBox &n) {
+        return (n.count > 0u && n.count <= 2u + lod) || n.offset == 0xFFFFFFFFu;
+    };
+    // the segment of an accepted leaf; a zero end of a fast slab is recomputed for its sign
+    auto accept = [&](uint32_t idx, float e, float x) {
+        if (FAST && (e == 0.0f || x == 0.0f)) {
+            const NodeBox n = src.node(idx);
+            slab_raw(n.mn, n.mx, o, d, e, x);
+        }
+        seg_mint = e;
+        seg_maxt = x;
+        seg_node = idx;
+    };
+    uint32_t idx = stack[--sp];
+    NodeBox node = src.node(idx);
+    for (;; budget--) {
+        if (budget <= 0) {
+            // out of node visits: put the current node back and report "not finished" (2); the next
+            // call pops it, so the traversal resumes exactly where it stopped. sp <= 23 here (a push
+            // that reached 24 returned -1), so the push fits.
+            stack[sp++] = idx;
+            return 2;
+        }
+        if (is_leaf(node)) { // popped: the bound may have shrunk since it was pushed
+            float e, x;
+            slab_any<FAST>(node.mn, node.mx, o, d, e, x);
+            if (leaf_accepts(e, x, rmaxt, mint_eps, maxt_eps)) {
+                accept(idx, e, x);
+                return 1;
+            }
+            if (sp == 0)
+                return 0;
+            idx = stack[--sp];
+            node = src.node(idx);
+            continue;
+        }
+        const uint32_t c1 = node.offset, c2 = node.offset + 1u;
+        const NodeBox n1 = src.node(c1);
+        const NodeBox n2 = src.node(c2);
+        float e1, x1, e2, x2;
+        slab_any<FAST>(n1.mn, n1.mx, o, d, e1, x1);
+        slab_any<FAST>(n2.mn, n2.mx, o, d, e2, x2);
+        const float m1 = FAST ? e1 : gmax(-FLT_MAX, e1), m2 = FAST ? e2 : gmax(-FLT_MAX, e2);
+        // intersect_traversal_bbox with check_ray_bounds (neural_bvh2.cuh:94-115), no hit = FLT_MAX
+        const float d1 = (FAST ? (m1 <= x1 && m1 <= rmaxt) : m1 <= gmin(rmaxt, x1)) ? m1 : FLT_MAX;
+        const float d2 = (FAST ? (m2 <= x2 && m2 <= rmaxt) : m2 <= gmin(rmaxt, x2)) ? m2 : FLT_MAX;
+        const bool l1 = is_leaf(n1), l2 = is_leaf(n2);
+        auto alive = [&](float dd, bool leaf, uint32_t ci, float e, float x) -> bool {
+            if (dd == FLT_MAX)
+                return false;
+            if (leaf)
+                return leaf_accepts(e, x, rmaxt, mint_eps, maxt_eps);
+            if (cull_ok && x <= cull_eps) {
+                V3 umn, umx;
+                src.bound(ci, umn, umx);
+                float ue, ux;
+                slab_any<FAST>(umn, umx, o, d, ue, ux);
+                if (!(ue <= ux) || ux <= cull_eps || ue >= rmaxt)
+                    return false;
+            }
+            return true;
+        };
+        const bool a1 = alive(d1, l1, c1, e1, x1);
+        const bool a2 = alive(d2, l2, c2, e2, x2);
+        const bool second = a2 && (!a1 || d1 > d2);
+        if (second) {
+            idx = c2;
+            if (a1) {
+                stack[sp++] = c1;
+                if (sp >= 24)
+                    return -1;
+            }
+            if (l2) {
+                accept(idx, e2, x2);
+                return 1;
+            }
+            node = n2;
+        } else if (a1) {
+            idx = c1;
+            if (a2) {
+                stack[sp++] = c2;
+                if (sp >= 24)
+                    return -1;
+            }
+            if (l1) {
+                accept(idx, e1, x1);
+                return 1;
+            }
+            node = n1;
+        } else {
+            if (sp == 0)
+                return 0;
+            idx = stack[--sp];
+            node = src.node(idx);
+        }
+    }
+}
+
 template <typename Src, typename Stack>
 __device__ __forceinline__ int neural_intersect_inference(const Src &src, uint32_t lod, V3 o, const RayDiv &d,
                                                           bool cull_ok, Stack &stack, int &sp, float mint_eps,
@@ -496,107 +700,10 @@ __device__ __forceinline__ int neural_intersect_inference(const Src &src, uint32
                                                           float &seg_maxt, uint32_t &seg_node,
                                                           int budget = 0x7FFFFFFF)
 {
-    const float rmint = -FLT_MAX, rmaxt = current_maxt;
-    const float cull_eps = gmin(mint_eps, maxt_eps);
-    uint32_t node_idx = stack[--sp];
-    NodeBox node = src.node(node_idx);
-    bool have_slab = false;
-    float cur_e = 0.f, cur_x = 0.f;
-    for (;; budget--) {
-        if (budget <= 0) {
-            // out of node visits: put the current node back and report "not finished" (2); the next
-            // call pops it and recomputes its slab, so the traversal resumes exactly where it
-            // stopped. sp <= 23 here (a push that reached 24 returned -1), so the push fits.
-            stack[sp++] = node_idx;
-            return 2;
-        }
-        const bool leaf = (node.count > 0u && node.count <= 2u + lod) || node.offset == 0xFFFFFFFFu;
-        if (leaf) {
-            if (!have_slab)
-                slab_raw(node.mn, node.mx, o, d, cur_e, cur_x);
-            if (leaf_accepts(cur_e, cur_x, rmaxt, mint_eps, maxt_eps)) {
-                seg_mint = cur_e;
-                seg_maxt = cur_x;
-                seg_node = node_idx;
-                return 1;
-            }
-            if (sp == 0)
-                return 0;
-            node_idx = stack[--sp];
-            node = src.node(node_idx);
-            have_slab = false;
-            continue;
-        }
-        uint32_t c1 = node.offset, c2 = node.offset + 1u;
-        NodeBox n1 = src.node(c1);
-        NodeBox n2 = src.node(c2);
-        float e1, x1, e2, x2;
-        slab_raw(n1.mn, n1.mx, o, d, e1, x1);
-        slab_raw(n2.mn, n2.mx, o, d, e2, x2);
-        // intersect_traversal_bbox with check_ray_bounds (neural_bvh2.cuh:94-115)
-        float m1 = gmax(rmint, e1), m2 = gmax(rmint, e2);
-        float d1 = (m1 <= gmin(rmaxt, x1)) ? m1 : FLT_MAX;
-        float d2 = (m2 <= gmin(rmaxt, x2)) ? m2 : FLT_MAX;
-        if (d1 > d2) {
-            float t = d1;
-            d1 = d2;
-            d2 = t;
-            uint32_t tc = c1;
-            c1 = c2;
-            c2 = tc;
-            NodeBox tn = n1;
-            n1 = n2;
-            n2 = tn;
-            t = e1;
-            e1 = e2;
-            e2 = t;
-            t = x1;
-            x1 = x2;
-            x2 = t;
-        }
-        auto alive = [&](const NodeBox &nb, uint32_t ci, float e, float x, float dd) -> bool {
-            if (dd == FLT_MAX)
-                return false;
-            const bool cleaf = (nb.count > 0u && nb.count <= 2u + lod) || nb.offset == 0xFFFFFFFFu;
-            if (cleaf)
-                return leaf_accepts(e, x, rmaxt, mint_eps, maxt_eps);
-            if (cull_ok && x <= cull_eps) {
-                V3 umn, umx;
-                src.bound(ci, umn, umx);
-                float ue, ux;
-                slab_raw(umn, umx, o, d, ue, ux);
-                if (!(ue <= ux) || ux <= cull_eps || ue >= rmaxt)
-                    return false;
-            }
-            return true;
-        };
-        const bool a1 = alive(n1, c1, e1, x1, d1);
-        const bool a2 = alive(n2, c2, e2, x2, d2);
-        if (a1) {
-            node_idx = c1;
-            node = n1;
-            cur_e = e1;
-            cur_x = x1;
-            have_slab = true;
-            if (a2) {
-                stack[sp++] = c2;
-                if (sp >= 24)
-                    return -1;
-            }
-        } else if (a2) {
-            node_idx = c2;
-            node = n2;
-            cur_e = e2;
-            cur_x = x2;
-            have_slab = true;
-        } else {
-            if (sp == 0)
-                return 0;
-            node_idx = stack[--sp];
-            node = src.node(node_idx);
-            have_slab = false;
-        }
-    }
+    return d.fast ? neural_intersect_impl<true>(src, lod, o, d, cull_ok, stack, sp, mint_eps, maxt_eps, current_maxt,
+                                                seg_mint, seg_maxt, seg_node, budget)
+                  : neural_intersect_impl<false>(src, lod, o, d, cull_ok, stack, sp, mint_eps, maxt_eps, current_maxt,
+                                                 seg_mint, seg_maxt, seg_node, budget);
 }
 
 // Segment encoding into the hash-grid unit cube, src/cuda/neural/neural_bvh_module_kernels.cu:48-55

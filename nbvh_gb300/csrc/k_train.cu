@@ -34,6 +34,8 @@ struct SampleArgs {
     GridParams grid;
     NeuralConsts nc;
     const float4 *neural_nodes;
+    TrainCut cut;
+    uint32_t neural_fast_div; // neural coordinates in the fast-division domain at every dilation
     const float4 *nodes;
     const float4 *tris;
     const float *albedo;
@@ -90,7 +92,8 @@ __global__ void __launch_bounds__(kFindThreads, 4) k_training_find(const __grid_
     V3 o = mk3(0, 0, 0), dir = mk3(0, 0, 0);
     uint32_t stack[kNeuralStackSize];
     int sp = 0;
-    bool active = false, need_origin = false, exhausted = false;
+    RayDiv rdiv;
+    bool active = false, need_origin = false, exhausted = false, cull_ok = false;
     for (;;) {
         const unsigned idle = __ballot_sync(0xFFFFFFFFu, !active);
         if (idle != 0u && !exhausted) {
@@ -133,12 +136,13 @@ __global__ void __launch_bounds__(kFindThreads, 4) k_training_find(const __grid_
                 const float pz = lcg_randomf(rng);
                 V3 ps = sub3(scale3(mk3(px, py, pz), c.sampling_bbox_scaling), mk3(h, h, h));
                 o = add3(mul3(ps, sub3(smax, smin)), smin);
+                rdiv = make_raydiv(o, dir, a.neural_fast_div != 0u);
+                cull_ok = dir.x != 0.0f && dir.y != 0.0f && dir.z != 0.0f;
                 need_origin = false;
             }
-            const int res = neural_intersect(a.neural_nodes, sampled_lod, o, dir, stack, sp, false,
-                                             c.inference_mint_epsilon, c.inference_maxt_epsilon,
-                                             c.learning_mint_epsilon, c.learning_maxt_epsilon, FLT_MAX, dil, mint,
-                                             maxt, node, kFindVisits);
+            const int res = neural_intersect_train(a.cut, sampled_lod, o, rdiv, cull_ok, stack, sp,
+                                                   c.learning_mint_epsilon, c.learning_maxt_epsilon, dil, mint, maxt,
+                                                   node, kFindVisits);
             if (res != 2) {
                 if (res < 0)
                     sp = 0;
@@ -984,12 +988,14 @@ cudaError_t launch_training_samples(const float4 *neural_nodes, const float4 *no
                                     const float *albedo, const NeuralConsts &nc, const GridParams &grid,
                                     uint32_t training_step, uint32_t batch_size, uint32_t n, float *positions,
                                     float *targets, uint32_t *sample_nodes, uint32_t learned_lod,
-                                    const NodeSurvival *survival, float4 *state, bool classic_fast_div, int num_sms,
-                                    cudaStream_t s)
+                                    const NodeSurvival *survival, float4 *state, bool classic_fast_div,
+                                    const TrainCull &cull, int num_sms, cudaStream_t s)
 {
     if (n == 0)
         return cudaSuccess;
     SampleArgs a;
+    a.cut = TrainCut{neural_nodes, cull.bounds, cull.grow};
+    a.neural_fast_div = cull.fast_div ? 1u : 0u;
     a.grid = grid;
     a.nc = nc;
     a.neural_nodes = neural_nodes;

@@ -305,6 +305,7 @@ void upload_bvh(nbvh_handle *h)
     h->model_version++;
     // nodes: two float4 per node in the reference layout
     h->classic_fast_div = nodes_in_fast_div_domain(h->nodes);
+    h->classic_train_div = nodes_in_train_div_domain(h->nodes);
     cuda_check(h->d_nodes.resize(2u * h->nodes.size()), "alloc nodes");
     cuda_check(cudaMemcpy(h->d_nodes.ptr, h->nodes.data(), h->nodes.size() * sizeof(BVHNode), cudaMemcpyHostToDevice),
                "upload nodes");
@@ -361,6 +362,9 @@ void nbvh::upload_inference_nodes(nbvh_handle *h)
     std::vector<float> bounds;
     build_inference_nodes(h->neural_nodes, h->cfg.bvh.fixed_node_dilation, dilated, bounds);
     h->neural_fast_div = nodes_in_fast_div_domain(dilated) && coords_in_fast_div_domain(bounds.data(), bounds.size());
+    h->neural_train_div = nodes_in_train_div_domain(h->neural_nodes);
+    h->neural_train_cull =
+        cut_allows_train_cull(h->neural_nodes, kNeuralStackSize - 1u, h->neural_leaf_extent, h->neural_max_coord);
     cuda_check(h->d_neural_dilated.resize(2u * dilated.size()), "alloc dilated nodes");
     cuda_check(cudaMemcpy(h->d_neural_dilated.ptr, dilated.data(), dilated.size() * sizeof(BVHNode),
                           cudaMemcpyHostToDevice),
@@ -1402,6 +1406,24 @@ nbvh_status nbvh_encode(nbvh_handle *h, const float *d_positions, uint32_t n, fl
 
 namespace {
 
+// What the sampler's traversal may use (TrainCull). A tree-cut session splits the cut on the device
+// between steps: its nodes come from the classic BVH, and the host's subtree bounds do not follow.
+TrainCull train_cull(const nbvh_handle *h)
+{
+    const float fixed = h->cfg.bvh.fixed_node_dilation, extent = h->cfg.bvh.node_extent_dilation;
+    TrainCull c{nullptr, 0.f, false};
+    if (!(fixed >= 0.f && extent >= 0.f && fixed + extent <= 1.f))
+        return c;
+    c.fast_div = h->neural_train_div && (!h->cut.active || h->classic_train_div);
+    if (h->neural_train_cull && !h->cut.active && h->neural_train_div) {
+        c.bounds = h->d_neural_bounds.ptr;
+        // the leaves' extra dilation over the bounds' fixed one, and 32 units in the last place of the
+        // largest coordinate for the roundings of the dilated corners
+        c.grow = 0.501f * extent * h->neural_leaf_extent + 0x1p-18f * h->neural_max_coord;
+    }
+    return c;
+}
+
 // forward + loss + backward of one batch into h->d_grad (scaled by the loss scale) and loss_sum
 void gradients_into_workspace(nbvh_handle *h, const float *d_pos, const float *d_tgt, uint32_t n, cudaStream_t s,
                               float *loss_slot, const cudaEvent_t *marks = nullptr)
@@ -1473,7 +1495,7 @@ nbvh_status nbvh_generate_training_batch(nbvh_handle *h, uint32_t training_step,
         cuda_check(launch_training_samples(h->d_neural_nodes.ptr, h->d_nodes.ptr, h->d_tris.ptr,
                                            h->albedo.empty() ? nullptr : h->d_albedo.ptr, nc, h->grid, training_step,
                                            h->cfg.batch_size, n, d_positions, d_targets, d_nodes, kNumBvhLods - 1u,
-                                           nullptr, h->d_sample_state.ptr, h->classic_fast_div, h->num_sms,
+                                           nullptr, h->d_sample_state.ptr, h->classic_fast_div, train_cull(h), h->num_sms,
                                            reinterpret_cast<cudaStream_t>(stream)),
                    "training samples");
         h->last_launches = 2;
@@ -1509,7 +1531,7 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
                                                h->albedo.empty() ? nullptr : h->d_albedo.ptr, nc, h->grid,
                                                h->training_step, n, n, h->d_train_pos.ptr, h->d_train_tgt.ptr,
                                                h->d_train_nodes.ptr, learned_lod, &survival, h->d_sample_state.ptr,
-                                               h->classic_fast_div, h->num_sms, s),
+                                               h->classic_fast_div, train_cull(h), h->num_sms, s),
                        "training samples");
             gradients_into_workspace(h, h->d_train_pos.ptr, h->d_train_tgt.ptr, n, s, h->d_loss_sum.ptr + i,
                                      prof ? h->kprof->train_ev + 1 : nullptr);

@@ -336,6 +336,9 @@ struct nbvh_handle {
     bool any_non_neural = false;
     bool neural_fast_div = false;  // box coordinates of the cut inside the fast-division domain
     bool classic_fast_div = false; // same for the classic BVH
+    bool neural_train_div = false, classic_train_div = false; // coordinates that stay in the domain at any dilation up to 1
+    bool neural_train_cull = false; // one leaf set for all LoDs, depth below the stack size
+    float neural_leaf_extent = 0.f, neural_max_coord = 0.f; // over the cut's leaves / nodes
 
     // parameters
     nbvh_param_layout layout{};
@@ -628,6 +631,16 @@ struct NodeSurvival {
     uint32_t enabled;
 };
 
+// What the training traversal may take for granted about the cut: the fast division (every box
+// coordinate in its domain at every dilation the sampler draws), and for cuts that stay as they are,
+// with one leaf set for all LoDs and a depth that cannot overflow the stack, the subtree bounds and
+// the growth that makes them hold at every dilation (bounds NULL: no culling).
+struct TrainCull {
+    const float4 *bounds;
+    float grow;
+    bool fast_div;
+};
+
 // Training rays of one step: the leaf-segment search, then the labels (two kernels). state:
 // sample_state_float4s(n) float4 of device scratch.
 inline size_t sample_state_float4s(uint32_t n) { return (size_t)n * 3u + 1u; }
@@ -635,8 +648,8 @@ cudaError_t launch_training_samples(const float4 *neural_nodes, const float4 *no
                                     const float *albedo, const NeuralConsts &nc, const GridParams &grid,
                                     uint32_t training_step, uint32_t batch_size, uint32_t n, float *positions,
                                     float *targets, uint32_t *sample_nodes, uint32_t learned_lod,
-                                    const NodeSurvival *survival, float4 *state, bool classic_fast_div, int num_sms,
-                                    cudaStream_t s);
+                                    const NodeSurvival *survival, float4 *state, bool classic_fast_div,
+                                    const TrainCull &cull, int num_sms, cudaStream_t s);
 
 // One training pass over n rows (positions n x points x 3, targets n x 8): the hash-grid features
 // into `features` (n x n_inputs, 16-bit), the network matrices packed into `wpacked`
@@ -698,6 +711,9 @@ void build_inference_nodes(const std::vector<BVHNode> &neural, float dil, std::v
 // the box-coordinate precondition of the fast slab division
 bool coords_in_fast_div_domain(const float *c, size_t n);
 bool nodes_in_fast_div_domain(const std::vector<BVHNode> &nodes);
+bool nodes_in_train_div_domain(const std::vector<BVHNode> &nodes);
+bool cut_allows_train_cull(const std::vector<BVHNode> &neural, uint32_t max_depth, float &leaf_extent,
+                           float &max_coord);
 
 } // namespace nbvh
 
