@@ -876,8 +876,8 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
                                                                              uint32_t it)
 {
     const uint32_t count_in = *reinterpret_cast<volatile const uint32_t *>(&a.wave_counts[it % 3u]);
-    if (blockIdx.x * kTailThreads >= count_in)
-        return;
+    if (blockIdx.x >= count_in)
+        return; // warp w of block b has the deal position w * gridDim.x + b: none is left for this block
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t n_in = a.grid.n_inputs, H = a.n_hidden_layers, P = a.grid.n_points;
     const TailLayout TL = tail_layout(a.n_cut_nodes, SMEM_CUT, n_in, H);
@@ -932,10 +932,16 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
     const bool ahead_ok = a.grid.segment_distribution != NBVH_SEGMENT_UNIFORM && a.non_neural == nullptr;
     uint32_t st_segments = 0, st_capped = 0, st_overflow = 0, st_fallback = 0;
 
-    // Rays that need many more segments cluster in space, and so in the node-sorted list: handing
-    // out consecutive rows would leave a few warps with 32 long rays each. Rows are dealt in
-    // transposed order instead (claim i -> row (i mod 32) * R + i / 32), so each warp gets rays
-    // from 32 places of the list.
+    // Lists of up to 32 rays per warp of the grid are dealt at once, ceil(count / warps) rays per warp:
+    // the time of such a list is the latency of its rounds, and a round with few rays gathers and
+    // lists little. (Filling warps with 32 rays left most of the GPU idle: 395 us for the 4,092 rays
+    // that a 512 x 512 frame has here and 379 us for the 26,397 of a 2^22-ray batch; dealt evenly, with
+    // the tile encoder's exact rows, 87 and about 265 us.) Longer lists are claimed by counter. Rays that need many more segments cluster in space, and so in the node-sorted list; claims take rows
+    // in transposed order (claim i -> row (i mod 32) * R + i / 32) and the deal takes every n_warps-th
+    // row, so each warp gets rays from all over the list.
+    const uint32_t n_warps = gridDim.x * kTailWarps, my_deal = warp * gridDim.x + blockIdx.x;
+    const uint32_t per_warp = min(32u, (count_in + n_warps - 1u) / n_warps);
+    const bool dealt = count_in <= 32u * n_warps;
     const uint32_t deal_rows = (count_in + 31u) / 32u, deal_total = 32u * deal_rows;
     RayState s;
     uint32_t stack[kNeuralStackSize];
@@ -948,15 +954,21 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
         // refill: lanes without a ray take the next rows of the list (node order when sorted)
         const unsigned idle = __ballot_sync(kFull, !active);
         if (idle != 0u && !exhausted) {
-            const int leader = __ffs(idle) - 1;
-            uint32_t base = 0;
-            if (lane == leader)
-                base = atomicAdd(head, (uint32_t)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            exhausted = base + (uint32_t)__popc(idle) >= deal_total;
-            const uint32_t c = base + __popc(idle & ((1u << lane) - 1u));
-            const uint32_t i = (c & 31u) * deal_rows + (c >> 5);
-            if (!active && c < deal_total && i < count_in) {
+            uint32_t i;
+            if (dealt) {
+                exhausted = true;
+                i = (uint32_t)lane < per_warp ? (uint32_t)lane * n_warps + my_deal : count_in;
+            } else {
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if (lane == leader)
+                    base = atomicAdd(head, (uint32_t)__popc(idle));
+                base = __shfl_sync(kFull, base, leader);
+                exhausted = base + (uint32_t)__popc(idle) >= deal_total;
+                const uint32_t c = base + __popc(idle & ((1u << lane) - 1u));
+                i = c < deal_total ? (c & 31u) * deal_rows + (c >> 5) : count_in;
+            }
+            if (!active && i < count_in) {
                 load_state(in, sorted ? a.perm[i] : i, s, stack);
                 active = true;
                 cull_ok = s.d.x != 0.0f && s.d.y != 0.0f && s.d.z != 0.0f;
@@ -1042,7 +1054,6 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
         __syncwarp();
         for (uint32_t tile = 0; tile * 16u < rows; tile++) {
             const uint32_t n_t = min(16u, rows - tile * 16u);
-            const uint32_t mask = n_t >= 16u ? 0xFFFFu : ((1u << n_t) - 1u);
             auto pos = [&](uint32_t r, uint32_t p) -> V3 {
                 const float4 e0 = ends[2u * (16u * tile + r)], e1 = ends[2u * (16u * tile + r) + 1u];
                 float t;
@@ -1056,7 +1067,7 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
                 }
                 return segment_point(mk3(e0.x, e0.y, e0.z), mk3(e1.x, e1.y, e1.z), t);
             };
-            encode_tile_any<BF16>(a.table, gp, pos, mask, feat, TL.fld);
+            encode_tile_any<BF16>(a.table, gp, pos, n_t, feat, TL.fld);
             float o4[4];
             mlp_tile_from_smem<BF16, FP8>(sw, feat, TL.fld, n_in, H, o4);
             float *ob = outs + 16u * tile * 8u;

@@ -46,25 +46,32 @@ __host__ __device__ inline SmemNetLayout smem_net_layout(uint32_t n_inputs, uint
 }
 
 // Copies the FP16 network matrices (packed [rows][cols], network-first parameter layout) into
-// the padded shared-memory layout. Whole block participates.
+// the padded shared-memory layout, 16 bytes (8 columns) at a time, four loads of a thread in flight
+// (word by word this copy took 13,000 cycles of every block). Whole block participates.
 __device__ __forceinline__ void load_weights_to_smem(const __half *__restrict__ w, __half *sw, uint32_t n_inputs,
                                                      uint32_t n_hidden_layers)
 {
-    SmemNetLayout L = smem_net_layout(n_inputs, n_hidden_layers);
-    const uint32_t *w32 = reinterpret_cast<const uint32_t *>(w);
-    // matrix 0: 64 x n_inputs
-    uint32_t words0 = kNeurons * n_inputs / 2u;
-    for (uint32_t i = threadIdx.x; i < words0; i += blockDim.x) {
-        uint32_t r = (2u * i) / n_inputs, c = (2u * i) % n_inputs;
-        *reinterpret_cast<uint32_t *>(sw + r * L.ld0 + c) = __ldg(w32 + i);
-    }
-    // hidden 64x64 matrices and the 16x64 output matrix
-    uint32_t rows_rest = (n_hidden_layers - 1u) * kNeurons + kOutputsPadded;
-    uint32_t words_rest = rows_rest * kNeurons / 2u;
-    const uint32_t *wr = w32 + words0;
-    for (uint32_t i = threadIdx.x; i < words_rest; i += blockDim.x) {
-        uint32_t r = (2u * i) / kNeurons, c = (2u * i) % kNeurons;
-        *reinterpret_cast<uint32_t *>(sw + L.hidden_off + r * kHiddenLd + c) = __ldg(wr + i);
+    const SmemNetLayout L = smem_net_layout(n_inputs, n_hidden_layers);
+    const uint4 *src = reinterpret_cast<const uint4 *>(w);
+    // matrix 0 (64 x n_inputs, n_inputs a multiple of 16), then the 64-wide matrices
+    const uint32_t per_row0 = n_inputs / 8u, n0 = kNeurons * per_row0;
+    const uint32_t total = n0 + ((n_hidden_layers - 1u) * kNeurons + kOutputsPadded) * (kNeurons / 8u);
+    auto dst = [&](uint32_t i) {
+        if (i < n0)
+            return sw + (i / per_row0) * L.ld0 + (i % per_row0) * 8u;
+        const uint32_t j = i - n0;
+        return sw + L.hidden_off + (j / (kNeurons / 8u)) * kHiddenLd + (j % (kNeurons / 8u)) * 8u;
+    };
+    for (uint32_t i = threadIdx.x; i < total; i += 4u * blockDim.x) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; k++)
+            if (i + k * blockDim.x < total)
+                v[k] = __ldg(src + i + k * blockDim.x);
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; k++)
+            if (i + k * blockDim.x < total)
+                *reinterpret_cast<uint4 *>(dst(i + k * blockDim.x)) = v[k];
     }
 }
 
@@ -343,6 +350,14 @@ __device__ __forceinline__ void relu_pack(const float (&acc)[8][4], uint32_t (&a
     }
 }
 
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+
 // Forward of one 16-row tile. make_a(kb, a) fills the layer-0 A fragment of k-block kb (16
 // inputs). On return o[0..1] are the sigmoid outputs (row g, cols 2*tig, 2*tig+1) and o[2..3]
 // those of row g + 8 (g = lane / 4, tig = lane % 4), for output columns 0..7.
@@ -353,6 +368,9 @@ __device__ __forceinline__ void mlp_forward_tile(const __half *sw, uint32_t n_in
     using Pr = MlpPrec<BF16>;
     const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const SmemNetLayout L = smem_net_layout(n_inputs, n_hidden_layers);
+    // B fragments of two 8-column blocks by one ldmatrix: lane i addresses row (i & 7) of block (i >> 4),
+    // k half (i >> 3) & 1
+    const uint32_t brow = (lane & 7) + ((lane >> 4) << 3), bcol = ((lane >> 3) & 1) * 8;
     float acc[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; nt++)
@@ -361,12 +379,13 @@ __device__ __forceinline__ void mlp_forward_tile(const __half *sw, uint32_t n_in
     for (uint32_t kb = 0; kb < nkb; kb++) {
         uint32_t a[4];
         make_a(kb, a);
-        const __half *wrow = sw + g * L.ld0 + kb * 16u + tig * 2;
+        const __half *wrow = sw + brow * L.ld0 + kb * 16u + bcol;
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            uint32_t b0 = *reinterpret_cast<const uint32_t *>(wrow + nt * 8 * L.ld0);
-            uint32_t b1 = *reinterpret_cast<const uint32_t *>(wrow + nt * 8 * L.ld0 + 8);
-            Pr::mma(acc[nt], a, b0, b1);
+        for (int nt = 0; nt < 8; nt += 2) {
+            uint32_t b[4];
+            ldsm_x4(b, wrow + nt * 8 * L.ld0);
+            Pr::mma(acc[nt], a, b[0], b[1]);
+            Pr::mma(acc[nt + 1], a, b[2], b[3]);
         }
     }
     const __half *wl = sw + L.hidden_off;
@@ -378,12 +397,13 @@ __device__ __forceinline__ void mlp_forward_tile(const __half *sw, uint32_t n_in
             acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
 #pragma unroll
         for (int kb = 0; kb < 4; kb++) {
-            const __half *wrow = wl + g * kHiddenLd + kb * 16 + tig * 2;
+            const __half *wrow = wl + brow * kHiddenLd + kb * 16 + bcol;
 #pragma unroll
-            for (int nt = 0; nt < 8; nt++) {
-                uint32_t b0 = *reinterpret_cast<const uint32_t *>(wrow + nt * 8 * kHiddenLd);
-                uint32_t b1 = *reinterpret_cast<const uint32_t *>(wrow + nt * 8 * kHiddenLd + 8);
-                Pr::mma(acc[nt], a[kb], b0, b1);
+            for (int nt = 0; nt < 8; nt += 2) {
+                uint32_t b[4];
+                ldsm_x4(b, wrow + nt * 8 * kHiddenLd);
+                Pr::mma(acc[nt], a[kb], b[0], b[1]);
+                Pr::mma(acc[nt + 1], a[kb], b[2], b[3]);
             }
         }
         wl += kNeurons * kHiddenLd;
@@ -403,113 +423,76 @@ __device__ __forceinline__ void mlp_forward_tile(const __half *sw, uint32_t n_in
         o[i] = 1.0f / (1.0f + expf(-oc[i]));
 }
 
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p)
-{
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(a));
-}
+// Encode phase of a tile of `rows` (at most 16) rows: the 16-bit features of every (row, point, level)
+// written to the warp's feature tile feat[16][ld] (ld = n_inputs + 8 halves); the rows past them keep
+// whatever they hold (an MLP row depends on its own features alone). The warp's lanes take the
+// (row, level, point) items in turn, points fastest (a row's points are neighbours, so their corners
+// share cache lines on the coarser levels), kTileItems at a time: the positions first, then the
+// gathers of all of them without branches in between, so that they are in flight together. A lane
+// past the last item repeats its first one. No MLP accumulator is live here.
+//
+// The gathers bound this phase: a lane's 8 corners lie in as many cache lines, and the L1 takes one
+// line per cycle, so work for rows that do not exist costs as much as work for rows that do (the
+// form before this one rounded up to 4 rows and put 32 (point, level) pairs of one row in a warp).
+// Two items at once: 700 us per 512 x 512 frame and 2,925 per 2^22-ray query against 707 and 2,970
+// with four, which spill.
+constexpr uint32_t kTileItems = 2;
 
-// Encode phase of a 16-row tile: FP16 features of every (row, point, level) written to the warp's
-// feature tile feat[16][ld] (ld = n_inputs + 8 halves); rows not in active_mask16 are zero. Lane j
-// handles the (point, level) pairs j, j + 32, ... for all rows, four rows at a time: the four
-// rows' points are formed first (an inactive row takes the cube centre, whose gathers are cheap L1
-// hits) and then encoded without branches in between, so that the 32 gathers are in flight
-// together; groups of four inactive rows are skipped. No MLP accumulator is live here.
-template <bool BF16, typename PosFn>
-__device__ __forceinline__ void encode_tile_to_smem(const uint32_t *__restrict__ table, const GridParams &gp,
-                                                    PosFn &&pos, uint32_t active_mask16, __half *feat, uint32_t ld)
-{
-    const int lane = threadIdx.x & 31;
-    const uint32_t L = gp.n_levels, PL = gp.n_points * gp.n_levels;
-    for (uint32_t j = (uint32_t)lane; j < PL; j += 32u) {
-        const uint32_t p = j / L, l = j - p * L;
-        for (uint32_t r0 = 0; r0 < 16u; r0 += 4u) {
-            const uint32_t m4 = (active_mask16 >> r0) & 0xFu;
-            if (m4 == 0u) {
-#pragma unroll
-                for (uint32_t k = 0; k < 4u; k++)
-                    *reinterpret_cast<uint32_t *>(feat + (r0 + k) * ld + 2u * j) = 0u;
-                continue;
-            }
-            V3 q[4];
-#pragma unroll
-            for (uint32_t k = 0; k < 4u; k++)
-                q[k] = ((m4 >> k) & 1u) ? pos(r0 + k, p) : mk3(0.5f, 0.5f, 0.5f);
-            float2 f[4];
-#pragma unroll
-            for (uint32_t k = 0; k < 4u; k++)
-                f[k] = encode_level<false>(table, gp, l, q[k]);
-#pragma unroll
-            for (uint32_t k = 0; k < 4u; k++)
-                *reinterpret_cast<uint32_t *>(feat + (r0 + k) * ld + 2u * j) =
-                    ((m4 >> k) & 1u) ? MlpPrec<BF16>::pack(f[k].x, f[k].y) : 0u;
-        }
-    }
-    __syncwarp();
-}
-
-// encode_tile_to_smem for 4 or 8 features per level: lane j handles the (point, level) pairs
-// j, j + 32, ... and writes their F features (one 8- or 16-byte store per row), 8 / F rows at a
-// time so that the same number of gathered words is in flight as in the 2-feature form.
 template <bool BF16, uint32_t F, typename PosFn>
-__device__ __forceinline__ void encode_tile_to_smem_wide(const void *__restrict__ table, const GridParams &gp,
-                                                         PosFn &&pos, uint32_t active_mask16, __half *feat,
-                                                         uint32_t ld)
+__device__ __forceinline__ void encode_tile_to_smem(const uint32_t *__restrict__ table, const GridParams &gp,
+                                                    PosFn &&pos, uint32_t rows, __half *feat, uint32_t ld)
 {
-    constexpr uint32_t RB = 8u / F; // rows per batch
-    const int lane = threadIdx.x & 31;
-    const uint32_t L = gp.n_levels, PL = gp.n_points * gp.n_levels;
-    for (uint32_t j = (uint32_t)lane; j < PL; j += 32u) {
-        const uint32_t p = j / L, l = j - p * L;
-        for (uint32_t r0 = 0; r0 < 16u; r0 += RB) {
-            const uint32_t mb = (active_mask16 >> r0) & ((1u << RB) - 1u);
-            uint32_t w[RB][F / 2];
-            if (mb == 0u) {
+    constexpr uint32_t N = F == 2u ? kTileItems : 8u / F; // the same number of gathered words in flight
+    const uint32_t lane = threadIdx.x & 31u, P = gp.n_points, L = gp.n_levels, PL = P * L, total = rows * PL;
+    for (uint32_t i0 = lane; i0 < total; i0 += 32u * N) {
+        V3 q[N];
+        uint32_t lev[N], dst[N];
 #pragma unroll
-                for (uint32_t k = 0; k < RB; k++)
+        for (uint32_t k = 0; k < N; k++) {
+            const uint32_t i = i0 + 32u * k < total ? i0 + 32u * k : i0;
+            const uint32_t r = i / PL, j = i - r * PL, l = j / P, p = j - l * P;
+            q[k] = pos(r, p);
+            lev[k] = l;
+            dst[k] = r * ld + (p * L + l) * F;
+        }
+        uint32_t w[N][F / 2u];
 #pragma unroll
-                    for (uint32_t q = 0; q < F / 2; q++)
-                        w[k][q] = 0u;
+        for (uint32_t k = 0; k < N; k++) {
+            if constexpr (F == 2u) {
+                const float2 f = encode_level<false>(table, gp, lev[k], q[k]);
+                w[k][0] = MlpPrec<BF16>::pack(f.x, f.y);
             } else {
-                V3 qp[RB];
+                float f[F];
+                encode_level_wide<F>(table, gp, lev[k], q[k], f);
 #pragma unroll
-                for (uint32_t k = 0; k < RB; k++)
-                    qp[k] = ((mb >> k) & 1u) ? pos(r0 + k, p) : mk3(0.5f, 0.5f, 0.5f);
-#pragma unroll
-                for (uint32_t k = 0; k < RB; k++) {
-                    float f[F];
-                    encode_level_wide<F>(table, gp, l, qp[k], f);
-#pragma unroll
-                    for (uint32_t q = 0; q < F / 2; q++)
-                        w[k][q] = ((mb >> k) & 1u) ? MlpPrec<BF16>::pack(f[2 * q], f[2 * q + 1]) : 0u;
-                }
+                for (uint32_t c = 0; c < F / 2u; c++)
+                    w[k][c] = MlpPrec<BF16>::pack(f[2u * c], f[2u * c + 1u]);
             }
+        }
 #pragma unroll
-            for (uint32_t k = 0; k < RB; k++) {
-                __half *dst = feat + (r0 + k) * ld + F * j;
-                if constexpr (F == 4)
-                    *reinterpret_cast<uint2 *>(dst) = make_uint2(w[k][0], w[k][1]);
-                else
-                    *reinterpret_cast<uint4 *>(dst) = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
-            }
+        for (uint32_t k = 0; k < N; k++) { // one 4-, 8- or 16-byte store (a repeated item writes the same bits)
+            if constexpr (F == 2u)
+                *reinterpret_cast<uint32_t *>(feat + dst[k]) = w[k][0];
+            else if constexpr (F == 4u)
+                *reinterpret_cast<uint2 *>(feat + dst[k]) = make_uint2(w[k][0], w[k][1]);
+            else
+                *reinterpret_cast<uint4 *>(feat + dst[k]) = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
         }
     }
     __syncwarp();
 }
 
-// The encode phase of a 16-row tile for the grid's features per level (2, 4 or 8).
+// The encode phase of a tile for the grid's features per level (2, 4 or 8).
 template <bool BF16, typename PosFn>
 __device__ __forceinline__ void encode_tile_any(const uint32_t *__restrict__ table, const GridParams &gp, PosFn &&pos,
-                                                uint32_t active_mask16, __half *feat, uint32_t ld)
+                                                uint32_t rows, __half *feat, uint32_t ld)
 {
     if (gp.n_features == 4u)
-        encode_tile_to_smem_wide<BF16, 4>(table, gp, pos, active_mask16, feat, ld);
+        encode_tile_to_smem<BF16, 4>(table, gp, pos, rows, feat, ld);
     else if (gp.n_features == 8u)
-        encode_tile_to_smem_wide<BF16, 8>(table, gp, pos, active_mask16, feat, ld);
+        encode_tile_to_smem<BF16, 8>(table, gp, pos, rows, feat, ld);
     else
-        encode_tile_to_smem<BF16>(table, gp, pos, active_mask16, feat, ld);
+        encode_tile_to_smem<BF16, 2>(table, gp, pos, rows, feat, ld);
 }
 
 // MLP phase of a 16-row tile whose 16-bit features are in feat[16][ld]; outputs as mlp_forward_tile.
