@@ -57,27 +57,11 @@ __host__ __device__ inline uint32_t w0_bytes(uint32_t n_inputs) { return kNeuron
 __host__ __device__ inline uint32_t hidden_w_bytes() { return kNeurons * kNeurons * 2u; }
 __host__ __device__ inline uint32_t out_w_bytes() { return kOutputsPadded * kNeurons * 2u; }
 
-// FP16 network matrices (network-first parameter order, each [rows][cols] row-major) -> the
-// K-major core-matrix operand layout, matrices back to back.
 __global__ void k_pack_weights(const __half *__restrict__ w, uint32_t n_inputs, uint32_t n_hidden_layers,
                                __half *__restrict__ packed)
 {
-    const uint32_t n0 = kNeurons * n_inputs, nh = (n_hidden_layers - 1u) * kNeurons * kNeurons;
-    const uint32_t total = n0 + nh + kOutputsPadded * kNeurons;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        uint32_t byte;
-        if (i < n0) {
-            byte = tc::operand_offset(i / n_inputs, i % n_inputs, kNeurons);
-        } else if (i < n0 + nh) {
-            const uint32_t j = i - n0, m = j / (kNeurons * kNeurons), e = j % (kNeurons * kNeurons);
-            byte = w0_bytes(n_inputs) + m * hidden_w_bytes() + tc::operand_offset(e / kNeurons, e % kNeurons, kNeurons);
-        } else {
-            const uint32_t e = i - n0 - nh;
-            byte = w0_bytes(n_inputs) + (n_hidden_layers - 1u) * hidden_w_bytes() +
-                   tc::operand_offset(e / kNeurons, e % kNeurons, kOutputsPadded);
-        }
-        packed[byte / 2u] = w[i];
-    }
+    tc::pack_weights(w, n_inputs, n_hidden_layers, packed, blockIdx.x * blockDim.x + threadIdx.x,
+                     gridDim.x * blockDim.x);
 }
 
 struct MlpTcArgs {
@@ -376,8 +360,8 @@ uint32_t packed_weight_bytes(uint32_t n_inputs, uint32_t n_hidden_layers)
 cudaError_t launch_pack_weights(const __half *params_h, uint32_t n_inputs, uint32_t n_hidden_layers, __half *packed,
                                 cudaStream_t s)
 {
-    const uint32_t total = packed_weight_bytes(n_inputs, n_hidden_layers) / 2u;
-    k_pack_weights<<<(total + 255u) / 256u, 256, 0, s>>>(params_h, n_inputs, n_hidden_layers, packed);
+    const uint32_t pieces = packed_weight_bytes(n_inputs, n_hidden_layers) / 16u;
+    k_pack_weights<<<(pieces + 127u) / 128u, 128, 0, s>>>(params_h, n_inputs, n_hidden_layers, packed);
     return cudaGetLastError();
 }
 

@@ -22,6 +22,7 @@
 #include "device_math.cuh"
 #include "net_device.cuh"
 #include "nbvh_internal.h"
+#include "tc_device.cuh"
 
 namespace nbvh {
 
@@ -49,14 +50,22 @@ constexpr uint32_t kDefaultVisitsPerRound = 12;
 constexpr uint32_t kEncodeBlocksPerSm = 4;
 // From step tail_step() on, the rays still listed are finished by one persistent kernel
 // (k_wave_tail) instead of one short wavefront step after another: the lists are short by then and
-// each step would cost about the same fixed 60-80 us whatever its length. The switch depends only
-// on the step (how many segments a ray has evaluated) and on the cut, so a ray's record does not
-// depend on the other rays of its batch. Measured on GB300: cuts up to kMaxSortNodes nodes (their
-// later steps still fill the GPU) gain most from step 5 on, larger learned cuts (long runs of
-// small leaves, lists that stay short for 20-30 steps) from step 3 on.
-__host__ __device__ constexpr uint32_t tail_step(uint32_t n_cut_nodes)
+// each step would cost about the same fixed 40-60 us whatever its length. The step follows from the
+// size of the batch and of the cut; which kernel evaluates a segment does not show in its record,
+// since mma.sync and tcgen05 give the same bits on the same FP16 or BF16 rows (a test holds both to
+// that). Each wavefront step costs a batch of n rays about 30 us + what its kernels take; the tail
+// kernel costs no fixed time but about four times as much per segment. Measured on GB300 with the
+// tail from step 0 / 1 / 2 / 3 / 4 / 5 on, us per call (1,024-leaf cut, uniform rays; secondary and
+// camera rays cross at the same sizes within a factor of two):
+//   n =     2,048   110 / 148 / 187 / 210 / 248 / 280     n =   131,072   400 / 383 / 366 / 373 / 388 / 425
+//   n =    16,384   184 / 190 / 203 / 236 / 269 / 299     n =   524,288  1062 / 891 / 771 / 739 / 743 / 760
+//   n =    32,768   238 / 229 / 226 / 252 / 279 / 310     n = 1,048,576  1827 / 1389 / 1145 / 1081 / 1056 / 1072
+// Larger learned cuts (long runs of small leaves, lists that stay short for 20-30 steps) gain from
+// step 3 on whatever the batch.
+__host__ __device__ constexpr uint32_t tail_step(uint32_t n_cut_nodes, uint32_t n)
 {
-    return n_cut_nodes <= kMaxSortNodes ? 5u : 3u;
+    const uint32_t step = n <= (1u << 14) ? 0u : n <= (1u << 17) ? 2u : n <= (1u << 19) ? 3u : n <= (1u << 20) ? 4u : 5u;
+    return n_cut_nodes > kMaxSortNodes && step > 3u ? 3u : step;
 }
 constexpr uint32_t kTailWarps = 8;
 constexpr uint32_t kTailThreads = kTailWarps * 32;
@@ -101,6 +110,7 @@ struct WaveArgs {
     uint32_t *late_list;
     uint32_t *late_count;
     uint32_t late_from;
+    uint32_t tail_at; // the step the tail kernel takes over at
 };
 
 __device__ __forceinline__ void write_hit(nbvh_neural_hit *hits, uint32_t id, float t, V3 nrm, V3 alb, float vis,
@@ -351,6 +361,26 @@ __global__ void __launch_bounds__(kRayBinThreads) k_ray_bin_place(const __grid_c
     __syncthreads();
     for (uint32_t i = r0 + threadIdx.x; i < r1; i += blockDim.x)
         a.order[atomicAdd(&cnt[a.keys[i]], 1u)] = i;
+}
+
+// What a query needs before its first pass, in one launch (it was four memsets and a launch): its
+// counters cleared, the sort's counts and cursors cleared, the matrices packed for k_mlp_tc.
+struct BeginArgs {
+    uint32_t *zero[5];
+    uint32_t n_zero[5];
+    const __half *weights; // nullptr: no tensor-core step will run
+    __half *wpacked;
+    uint32_t n_inputs, n_hidden_layers;
+};
+__global__ void __launch_bounds__(128) k_query_begin(const __grid_constant__ BeginArgs a)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (a.weights)
+        tc::pack_weights(a.weights, a.n_inputs, a.n_hidden_layers, a.wpacked, i, stride);
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+        for (uint32_t j = i; j < a.n_zero[k]; j += stride)
+            a.zero[k][j] = 0u;
 }
 
 // K2 first pass: the first entered leaf of every ray (the first leaf is searched with an unbounded
@@ -936,9 +966,10 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
     // the time of such a list is the latency of its rounds, and a round with few rays gathers and
     // lists little. (Filling warps with 32 rays left most of the GPU idle: 395 us for the 4,092 rays
     // that a 512 x 512 frame has here and 379 us for the 26,397 of a 2^22-ray batch; dealt evenly, with
-    // the tile encoder's exact rows, 87 and about 265 us.) Longer lists are claimed by counter. Rays that need many more segments cluster in space, and so in the node-sorted list; claims take rows
-    // in transposed order (claim i -> row (i mod 32) * R + i / 32) and the deal takes every n_warps-th
-    // row, so each warp gets rays from all over the list.
+    // the tile encoder's exact rows, 87 and about 265 us.) Longer lists are claimed by counter. Rays
+    // that need many more segments cluster in space, and so in the node-sorted list; claims take rows in
+    // transposed order (claim i -> row (i mod 32) * R + i / 32) and the deal takes every n_warps-th row,
+    // so each warp gets rays from all over the list.
     const uint32_t n_warps = gridDim.x * kTailWarps, my_deal = warp * gridDim.x + blockIdx.x;
     const uint32_t per_warp = min(32u, (count_in + n_warps - 1u) / n_warps);
     const bool dealt = count_in <= 32u * n_warps;
@@ -1250,9 +1281,9 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
     const uint32_t enc_blocks = (uint32_t)num_sms * enc_per_sm;
     const uint32_t dec_blocks = (uint32_t)num_sms * (SMEM_CUT ? 1u : 2u);
     for (uint32_t it = it0; it < it1; it++) {
-        if (it == tail_step(a.n_cut_nodes)) {
-            // the rest of the query in one launch; the list counters are cleared after it, so every
-            // later check (or the counters a captured graph copies out) reads an empty list
+        if (it == a.tail_at) {
+            // the rest of the query in one launch; in a captured graph the list counters are cleared
+            // after it, so that the copy the graph ends with reads an empty list
             if (a.perm) {
                 k_wave_sort<<<(uint32_t)num_sms, kSortThreads, 3u * a.n_sort_nodes * 4u, s>>>(a, it);
                 e = cudaGetLastError();
@@ -1261,7 +1292,7 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
                 launches++;
             }
             e = launch_tail(a, it, num_sms, !r.capture_only, r.stage_cut, s);
-            if (e == cudaSuccess)
+            if (e == cudaSuccess && r.capture_only)
                 e = cudaMemsetAsync(a.wave_counts, 0, 3u * sizeof(uint32_t), s);
             if (e != cudaSuccess)
                 return e;
@@ -1345,10 +1376,12 @@ cudaError_t check_done(const WaveArgs &a, const StepResources &r, uint32_t it, c
 }
 
 // The step loop from step `from` (after `unchecked` steps launched without a host check when from
-// is 0): batches of kStepsPerCheck steps, the host reading the list length after each batch. The
-// loop ends when a list comes out empty or at the step cap (each ray at most
-// max_traversal_steps + 1 segments) plus the final capping step. With capture_only the unchecked
-// steps and the copy of the counters are only enqueued (for stream capture) and nothing waits.
+// is 0): the steps up to and with the tail kernel, which answers every ray left, then one host
+// check; where no tail kernel comes (a step limit below it, a resumed query) batches of
+// kStepsPerCheck steps, the host reading the list length after each. The loop ends when a list comes
+// out empty or at the step cap (each ray at most max_traversal_steps + 1 segments) plus the final
+// capping step. With capture_only the unchecked steps and the copy of the counters are only
+// enqueued (for stream capture) and nothing waits.
 template <bool SMEM_CUT>
 cudaError_t run_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem, int num_sms, uint32_t max_steps,
                       uint32_t from, cudaStream_t s, uint32_t &launches)
@@ -1373,18 +1406,19 @@ cudaError_t run_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem
             return cudaMemcpyAsync(r.h_words, a.wave_counts, 4u * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
         bool done = false;
         e = check_done(a, r, it, s, done);
-        if (e != cudaSuccess || done)
+        if (e != cudaSuccess || done || it > a.tail_at)
             return e;
     }
     while (it < limit) {
-        const uint32_t batch = (limit - it) < kStepsPerCheck ? (limit - it) : kStepsPerCheck;
+        const uint32_t want = it <= a.tail_at ? a.tail_at + 1u - it : kStepsPerCheck;
+        const uint32_t batch = (limit - it) < want ? (limit - it) : want;
         e = enqueue_steps<SMEM_CUT>(a, r, dec_smem, num_sms, it, it + batch, s, launches);
         if (e != cudaSuccess)
             return e;
         it += batch;
         bool done = false;
         e = check_done(a, r, it, s, done);
-        if (e != cudaSuccess || done)
+        if (e != cudaSuccess || done || it > a.tail_at)
             return e;
     }
     return cudaSuccess;
@@ -1478,7 +1512,10 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     a.n_sort_nodes = a.sub_bins ? kSubBins * n_bins : n_bins;
     a.bf16 = prec == NBVH_PRECISION_BF16 ? 1u : 0u;
     a.prec = prec;
-    const bool sort = res.perm != nullptr && n_bins <= kMaxSortNodes;
+    // (no list of a batch below kSortMinRows rays is long enough to be sorted)
+    const bool sort = res.perm != nullptr && n_bins <= kMaxSortNodes && n >= kSortMinRows;
+    // a stalled wait (failure-path test) needs the tensor-core kernels to run
+    a.tail_at = tail_step(n_cut_nodes, res.stall ? 0xFFFFFFFFu : n);
     a.perm = sort ? res.perm : nullptr;
     a.row_keys = (sort && a.n_sort_nodes <= 65536u) ? res.row_keys : nullptr;
     a.ray_order = nullptr;
@@ -1499,19 +1536,18 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
                    : run_steps<false>(a, res, 0, num_sms, nc.max_traversal_steps, res.resume_from, s, *launches);
     // words 0-2: rotating list lengths; 3: the MLP's error word; 4-6: rotating work counters of
     // the decode kernel; 7: work counter of the first pass
-    cudaError_t e = cudaMemsetAsync(wave_counts, 0, 8u * sizeof(uint32_t), s);
-    if (e == cudaSuccess && res.drain_host)
-        e = cudaMemsetAsync(res.late_count, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess)
-        return e;
-    if (sort) {
-        e = cudaMemsetAsync(res.node_bins, 0, 2u * a.n_sort_nodes * sizeof(uint32_t), s);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(res.node_cursor, 0, 2u * a.n_sort_nodes * sizeof(uint32_t), s);
-        if (e != cudaSuccess)
-            return e;
-    }
-    e = launch_pack_weights(params_h, grid.n_inputs, n_hidden_layers, res.wpacked, s);
+    const uint32_t sort_words = sort ? 2u * a.n_sort_nodes : 0u;
+    static_assert(sizeof(QueryCounters) % sizeof(uint32_t) == 0, "counters are cleared word by word");
+    const BeginArgs ba = {{reinterpret_cast<uint32_t *>(counters), wave_counts, res.late_count, res.node_bins,
+                           res.node_cursor},
+                          {(uint32_t)(sizeof(QueryCounters) / sizeof(uint32_t)), 8u, res.drain_host ? 1u : 0u,
+                           sort_words, sort_words},
+                          a.tail_at > 0u ? params_h : nullptr,
+                          res.wpacked,
+                          grid.n_inputs,
+                          n_hidden_layers};
+    k_query_begin<<<a.tail_at > 0u ? 2u * (uint32_t)num_sms / 8u : 1u, 128, 0, s>>>(ba);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
     *launches = 2;

@@ -553,8 +553,8 @@ void neural_query_noalloc(nbvh_handle *h, const nbvh_ray *d_rays, uint32_t n, ui
     cuda_check(noalloc_scratch(h->device, &sc), "fixed scratch address");
     if (n == 0)
         return;
-    cuda_check(cudaMemsetAsync(sc.counters, 0, sizeof(QueryCounters), s), "reset counters");
     if (h->cfg.bvh.ignore_neural_blas) {
+        cuda_check(cudaMemsetAsync(sc.counters, 0, sizeof(QueryCounters), s), "reset counters");
         cuda_check(launch_classic_as_neural(h->d_nodes.ptr, h->d_tris.ptr, d_rays, n, d_hits, false,
                                             h->classic_fast_div, s),
                    "classic");
@@ -2120,9 +2120,8 @@ uint32_t run_neural_query(const nbvh_handle *h, QueryContext &q, QueryCounters *
                           const StepResources *tune)
 {
     uint32_t *list = q.fallback_list.ptr;
-    if (!tune || tune->resume_from == 0u)
-        cuda_check(cudaMemsetAsync(counters, 0, sizeof(QueryCounters), s), "reset counters");
     if (h->cfg.bvh.ignore_neural_blas) {
+        cuda_check(cudaMemsetAsync(counters, 0, sizeof(QueryCounters), s), "reset counters");
         // the non-neural BLAS switch: the mesh goes to the classic traversal
         // (include/cuda/neural/neural_bvh_module_common.cuh:323)
         cuda_check(launch_classic_as_neural(h->d_nodes.ptr, h->d_tris.ptr, d_rays, n, d_hits, vis_only,

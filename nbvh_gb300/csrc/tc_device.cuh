@@ -13,7 +13,10 @@
 #pragma once
 
 #include <cstdint>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
+
+#include "nbvh_internal.h"
 
 namespace nbvh {
 namespace tc {
@@ -24,6 +27,30 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)
 __host__ __device__ constexpr uint32_t operand_offset(uint32_t r, uint32_t k, uint32_t rows)
 {
     return (k >> 3) * (rows * 16u) + r * 16u + (k & 7u) * 2u;
+}
+
+// The network matrices (parameter order, each [rows][cols] row-major) -> the operand layout, matrices
+// back to back; 16-byte pieces (8 columns of one row) `first`, `first + stride`, ... of them.
+__device__ __forceinline__ void pack_weights(const __half *__restrict__ w, uint32_t n_inputs, uint32_t n_hidden_layers,
+                                             __half *__restrict__ packed, uint32_t first, uint32_t stride)
+{
+    constexpr uint32_t per = kNeurons / 8u, hidden = kNeurons * per; // pieces of a row and of a 64 x 64 matrix
+    const uint32_t per0 = n_inputs / 8u, n0 = kNeurons * per0, nh = (n_hidden_layers - 1u) * hidden;
+    const uint4 *src = reinterpret_cast<const uint4 *>(w);
+    uint4 *dst = reinterpret_cast<uint4 *>(packed);
+    for (uint32_t i = first; i < n0 + nh + kOutputsPadded * per; i += stride) {
+        uint32_t base, r, c, rows = kNeurons;
+        if (i < n0) {
+            base = 0u, r = i / per0, c = i % per0;
+        } else if (i < n0 + nh) {
+            const uint32_t e = (i - n0) % hidden;
+            base = i - e, r = e / per, c = e % per;
+        } else {
+            const uint32_t e = i - n0 - nh;
+            base = n0 + nh, r = e / per, c = e % per, rows = kOutputsPadded;
+        }
+        dst[base + c * rows + r] = __ldg(src + i);
+    }
 }
 
 // ---- mbarrier ----------------------------------------------------------------------------------

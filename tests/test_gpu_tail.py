@@ -1,5 +1,6 @@
-"""The tail kernel deals short lists over all its warps and claims long ones by counter; the answer
-of a ray depends on neither. Whole batches against the same rays in pieces, word for word, with
+"""The tail kernel deals short lists over all its warps and claims long ones by counter, and takes over
+from the wavefront steps earlier the smaller the batch, from the first segment on for the smallest:
+its mma.sync tiles and the tcgen05 MLP have to give the same bits. Whole batches against the same rays in pieces, word for word, with
 networks that accept about half of the segments and with none accepted (every ray then evaluates
 every leaf it enters, as the segment enumeration counts them)."""
 
@@ -13,17 +14,18 @@ from nbvh_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
 
-# (points, levels, features, precision): one row of a tile is points x levels items of the encoder
-NETS = [(4, 16, 2, 0), (3, 8, 4, 1), (2, 4, 8, 2), (1, 8, 2, 0)]
+# (points, levels, features, precision, hidden layers): a row of a tile is points x levels items of the encoder
+NETS = [(4, 16, 2, 0, 4), (3, 8, 4, 1, 4), (2, 4, 8, 2, 4), (1, 8, 2, 0, 1), (4, 16, 2, 1, 8), (4, 8, 4, 2, 3)]
 
 
 @pytest.mark.parametrize("net", NETS)
 @pytest.mark.parametrize("threshold", [0.5, 2.0])
 def test_tail_lists_of_every_length(built, net, threshold):
-    P, L, F, prec = net
+    P, L, F, prec, H = net
     cfg = nb.default_config(**{"hashgrid.n_levels": L, "hashgrid.n_features_per_level": F, "hashgrid.base_resolution": 8,
                                "hashgrid.log2_hashmap_size": 14, "module.input_segment_points": P,
-                               "network.precision": prec, "output.primary_visibility_threshold": threshold})
+                               "network.precision": prec, "network.n_hidden_layers": H,
+                               "output.primary_visibility_threshold": threshold})
     h, s = handle(cfg, kind="soup64k", seed=2, depth=12)
     with h:
         rng = np.random.default_rng(5)
