@@ -356,45 +356,86 @@ __device__ __forceinline__ void composite_loss(const LossConsts &lc, uint32_t ch
 }
 
 // ---------------------------------------------------------------------------------------------
-// The hash-grid features of the training rows, in the MLP precision, into rows of row_stride
-// halves (n_inputs: the tensor-core kernel's feature rows): one thread per (row, point), the
-// levels in order, F features per level stored together (K3 forward).
+// The hash-grid features of explicit rows (training batches, nbvh_network_inference), in the MLP
+// precision, into rows of n_inputs halves: one thread per (row, point), the levels in order, 8
+// features (LPS levels) per 16-byte store (K3 forward). `split`: the point's levels are spread over
+// L / LPS threads instead, one store each; batches too small to fill the GPU otherwise are bound by
+// the latency of one thread's gathers, level after level (3,001 rows: 37 -> 15 us). Large batches are
+// bound by the L1's misses to L2 (ncu: L1 88%, L2 68%); 4-byte stores, sixteen partial sectors a
+// point, were the rest of 289 us per 2^18 rows, 222 now (264 -> 206 in a training step).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_train_encode(const __grid_constant__ GridParams grid,
-                                                      const uint32_t *__restrict__ table,
-                                                      const float *__restrict__ positions, uint32_t n,
-                                                      __half *__restrict__ feat, uint32_t row_stride, uint32_t bf16)
+template <uint32_t F>
+__global__ void __launch_bounds__(256, 4) k_encode_rows(const __grid_constant__ GridParams grid,
+                                                     const uint32_t *__restrict__ table,
+                                                     const float *__restrict__ positions, uint32_t n,
+                                                     __half *__restrict__ feat, uint32_t bf16_, uint32_t split)
 {
-    const uint32_t P = grid.n_points, L = grid.n_levels, F = grid.n_features;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)n * P)
+    constexpr uint32_t LPS = 8u / F;
+    const uint32_t P = grid.n_points, L = grid.n_levels, G = split ? L / LPS : 1u, LG = L / G;
+    const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= (uint64_t)n * P * G)
         return;
-    const uint32_t row = (uint32_t)(i / P), p = (uint32_t)(i - (uint64_t)row * P);
+    const uint64_t i = w / G; // (row, point)
+    const uint32_t l0 = (uint32_t)(w - i * G) * LG;
     const float *src = positions + i * 3u;
     const V3 pos = mk3(__ldg(src), __ldg(src + 1), __ldg(src + 2));
+    const bool bf16 = bf16_ != 0u;
     auto pack16 = [bf16](float lo, float hi) { return bf16 ? pack_bf162(lo, hi) : pack_half2(lo, hi); };
-    __half *dst = feat + (size_t)row * row_stride + (size_t)p * L * F;
-    for (uint32_t l = 0; l < L; l++) {
-        if (F == 4u) {
-            float f[4];
-            encode_level_wide<4>(table, grid, l, pos, f);
-            *reinterpret_cast<uint2 *>(dst + 4u * l) = make_uint2(pack16(f[0], f[1]), pack16(f[2], f[3]));
-        } else if (F == 8u) {
-            float f[8];
-            encode_level_wide<8>(table, grid, l, pos, f);
-            *reinterpret_cast<uint4 *>(dst + 8u * l) =
-                make_uint4(pack16(f[0], f[1]), pack16(f[2], f[3]), pack16(f[4], f[5]), pack16(f[6], f[7]));
-        } else {
-            const float2 f = encode_level<true>(table, grid, l, pos);
-            *reinterpret_cast<uint32_t *>(dst + 2u * l) = pack16(f.x, f.y);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(feat) + i * L * (F / 2u);
+    if (L % LPS == 0u) { // every point's block of L * F halves starts 16-byte aligned
+        for (uint32_t l = l0; l < l0 + LG; l += LPS) {
+            uint32_t q[4];
+#pragma unroll
+            for (uint32_t k = 0; k < LPS; k++) {
+                if constexpr (F == 2u) {
+                    const float2 f = encode_level<true>(table, grid, l + k, pos);
+                    q[k] = pack16(f.x, f.y);
+                } else {
+                    float f[F];
+                    encode_level_wide<F>(table, grid, l + k, pos, f);
+#pragma unroll
+                    for (uint32_t c = 0; c < F / 2u; c++)
+                        q[k * (F / 2u) + c] = pack16(f[2u * c], f[2u * c + 1u]);
+                }
+            }
+            *reinterpret_cast<uint4 *>(dst + l * (F / 2u)) = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+    } else { // level by level (4 bytes for F = 2, 8 for F = 4; F = 8 never comes here)
+        for (uint32_t l = 0; l < L; l++) {
+            if constexpr (F == 2u) {
+                const float2 f = encode_level<true>(table, grid, l, pos);
+                dst[l] = pack16(f.x, f.y);
+            } else if constexpr (F == 4u) {
+                float f[4];
+                encode_level_wide<4>(table, grid, l, pos, f);
+                *reinterpret_cast<uint2 *>(dst + 2u * l) = make_uint2(pack16(f[0], f[1]), pack16(f[2], f[3]));
+            }
         }
     }
+}
+
+cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const float *positions, uint32_t n,
+                        __half *features, bool bf16, int num_sms, cudaStream_t s)
+{
+    const uint32_t lps = 8u / grid.n_features, groups = grid.n_levels / lps;
+    const uint64_t points = (uint64_t)n * grid.n_points, lanes = (uint64_t)num_sms * 2048u;
+    const bool split = grid.n_levels % lps == 0u && points * groups <= lanes;
+    const uint64_t threads = points * (split ? groups : 1u);
+    const unsigned blocks = (unsigned)((threads + 255u) / 256u);
+    const uint32_t b = bf16 ? 1u : 0u, sp = split ? 1u : 0u;
+    if (grid.n_features == 4u)
+        k_encode_rows<4><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+    else if (grid.n_features == 8u)
+        k_encode_rows<8><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+    else
+        k_encode_rows<2><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------
 // Training forward + composite loss + backward on the tensor cores (K3/K4 backward).
 //
-// k_train_encode writes each row's FP16 features; then one CTA per SM (128 threads, one tile row
+// k_encode_rows writes each row's FP16 features; then one CTA per SM (128 threads, one tile row
 // per thread and TMEM lane) runs 128-row tiles through
 //   forward   Z_{j+1} = X_j W_j^T for every matrix j (tcgen05, M = 128 rows), the ReLU'd 16-bit
 //             activations X_{j+1} written back to shared memory (and their ReLU masks kept in
@@ -749,86 +790,117 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------------
-// Hash-grid gradient scatter: one thread per (row, point), the levels in order; the corners and
-// weights of the forward encoding, each corner's F feature gradients added with vector atomics
-// (the 16-bit input-feature gradients come from k_train_tc).
+// Hash-grid gradient scatter (K3 backward): the corners and weights of the forward encoding, each
+// corner's feature gradients added with vector atomics (the 16-bit input-feature gradients come from
+// k_train_tc). Two neighbouring lanes take one level of one row, the even lane the lower x corners,
+// the odd lane the upper ones, and go through the row's points; points in the same cell are summed
+// in registers and leave as one set of atomics.
+//
+// The L2 bounds this kernel: it takes about 2e11 32-byte sectors of atomics a second, whatever part
+// of the sector they touch. The points of a row lie on a short segment, so on the coarser levels most
+// share a cell (45 sets of corners instead of 64 for the 64 (point, level) pairs of a row). And the
+// entries of x and x + 1 lie in one sector 3 times in 4 (2 features; tcnn's hash multiplies x by 1), so
+// the two lanes' atomics of one instruction merge into one. Warps are 16 rows of one level: the
+// levels' parameters are uniform and a coarse level's warp skips the atomics it merges. 2^18 rows:
+// 511 -> 354 us with gradients everywhere (428 with the points merged but one lane for both x
+// corners), 352 -> 232 us in a training step of the trained network.
 // ---------------------------------------------------------------------------------------------
 
-template <bool BF16>
-__global__ void __launch_bounds__(256) k_grid_scatter(const __grid_constant__ GridParams grid,
-                                                      const float *__restrict__ positions,
-                                                      const __half *__restrict__ dfeat, uint32_t n,
-                                                      float *__restrict__ grid_grad)
+constexpr uint32_t kScatterThreads = 256, kScatterRows = 32; // rows of a block
+// features one thread sums: all of an entry, or 4 of 8
+template <uint32_t F>
+constexpr uint32_t kScatterFeatures = F < 4u ? F : 4u;
+
+template <bool BF16, uint32_t F>
+__global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_constant__ GridParams grid,
+                                                                 const float *__restrict__ positions,
+                                                                 const __half *__restrict__ dfeat, uint32_t n,
+                                                                 float *__restrict__ grid_grad)
 {
-    const uint32_t P = grid.n_points, L = grid.n_levels, F = grid.n_features, n_in = grid.n_inputs;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)n * P)
-        return;
-    const uint32_t row = (uint32_t)(i / P), p = (uint32_t)(i - (uint64_t)row * P);
-    const float *src = positions + i * 3u;
-    const V3 pp = mk3(__ldg(src), __ldg(src + 1), __ldg(src + 2));
-    const uint32_t *gw = reinterpret_cast<const uint32_t *>(dfeat + (size_t)row * n_in + (size_t)p * L * F);
-    for (uint32_t l = 0; l < L; l++) {
-        float g[8];
-        bool any = false;
-        for (uint32_t q = 0; q < F / 2u; q++) {
-            const float2 v = MlpPrec<BF16>::unpack(__ldg(gw + l * (F / 2u) + q));
-            g[2 * q] = v.x;
-            g[2 * q + 1] = v.y;
-            any |= v.x != 0.f || v.y != 0.f;
-        }
-        if (!any)
+    constexpr uint32_t FT = kScatterFeatures<F>, parts = F / FT;
+    const uint32_t P = grid.n_points, L = grid.n_levels;
+    for (uint32_t k = threadIdx.x; k < 2u * kScatterRows * L * parts; k += kScatterThreads) {
+        const uint32_t up = k & 1u, row = blockIdx.x * kScatterRows + ((k >> 1) & (kScatterRows - 1u));
+        const uint32_t lp = k / (2u * kScatterRows), l = lp / parts, part = lp % parts;
+        if (row >= n)
             continue;
         const float s = grid.scale[l];
-        const float px = __fmaf_rn(pp.x, s, 0.5f), py = __fmaf_rn(pp.y, s, 0.5f), pz = __fmaf_rn(pp.z, s, 0.5f);
-        const float flx = floorf(px), fly = floorf(py), flz = floorf(pz);
-        const uint32_t gx = (uint32_t)(int32_t)flx, gy = (uint32_t)(int32_t)fly, gz = (uint32_t)(int32_t)flz;
-        const float rx = __fsub_rn(px, flx), ry = __fsub_rn(py, fly), rz = __fsub_rn(pz, flz);
-        const uint32_t res = grid.res[l], size = grid.size[l], off = grid.offset[l];
+        const uint32_t res = grid.res[l], size = grid.size[l];
         const bool hashed = grid.hashed[l] != 0u;
-        auto corner = [&](uint32_t c, uint32_t &idx, float &w) {
-            const uint32_t x = gx + (c & 1u), y = gy + ((c >> 1) & 1u), z = gz + ((c >> 2) & 1u);
-            if (hashed) {
-                idx = (x ^ (y * 2654435761u) ^ (z * 805459861u)) & (size - 1u);
-            } else {
-                idx = x + y * res + z * res * res;
-                if (idx >= size)
-                    idx %= size;
-            }
-            w = __fmul_rn(__fmul_rn((c & 1u) ? rx : __fsub_rn(1.0f, rx), (c & 2u) ? ry : __fsub_rn(1.0f, ry)),
-                          (c & 4u) ? rz : __fsub_rn(1.0f, rz));
-        };
-        // corners in pairs (x, x + 1): with 2 features, a pair whose entries are the two halves of
-        // one aligned 16-byte word (every even x on hashed levels, every even entry on dense
-        // ones) takes one 16-byte atomic instead of two 8-byte ones
+        float *level = grid_grad + (size_t)grid.offset[l] * F + part * FT;
+        float acc[4][FT]; // corners (up, y, z)
+        uint32_t cx = 0u, cy = 0u, cz = 0u;
+        bool have = false;
+        auto flush = [&]() { // adds the sums of cell (cx, cy, cz)
 #pragma unroll
-        for (uint32_t c = 0; c < 8; c += 2) {
-            uint32_t i0, i1;
-            float w0, w1;
-            corner(c, i0, w0);
-            corner(c + 1u, i1, w1);
-            if (F == 2u) {
-                const uint32_t e0 = off + i0, e1 = off + i1;
-                if ((e0 ^ e1) == 1u) {
-                    const uint32_t lo = e0 < e1 ? e0 : e1;
-                    const float wl = e0 < e1 ? w0 : w1, wh = e0 < e1 ? w1 : w0;
-                    atomicAdd(reinterpret_cast<float4 *>(grid_grad + (size_t)lo * 2u),
-                              make_float4(wl * g[0], wl * g[1], wh * g[0], wh * g[1]));
+            for (uint32_t c = 0; c < 4u; c++) {
+                const uint32_t x = cx + up, y = cy + (c & 1u), z = cz + (c >> 1);
+                uint32_t i;
+                if (hashed) {
+                    i = (x ^ (y * 2654435761u) ^ (z * 805459861u)) & (size - 1u);
                 } else {
-                    atomicAdd(reinterpret_cast<float2 *>(grid_grad + (size_t)e0 * 2u), make_float2(w0 * g[0], w0 * g[1]));
-                    atomicAdd(reinterpret_cast<float2 *>(grid_grad + (size_t)e1 * 2u), make_float2(w1 * g[0], w1 * g[1]));
+                    i = x + y * res + z * res * res;
+                    if (i >= size)
+                        i %= size;
                 }
-            } else {
-                float *ea = grid_grad + (size_t)(off + i0) * F, *eb = grid_grad + (size_t)(off + i1) * F;
-                for (uint32_t q = 0; q < F / 4u; q++) {
-                    atomicAdd(reinterpret_cast<float4 *>(ea) + q,
-                              make_float4(w0 * g[4 * q], w0 * g[4 * q + 1], w0 * g[4 * q + 2], w0 * g[4 * q + 3]));
-                    atomicAdd(reinterpret_cast<float4 *>(eb) + q,
-                              make_float4(w1 * g[4 * q], w1 * g[4 * q + 1], w1 * g[4 * q + 2], w1 * g[4 * q + 3]));
-                }
+                if constexpr (FT == 2u)
+                    atomicAdd(reinterpret_cast<float2 *>(level + 2u * (size_t)i), make_float2(acc[c][0], acc[c][1]));
+                else
+                    atomicAdd(reinterpret_cast<float4 *>(level + (size_t)i * F),
+                              make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]));
+            }
+        };
+        const float *src = positions + (size_t)row * P * 3u;
+        const uint32_t *gw = reinterpret_cast<const uint32_t *>(dfeat) + ((size_t)row * P * L + l) * (F / 2u) + part * 2u;
+        for (uint32_t p = 0; p < P; p++, src += 3, gw += L * (F / 2u)) {
+            float g[FT];
+            bool any = false;
+#pragma unroll
+            for (uint32_t q = 0; q < FT / 2u; q++) {
+                const float2 v = MlpPrec<BF16>::unpack(__ldg(gw + q));
+                g[2u * q] = v.x;
+                g[2u * q + 1u] = v.y;
+                any |= v.x != 0.f || v.y != 0.f;
+            }
+            if (!any)
+                continue;
+            const float px = __fmaf_rn(__ldg(src), s, 0.5f), py = __fmaf_rn(__ldg(src + 1), s, 0.5f),
+                        pz = __fmaf_rn(__ldg(src + 2), s, 0.5f);
+            const float flx = floorf(px), fly = floorf(py), flz = floorf(pz);
+            const uint32_t gx = (uint32_t)(int32_t)flx, gy = (uint32_t)(int32_t)fly, gz = (uint32_t)(int32_t)flz;
+            const float rx = __fsub_rn(px, flx), ry = __fsub_rn(py, fly), rz = __fsub_rn(pz, flz);
+            const bool same = have && gx == cx && gy == cy && gz == cz;
+            if (have && !same)
+                flush();
+            cx = gx, cy = gy, cz = gz;
+            have = true;
+            const float wx = up ? rx : __fsub_rn(1.0f, rx);
+#pragma unroll
+            for (uint32_t c = 0; c < 4u; c++) {
+                const float w = __fmul_rn(__fmul_rn(wx, (c & 1u) ? ry : __fsub_rn(1.0f, ry)),
+                                          (c & 2u) ? rz : __fsub_rn(1.0f, rz));
+#pragma unroll
+                for (uint32_t f = 0; f < FT; f++)
+                    acc[c][f] = same ? __fmaf_rn(w, g[f], acc[c][f]) : __fmul_rn(w, g[f]);
             }
         }
+        if (have)
+            flush();
     }
+}
+
+template <bool BF16>
+cudaError_t scatter_rows(const GridParams &grid, const float *positions, const __half *dfeat, uint32_t n,
+                         float *grid_grad, cudaStream_t s)
+{
+    const unsigned blocks = (n + kScatterRows - 1u) / kScatterRows;
+    if (grid.n_features == 4u)
+        k_grid_scatter<BF16, 4><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+    else if (grid.n_features == 8u)
+        k_grid_scatter<BF16, 8><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+    else
+        k_grid_scatter<BF16, 2><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1028,17 +1100,15 @@ cudaError_t launch_training_samples(const float4 *neural_nodes, const float4 *no
 }
 
 cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
-                               const float *positions, uint32_t n, __half *features, bool bf16, cudaStream_t s)
+                               const float *positions, uint32_t n, __half *features, bool bf16, int num_sms,
+                               cudaStream_t s)
 {
     if (n == 0)
         return cudaSuccess;
     const uint32_t n_network_params =
         kNeurons * grid.n_inputs + (n_hidden_layers - 1u) * kNeurons * kNeurons + kOutputsPadded * kNeurons;
     const uint32_t *table = reinterpret_cast<const uint32_t *>(params_h + n_network_params);
-    const uint64_t threads = (uint64_t)n * grid.n_points;
-    k_train_encode<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(grid, table, positions, n, features,
-                                                                      grid.n_inputs, bf16 ? 1u : 0u);
-    return cudaGetLastError();
+    return encode_rows(grid, table, positions, n, features, bf16, num_sms, s);
 }
 
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
@@ -1056,12 +1126,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     const uint32_t n_network_params =
         kNeurons * n_in + (H - 1u) * kNeurons * kNeurons + kOutputsPadded * kNeurons;
     const uint32_t *table = reinterpret_cast<const uint32_t *>(params_h + n_network_params);
-    {
-        const uint64_t threads = (uint64_t)n * grid.n_points;
-        k_train_encode<<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(grid, table, positions, n, features, n_in,
-                                                                          bf16 ? 1u : 0u);
-    }
-    e = cudaGetLastError();
+    e = encode_rows(grid, table, positions, n, features, bf16, num_sms, s);
     if (e == cudaSuccess)
         e = launch_pack_weights(params_h, n_in, H, wpacked, s);
     if (e == cudaSuccess && marks)
@@ -1099,14 +1164,8 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     }
     if (marks && (e = cudaEventRecord(marks[2], s)) != cudaSuccess)
         return e;
-    const uint64_t threads = (uint64_t)n * grid.n_points;
-    if (bf16)
-        k_grid_scatter<true><<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(grid, positions, dfeat, n,
-                                                                                 grad + n_network_params);
-    else
-        k_grid_scatter<false><<<(unsigned)((threads + 255u) / 256u), 256, 0, s>>>(grid, positions, dfeat, n,
-                                                                                  grad + n_network_params);
-    e = cudaGetLastError();
+    e = bf16 ? scatter_rows<true>(grid, positions, dfeat, n, grad + n_network_params, s)
+             : scatter_rows<false>(grid, positions, dfeat, n, grad + n_network_params, s);
     if (e == cudaSuccess && marks)
         e = cudaEventRecord(marks[3], s);
     return e;

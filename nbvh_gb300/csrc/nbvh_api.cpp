@@ -1341,7 +1341,8 @@ nbvh_status nbvh_network_inference(nbvh_handle *h, const float *d_positions, uin
         cuda_check(make_feature_map(h->d_infer_feat.ptr, ni, n, &map), "feature map");
         cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
         cuda_check(cudaEventRecord(h->ev0, s), "event");
-        cuda_check(launch_encode_rows(h->d_params_h.ptr, h->grid, H, d_positions, n, h->d_infer_feat.ptr, mlp_bf16(h), s),
+        cuda_check(launch_encode_rows(h->d_params_h.ptr, h->grid, H, d_positions, n, h->d_infer_feat.ptr, mlp_bf16(h),
+                                      h->num_sms, s),
                    "encode");
         cuda_check(launch_pack_weights(h->d_params_h.ptr, ni, H, h->d_wpacked.ptr, s), "pack weights");
         cuda_check(launch_mlp_tc(map, h->d_wpacked.ptr, ni, H, n, nullptr, d_outputs, h->d_status.ptr, mlp_prec(h),

@@ -573,7 +573,8 @@ cudaError_t launch_segments(const float4 *dilated_nodes, const float4 *bounds, c
 // The FP16 (BF16 when bf16) hash-grid features of n rows of encoded positions into rows of
 // n_inputs values (the tcgen05 MLP's input layout).
 cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
-                               const float *positions, uint32_t n, __half *features, bool bf16, cudaStream_t s);
+                               const float *positions, uint32_t n, __half *features, bool bf16, int num_sms,
+                               cudaStream_t s);
 
 // tcgen05 fully fused MLP (k_mlp_tc.cu): weights packed into the tensor-core operand layout, then
 // 128-row tiles of FP16 inputs (row-major [rows][n_inputs], 16-byte aligned) fed by TMA through
