@@ -193,12 +193,15 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
             atomicOr(a.status, 2u);
         return;
     }
-    const uint32_t tid = threadIdx.x, gid = tid / kGroupThreads, gtid = tid % kGroupThreads;
+    // (warp indices through a shuffle: uniform values for the MMA descriptors, see tc::elect_one)
+    const uint32_t tid = threadIdx.x, warp_index = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    const uint32_t gid = warp_index / (kGroupThreads / 32u), gtid = tid % kGroupThreads;
     const uint32_t warp = gtid >> 5, row = gtid;
     // the group's issuing thread: lane 0 of warp (gid mod 4), so that the groups' issuers sit on
     // different schedulers; it alone waits on the group's mbarriers, the other warps sleep in the
     // group barrier meanwhile
     const bool issuer = gtid == 32u * (gid & 3u);
+    const bool mma_warp = (warp_index & 3u) == (gid & 3u); // its warp
     unsigned char *tile = smem + tile_offset(a.wbytes) + gid * tile_bytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + tile_offset(a.wbytes) + G * tile_bytes);
     uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 2u * G + 2u);
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem_all = *slot;
+    const uint32_t tmem_all = __shfl_sync(0xFFFFFFFFu, *slot, 0);
     const uint32_t tmem = tmem_all + gid * kGroupCols;
     const uint32_t tmem_row = tmem + ((32u * warp) << 16);
 
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
         ph_load ^= 1u;
         load_pending = false;
         for (uint32_t layer = 0; layer <= H; layer++) {
-            if (issuer) {
+            if (mma_warp && tc::elect_one()) {
                 tc::fence_after_sync();
                 if (layer == 0 && sw128)
                     issue_layer_sw128(tmem, t_addr, w_addr, K, kNeurons, id_hidden);

@@ -435,8 +435,8 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 // ---------------------------------------------------------------------------------------------
 // Training forward + composite loss + backward on the tensor cores (K3/K4 backward).
 //
-// k_encode_rows writes each row's FP16 features; then one CTA per SM (128 threads, one tile row
-// per thread and TMEM lane) runs 128-row tiles through
+// k_encode_rows writes each row's FP16 features; then one CTA per SM (256 threads, two per tile row
+// and TMEM lane) runs 128-row tiles through
 //   forward   Z_{j+1} = X_j W_j^T for every matrix j (tcgen05, M = 128 rows), the ReLU'd 16-bit
 //             activations X_{j+1} written back to shared memory (and their ReLU masks kept in
 //             registers), then the sigmoid, the composite loss and dZ_out = dL/dZ_out;
@@ -448,11 +448,17 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 // added to the FP32 gradient once per CTA at the end. Every [128 rows][C columns] tile lives in
 // shared memory in the K-major core-matrix layout (8-column block c at c * 2,048 bytes, row r at
 // r * 16 within it): with M = rows it is a K-major operand (LBO 2,048, SBO 128), with K = rows an
-// MN-major one (LBO 128, SBO 2,048). The input tile arrives in that layout from TMA (8-value boxes).
+// MN-major one (LBO 128, SBO 2,048). The input tile is copied into that layout 16 bytes at a time.
 // ---------------------------------------------------------------------------------------------
 
 constexpr uint32_t kTcRows = 128;
-constexpr uint32_t kTcThreads = 128;
+// Two threads per tile row, each with half of its columns: the step is bound by the chain MMA ->
+// accumulator read -> rounding -> shared-memory tile -> next MMA, ten times per tile, and the half
+// rows shorten its epilogues. With that, the input tiles by cp.async, the weight-gradient MMAs under
+// the next epilogue and the MMAs issued from uniform registers (tc::elect_one) a pass over 2^18 rows
+// went from 218 to 188 us; only the last of the four shows alone (215 us without it), since the chain
+// waited for the MMAs to be issued.
+constexpr uint32_t kTcThreads = 256;
 constexpr uint32_t kColBlock = kTcRows * 16u; // bytes between 8-column blocks of a row tile
 constexpr uint32_t kTcAccCols = 128;          // TMEM columns of the current layer's accumulator
 constexpr uint32_t kTcTmemCols = 512;
@@ -460,7 +466,8 @@ constexpr uint32_t kTcWgColsMax = kTcTmemCols - kTcAccCols;
 constexpr uint32_t kTcMaxMatrices = kMaxHiddenLayers + 1u;
 
 struct TrainTcArgs {
-    const __half *wpacked; // 16-bit matrices in the K-major operand layout, back to back
+    const __half *features; // n x n_inputs
+    const __half *wpacked;  // 16-bit matrices in the K-major operand layout, back to back
     uint32_t wbytes;
     uint32_t n_inputs;
     uint32_t n_hidden_layers;
@@ -478,7 +485,8 @@ struct TrainTcArgs {
     // shared-memory offsets (bytes from the 1,024-byte aligned base)
     uint32_t x0_off;                      // two input tile buffers of n_inputs * 256 bytes
     uint32_t x_off[kTcMaxMatrices];       // X_j (j = 1..H): 64-column tile (shared when not in wg_mask)
-    uint32_t dz_off, dzo_off, bar_off;
+    uint32_t dz_off[2], dzo_off, bar_off; // dZ_j alternates between two tiles (one where only one fits)
+    uint32_t loss_off;                    // [kTcRows] loss of each row's upper four channels
     uint32_t wg_col[kTcMaxMatrices];      // TMEM column of the dW_j^T accumulator
     uint64_t wait_ns;                     // time limit of the phase waits
     uint32_t stall;                       // failure-path test: wait on an mbarrier nothing arrives at
@@ -509,8 +517,7 @@ __device__ __forceinline__ void store_row_chunks(unsigned char *tile, uint32_t r
 }
 
 template <bool BF16, bool FP8>
-__global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constant__ CUtensorMap fmap,
-                                                            const __grid_constant__ TrainTcArgs a)
+__global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constant__ TrainTcArgs a)
 {
     using Pr = MlpPrec<BF16>;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -518,21 +525,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     const uint32_t n_tiles = (a.n + kTcRows - 1u) / kTcRows;
     if (blockIdx.x >= n_tiles)
         return;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
-    const bool issuer = tid == 0u;
-    // weights, load 0, load 1, mma, and one nothing arrives at (failure-path test)
+    // this thread's tile row (= TMEM lane) and half of its columns
+    const uint32_t tid = threadIdx.x & (kTcRows - 1u), half = threadIdx.x / kTcRows, warp = tid >> 5;
+    const bool issuer = threadIdx.x == 0u;
+    const bool mma_warp = __shfl_sync(kFull, threadIdx.x >> 5, 0) == 0u; // allocates TMEM, issues the MMAs
+    // weights, mma, one nothing arrives at (failure-path test), end
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + a.bar_off);
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 5);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 4);
+    float *upper_loss = reinterpret_cast<float *>(smem + a.loss_off);
     const uint32_t base = tc::smem_addr(smem);
-    const uint32_t bar_w = tc::smem_addr(&bars[0]), bar_mma = tc::smem_addr(&bars[3]);
+    const uint32_t bar_w = tc::smem_addr(&bars[0]), bar_mma = tc::smem_addr(&bars[1]),
+                   bar_end = tc::smem_addr(&bars[3]);
     const uint32_t x0_bytes = K0 * kTcRows * 2u;
 
-    if (warp == 0u) {
+    if (mma_warp) {
         tc::tmem_alloc(tc::smem_addr(slot), kTcTmemCols);
         tc::tmem_relinquish();
     }
     if (issuer) {
-        for (uint32_t b = 0; b < 5u; b++)
+        for (uint32_t b = 0; b < 4u; b++)
             tc::mbar_init(tc::smem_addr(&bars[b]), 1u);
         tc::mbar_init_fence();
     }
@@ -542,29 +553,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     const uint32_t tmem = *slot;
     const uint32_t lane_off = (32u * warp) << 16; // this warp's TMEM lanes
 
+    // This thread's 16-byte pieces of tile t's input rows (zeros past the batch), K0 / 16 of them:
+    // neighbouring lanes take the two halves of a 32-byte sector. (As sixteen TMA boxes of 128 x 16
+    // bytes the tile took 9,000 of the 34,000 cycles a tile needs, and its issuing thread with it.)
     auto load_tile = [&](uint32_t t, uint32_t buf) {
-        const uint32_t bar = tc::smem_addr(&bars[1u + buf]);
-        const uint32_t dst = base + a.x0_off + buf * x0_bytes;
-        tc::mbar_expect_tx(bar, x0_bytes);
-        for (uint32_t c = 0; c < K0 / 8u; c++)
-            tc::tma_load_2d(dst + c * kColBlock, &fmap, (int32_t)(8u * c), (int32_t)(t * kTcRows), bar);
+        const uint32_t r = (threadIdx.x >> 1) & (kTcRows - 1u), row = t * kTcRows + r, odd = threadIdx.x & 1u;
+        const __half *src = a.features + (size_t)(row < a.n ? row : 0u) * K0 + 8u * odd;
+        const uint32_t dst = base + a.x0_off + buf * x0_bytes + odd * kColBlock + r * 16u;
+        for (uint32_t c = 0; c < K0 / 16u; c++)
+            tc::copy16_async(dst + 2u * c * kColBlock, src + 16u * c, row < a.n);
     };
     uint32_t t = blockIdx.x;
-    bool load_pending[2] = {false, false};
     if (issuer) {
         tc::mbar_expect_tx(bar_w, a.wbytes);
         for (uint32_t o = 0; o < a.wbytes; o += 16384u)
             tc::bulk_load(base + o, reinterpret_cast<const unsigned char *>(a.wpacked) + o,
                           a.wbytes - o < 16384u ? a.wbytes - o : 16384u, bar_w);
-        load_tile(t, 0u);
     }
-    load_pending[0] = true;
+    load_tile(t, 0u);
     bool ok = issuer ? tc::mbar_wait(bar_w, 0u, a.wait_ns) : true;
     if (a.stall && issuer) // nothing ever arrives at this barrier: the wait runs out
-        ok = ok && tc::mbar_wait(tc::smem_addr(&bars[4]), 0u, a.wait_ns);
+        ok = ok && tc::mbar_wait(tc::smem_addr(&bars[2]), 0u, a.wait_ns);
     ok = __syncthreads_and(ok);
 
-    uint32_t ph_load[2] = {0u, 0u}, ph_mma = 0u, buf = 0u;
+    uint32_t ph_mma = 0u, buf = 0u;
     bool mma_pending = false, first_tile = true;
     float loss_acc = 0.f;
     // waits for the MMAs committed so far; false (everyone) if the wait gave up
@@ -579,158 +591,157 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
         return r;
     };
     for (; ok && t < n_tiles; t += gridDim.x, buf ^= 1u) {
-        ok = issuer ? tc::mbar_wait(tc::smem_addr(&bars[1u + buf]), ph_load[buf], a.wait_ns) : true;
-        ok = __syncthreads_and(ok);
-        if (!ok)
-            break;
-        ph_load[buf] ^= 1u;
-        load_pending[buf] = false;
-        // the other buffer's last reader (the previous tile's MMAs) has completed
-        if (t + gridDim.x < n_tiles) {
-            if (issuer)
-                load_tile(t + gridDim.x, buf ^ 1u);
-            load_pending[buf ^ 1u] = true;
-        }
+        tc::copy_async_wait();
+        tc::fence_async_shared(); // the tile's pieces are read by the MMAs
+        __syncthreads();
         const uint32_t x0_addr = base + a.x0_off + buf * x0_bytes;
         auto x_addr = [&](uint32_t j) { return j == 0u ? x0_addr : base + a.x_off[j]; };
         const uint32_t row = t * kTcRows + tid;
         const bool valid = row < a.n;
-        uint32_t relu_mask[2u * kTcMaxMatrices]; // bit c of X_j's row: words 2j, 2j + 1
+        uint32_t relu_mask[kTcMaxMatrices]; // bit c: column 32 * half + c of X_j's row
+        float row_loss = 0.f;
         // ---------------- forward ----------------
         for (uint32_t j = 0; j <= H && ok; j++) {
             const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
-            if (issuer) {
+            if (mma_warp && tc::elect_one()) {
                 tc::fence_after_sync();
                 const uint32_t idesc = tc::idesc_f16(kTcRows, nout, BF16);
                 const uint32_t w_addr = base + tc_w_off(j, K0), a_addr = x_addr(j);
-                for (uint32_t k = 0; k < nin / 16u; k++) {
-                    const uint64_t ad = tc::smem_desc(a_addr + 2u * k * kColBlock, kColBlock, 128u);
-                    const uint64_t bd = tc::smem_desc(w_addr + 2u * k * (nout * 16u), nout * 16u, 128u);
-                    tc::mma_f16(tmem, ad, bd, idesc, k > 0u ? 1u : 0u);
-                }
+                tc::mma_chain(tmem, tc::smem_desc(a_addr, kColBlock, 128u), kColBlock / 8u,
+                              tc::smem_desc(w_addr, nout * 16u, 128u), 2u * nout, idesc, nin / 16u, 0u);
                 tc::mma_commit(bar_mma);
             }
             mma_pending = true;
             if (!(ok = mma_done()))
                 break;
+            // the other buffer's last readers, the previous tile's MMAs, are done as well
+            if (j == 0u && t + gridDim.x < n_tiles)
+                load_tile(t + gridDim.x, buf ^ 1u);
             if (j < H) { // X_{j+1} = relu(Z_{j+1}) in the MLP precision (FP8 mode: E4M3 into hidden matrices)
-                uint32_t v[4][16];
+                uint32_t v[2][16];
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    tc::tmem_ld16(tmem + lane_off + 16u * q, v[q]);
+                for (int q = 0; q < 2; q++)
+                    tc::tmem_ld16(tmem + lane_off + 32u * half + 16u * q, v[q]);
                 tc::tmem_wait_ld();
-                uint32_t packed[32];
+                uint32_t packed[16];
                 const bool quant = FP8 && j + 1u < H;
-                uint32_t m0 = 0u, m1 = 0u;
+                uint32_t m = 0u;
 #pragma unroll
-                for (int c = 0; c < 32; c++) {
+                for (int c = 0; c < 16; c++) {
                     const float lo = __uint_as_float(v[c >> 3][(2 * c) & 15]);
                     const float hi = __uint_as_float(v[c >> 3][(2 * c + 1) & 15]);
                     const uint32_t p = quant ? fp8_act_relu_half2(lo, hi) : pack_relu<BF16>(lo, hi);
                     packed[c] = p;
-                    const uint32_t bits = ((p & 0xFFFFu) != 0u ? 1u : 0u) | ((p >> 16) != 0u ? 2u : 0u);
-                    if (c < 16)
-                        m0 |= bits << (2 * c);
-                    else
-                        m1 |= bits << (2 * (c - 16));
+                    m |= (((p & 0xFFFFu) != 0u ? 1u : 0u) | ((p >> 16) != 0u ? 2u : 0u)) << (2 * c);
                 }
-                relu_mask[2u * (j + 1u)] = m0;
-                relu_mask[2u * (j + 1u) + 1u] = m1;
-                store_row_chunks(smem + a.x_off[j + 1u], tid, packed, 8u);
-            } else { // sigmoid, composite loss, dZ_out
+                relu_mask[j + 1u] = m;
+                store_row_chunks(smem + a.x_off[j + 1u] + 4u * half * kColBlock, tid, packed, 4u);
+            } else { // sigmoid, composite loss, dZ_out: this thread's four of the row's 8 channels
                 uint32_t v[8];
                 tc::tmem_ld8(tmem + lane_off, v);
                 tc::tmem_wait_ld();
-                float tgt[8];
+                float4 tgt = make_float4(0.f, 0.f, 0.f, 0.f);
+                float target_vis = 0.f;
                 if (valid) {
-                    const float4 t0 = __ldg(reinterpret_cast<const float4 *>(a.targets + (size_t)row * 8u));
-                    const float4 t1 = __ldg(reinterpret_cast<const float4 *>(a.targets + (size_t)row * 8u) + 1);
-                    tgt[0] = t0.x, tgt[1] = t0.y, tgt[2] = t0.z, tgt[3] = t0.w;
-                    tgt[4] = t1.x, tgt[5] = t1.y, tgt[6] = t1.z, tgt[7] = t1.w;
+                    tgt = __ldg(reinterpret_cast<const float4 *>(a.targets + (size_t)row * 8u) + half);
+                    target_vis = __ldg(a.targets + (size_t)row * 8u);
                 }
-                float dz[8], val[8];
+                const float t4[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
+                float dz[4], val[4];
 #pragma unroll
-                for (int ch = 0; ch < 8; ch++) {
-                    const float y = 1.0f / (1.0f + expf(-__uint_as_float(v[ch])));
+                for (int c = 0; c < 4; c++) {
+                    const float y = 1.0f / (1.0f + expf(-__uint_as_float(half ? v[4 + c] : v[c])));
                     float value = 0.f, gr = 0.f;
                     if (valid) {
-                        composite_loss(a.lc, (uint32_t)ch, y, tgt[ch], tgt[0], value, gr);
+                        composite_loss(a.lc, 4u * half + (uint32_t)c, y, t4[c], target_vis, value, gr);
                         gr = Pr::round(gr); // 16-bit output gradient
                     }
-                    val[ch] = value;
-                    dz[ch] = gr * y * (1.0f - y); // sigmoid backward
+                    val[c] = value;
+                    dz[c] = gr * y * (1.0f - y); // sigmoid backward
                 }
-                const float rl = ((val[0] + val[1]) + (val[2] + val[3])) + ((val[4] + val[5]) + (val[6] + val[7]));
-                loss_acc += rl;
-                if (valid && a.emit && a.sample_loss)
-                    a.sample_loss[row] = rl;
-                uint32_t packed[8] = {Pr::pack(dz[0], dz[1]), Pr::pack(dz[2], dz[3]), Pr::pack(dz[4], dz[5]),
-                                      Pr::pack(dz[6], dz[7]), 0u, 0u, 0u, 0u};
-                store_row_chunks(smem + a.dzo_off, tid, packed, 2u);
+                row_loss = (val[0] + val[1]) + (val[2] + val[3]);
+                if (half)
+                    upper_loss[tid] = row_loss;
+                unsigned char *dzo = smem + a.dzo_off + tid * 16u;
+                *reinterpret_cast<uint2 *>(dzo + 8u * half) = make_uint2(Pr::pack(dz[0], dz[1]), Pr::pack(dz[2], dz[3]));
+                *reinterpret_cast<uint2 *>(dzo + kColBlock + 8u * half) = make_uint2(0u, 0u); // padding outputs
             }
             tc::fence_async_shared(); // the tile rows written above are read by the next MMAs
             tc::fence_before_sync();
             __syncthreads();
         }
+        if (ok && half == 0u) {
+            row_loss += upper_loss[tid];
+            loss_acc += row_loss;
+            if (valid && a.emit && a.sample_loss)
+                a.sample_loss[row] = row_loss;
+        }
         // ---------------- backward ----------------
         for (int jj = (int)H; jj >= (int)a.min_matrix && ok; jj--) {
             const uint32_t j = (uint32_t)jj;
             const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
-            const uint32_t dz_addr = base + (j == H ? a.dzo_off : a.dz_off);
+            const uint32_t dz_addr = base + (j == H ? a.dzo_off : a.dz_off[(j + 1u) & 1u]);
             const bool dgrad = j > a.min_matrix || (j == 0u && a.emit);
             const bool wgrad = (a.wg_mask >> j) & 1u;
-            if (issuer) {
+            // With two dZ tiles the epilogue only waits for dX_j; dW_j's MMAs run under it. A later commit
+            // covers them, so they are done before the next step writes the tile they read (its own
+            // commit comes after them), before the next tile overwrites X_j, and at the end.
+            const bool overlap = dgrad && a.dz_off[0] != a.dz_off[1];
+            if (mma_warp && tc::elect_one()) {
                 tc::fence_after_sync();
                 if (dgrad) { // dX_j (128 x nin) = dZ_{j+1} (128 x nout) . W_j (nout x nin), W_j MN-major
                     const uint32_t idesc = tc::idesc_f16_major(kTcRows, nin, BF16, false, true);
                     const uint32_t w_addr = base + tc_w_off(j, K0);
-                    for (uint32_t k = 0; k < nout / 16u; k++) {
-                        const uint64_t ad = tc::smem_desc(dz_addr + 2u * k * kColBlock, kColBlock, 128u);
-                        const uint64_t bd = tc::smem_desc(w_addr + 256u * k, 128u, nout * 16u);
-                        tc::mma_f16(tmem, ad, bd, idesc, k > 0u ? 1u : 0u);
-                    }
+                    tc::mma_chain(tmem, tc::smem_desc(dz_addr, kColBlock, 128u), kColBlock / 8u,
+                                  tc::smem_desc(w_addr, 128u, nout * 16u), 16u, idesc, nout / 16u, 0u);
+                    if (overlap)
+                        tc::mma_commit(bar_mma);
                 }
                 if (wgrad) { // dW_j^T (128 x nout; rows >= nin unused) += X_j^T . dZ_{j+1}, K = the 128 rows
                     const uint32_t idesc = tc::idesc_f16_major(kTcRows, nout, BF16, true, true);
                     const uint32_t xa = x_addr(j);
-                    for (uint32_t k = 0; k < kTcRows / 16u; k++) {
-                        const uint64_t ad = tc::smem_desc(xa + 256u * k, 128u, kColBlock);
-                        const uint64_t bd = tc::smem_desc(dz_addr + 256u * k, 128u, kColBlock);
-                        tc::mma_f16(tmem + a.wg_col[j], ad, bd, idesc, (first_tile && k == 0u) ? 0u : 1u);
-                    }
+                    static_assert(kTcRows / 16u == 8u, "one chain");
+                    tc::mma_chain(tmem + a.wg_col[j], tc::smem_desc(xa, 128u, kColBlock), 16u,
+                                  tc::smem_desc(dz_addr, 128u, kColBlock), 16u, idesc, 8u, first_tile ? 0u : 1u);
                 }
-                tc::mma_commit(bar_mma);
+                if (!overlap)
+                    tc::mma_commit(bar_mma);
             }
             mma_pending = true;
             if (!(ok = mma_done()))
                 break;
             if (j >= 1u && j > a.min_matrix) { // dZ_j = dX_j * (X_j > 0), 16-bit
-                uint32_t v[4][16];
+                uint32_t v[2][16];
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    tc::tmem_ld16(tmem + lane_off + 16u * q, v[q]);
+                for (int q = 0; q < 2; q++)
+                    tc::tmem_ld16(tmem + lane_off + 32u * half + 16u * q, v[q]);
                 tc::tmem_wait_ld();
-                const uint32_t m0 = relu_mask[2u * j], m1 = relu_mask[2u * j + 1u];
-                uint32_t packed[32];
+                const uint32_t m = relu_mask[j];
+                uint32_t packed[16];
 #pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const uint32_t bits = (c < 16 ? m0 >> (2 * c) : m1 >> (2 * (c - 16))) & 3u;
+                for (int c = 0; c < 16; c++) {
+                    const uint32_t bits = (m >> (2 * c)) & 3u;
                     const float lo = (bits & 1u) ? __uint_as_float(v[c >> 3][(2 * c) & 15]) : 0.f;
                     const float hi = (bits & 2u) ? __uint_as_float(v[c >> 3][(2 * c + 1) & 15]) : 0.f;
                     packed[c] = Pr::pack(lo, hi);
                 }
-                store_row_chunks(smem + a.dz_off, tid, packed, 8u);
+                store_row_chunks(smem + a.dz_off[j & 1u] + 4u * half * kColBlock, tid, packed, 4u);
             } else if (j == 0u && a.emit) { // dX_0, rounded to the MLP precision, for the grid scatter
                 uint4 *dst = reinterpret_cast<uint4 *>(a.dfeat + (size_t)row * K0);
-                for (uint32_t q = 0; q < K0 / 16u; q++) {
-                    uint32_t v[16];
-                    tc::tmem_ld16(tmem + lane_off + 16u * q, v); // warp-wide: rows past the batch too
-                    tc::tmem_wait_ld();
-                    if (valid) {
+                uint32_t v[4][16]; // 16-column pieces half, half + 2, ...: all in flight, one wait
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; i++)
+                    if (2u * i + half < K0 / 16u) // warp-wide: rows past the batch too
+                        tc::tmem_ld16(tmem + lane_off + 16u * (2u * i + half), v[i]);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; i++) {
+                    const uint32_t q = 2u * i + half;
+                    if (valid && q < K0 / 16u) {
                         uint32_t w[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++)
-                            w[c] = Pr::pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
+                            w[c] = Pr::pack(__uint_as_float(v[i][2 * c]), __uint_as_float(v[i][2 * c + 1]));
                         dst[2u * q] = make_uint4(w[0], w[1], w[2], w[3]);
                         dst[2u * q + 1u] = make_uint4(w[4], w[5], w[6], w[7]);
                     }
@@ -742,15 +753,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
         }
         first_tile = false;
     }
+    if (ok && !first_tile) { // the last weight-gradient MMAs
+        if (mma_warp && tc::elect_one())
+            tc::mma_commit(bar_end);
+        ok = issuer ? tc::mbar_wait(bar_end, 0u, a.wait_ns) : true;
+        ok = __syncthreads_and(ok);
+        tc::fence_after_sync();
+    }
     if (!ok) {
         // a wait ran out: record it, give copies and MMAs still in flight one more bounded wait
-        if (issuer) {
+        tc::copy_async_wait();
+        if (mma_warp && tc::elect_one()) {
             atomicOr(a.status, 1u);
-            for (uint32_t b = 0; b < 2u; b++)
-                if (load_pending[b])
-                    tc::mbar_wait(tc::smem_addr(&bars[1u + b]), ph_load[b]);
             if (mma_pending)
                 tc::mbar_wait(bar_mma, ph_mma);
+            tc::mma_commit(bar_end); // MMAs without a commit of their own
+            tc::mbar_wait(bar_end, 0u);
         }
     } else if (!first_tile) {
         // the CTA's weight gradients: lane m of the dW_j^T accumulator holds column m of dW_j
@@ -759,7 +777,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                 continue;
             const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
             float *g = a.grad + tc_param_off(j, K0);
-            for (uint32_t q = 0; q < nout / 16u; q++) {
+            for (uint32_t q = half; q < nout / 16u; q += 2u) {
                 uint32_t v[16];
                 tc::tmem_ld16(tmem + lane_off + a.wg_col[j] + 16u * q, v);
                 tc::tmem_wait_ld();
@@ -783,7 +801,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0u) {
+    if (mma_warp) {
         tc::fence_after_sync();
         tc::tmem_dealloc(tmem, kTcTmemCols);
     }
@@ -992,12 +1010,20 @@ bool plan_train_pass(uint32_t n_in, uint32_t H, uint32_t mask, bool emit, TrainT
     }
     // the weight-gradient MMAs read 128 columns of every X tile (rows past the matrix's input width
     // are ignored): a 64-column tile is always followed by at least 16 KB (the next tile or dZ)
-    a.dz_off = off;
+    a.dz_off[0] = a.dz_off[1] = off;
     off += kNeurons * kTcRows * 2u;
     a.dzo_off = off;
     off += kOutputsPadded * kTcRows * 2u;
     a.bar_off = off;
     off += 64u;
+    a.loss_off = off;
+    off += kTcRows * 4u;
+    // a second dZ tile where it fits (1,024-byte tiles first would not change what fits)
+    const uint32_t dz2 = (off + 127u) & ~127u;
+    if (dz2 + kNeurons * kTcRows * 2u <= kTcSmemLimit) {
+        a.dz_off[1] = dz2;
+        off = dz2 + kNeurons * kTcRows * 2u;
+    }
     uint32_t col = kTcAccCols;
     for (uint32_t j = 0; j <= H; j++) {
         if (!((mask >> j) & 1u))
@@ -1133,11 +1159,6 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
         e = cudaEventRecord(marks[1], s);
     if (e != cudaSuccess)
         return e;
-    TensorMapBytes mb;
-    if ((e = make_feature_map(features, n_in, n, &mb, false)) != cudaSuccess)
-        return e;
-    CUtensorMap fmap;
-    std::memcpy(&fmap, mb.bytes, sizeof(fmap));
     auto kernel = bf16 ? k_train_tc<true, false> : (fp8 ? k_train_tc<false, true> : k_train_tc<false, false>);
     if ((e = allow_max_dynamic_smem(kernel)) != cudaSuccess)
         return e;
@@ -1145,6 +1166,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     const uint32_t blocks = tiles < (uint32_t)num_sms ? tiles : (uint32_t)num_sms;
     for (TrainTcPass &p : plan_train_passes(n_in, H)) {
         TrainTcArgs &a = p.a;
+        a.features = features;
         a.wpacked = wpacked;
         a.n_inputs = n_in;
         a.n_hidden_layers = H;
@@ -1158,7 +1180,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
         a.status = status;
         a.wait_ns = wait_ns ? wait_ns : tc::kWaitLimitNs;
         a.stall = stall ? 1u : 0u;
-        kernel<<<blocks, kTcThreads, p.smem, s>>>(fmap, a);
+        kernel<<<blocks, kTcThreads, p.smem, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return e;
     }

@@ -53,6 +53,18 @@ __device__ __forceinline__ void pack_weights(const __half *__restrict__ w, uint3
     }
 }
 
+// ---- asynchronous 16-byte copies ---------------------------------------------------------------
+
+// 16 bytes from global to shared memory; zeros instead when `valid` is false (src is not read)
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u)
+                 : "memory");
+}
+
+// waits for every copy this thread has issued
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 // ---- mbarrier ----------------------------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
@@ -144,6 +156,17 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 // Makes generic-proxy shared-memory writes visible to the tensor core (async proxy).
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
+// One lane of a fully converged warp (always the same one). MMAs are issued inside
+// `if (warp index, made uniform by a shuffle) if (elect_one())`: the compiler then keeps their
+// descriptors in uniform registers; in a branch on threadIdx alone it moves every operand of every MMA
+// over from vector registers.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0u;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, both K-major; issued by one thread.
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate)
@@ -163,6 +186,23 @@ __device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uin
                  " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
                  "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
                  : "memory");
+}
+
+// A chain of `count` MMAs over K in steps of 16 into one accumulator, `acc` for the first: the
+// descriptors are formed once and advance by a_step / b_step (16-byte units; operands lie below
+// 256 KB, so the address field does not carry). The issuing thread is alone in its warp and pays the
+// latency of every integer instruction between two MMAs: with both descriptors rebuilt for each, an
+// MMA took about 125 cycles to issue.
+__device__ __forceinline__ void mma_chain(uint32_t d_tmem, uint64_t a_desc, uint32_t a_step, uint64_t b_desc,
+                                          uint32_t b_step, uint32_t idesc, uint32_t count, uint32_t acc)
+{
+#pragma unroll 1
+    for (uint32_t k = 0; k < count; k++) {
+        mma_f16(d_tmem, a_desc, b_desc, idesc, acc);
+        a_desc += a_step;
+        b_desc += b_step;
+        acc = 1u;
+    }
 }
 
 // The mbarrier receives one arrival when every MMA issued so far by this thread has completed.
