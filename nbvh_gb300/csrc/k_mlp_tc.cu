@@ -58,8 +58,14 @@ __host__ __device__ inline uint32_t hidden_w_bytes() { return kNeurons * kNeuron
 __host__ __device__ inline uint32_t out_w_bytes() { return kOutputsPadded * kNeurons * 2u; }
 
 __global__ void k_pack_weights(const __half *__restrict__ w, uint32_t n_inputs, uint32_t n_hidden_layers,
-                               __half *__restrict__ packed)
+                               __half *__restrict__ packed, uint32_t *clear0, uint32_t *clear1)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { // words the kernels after this one add to
+        if (clear0)
+            *clear0 = 0u;
+        if (clear1)
+            *clear1 = 0u;
+    }
     tc::pack_weights(w, n_inputs, n_hidden_layers, packed, blockIdx.x * blockDim.x + threadIdx.x,
                      gridDim.x * blockDim.x);
 }
@@ -361,10 +367,10 @@ uint32_t packed_weight_bytes(uint32_t n_inputs, uint32_t n_hidden_layers)
 }
 
 cudaError_t launch_pack_weights(const __half *params_h, uint32_t n_inputs, uint32_t n_hidden_layers, __half *packed,
-                                cudaStream_t s)
+                                cudaStream_t s, uint32_t *clear0, uint32_t *clear1)
 {
     const uint32_t pieces = packed_weight_bytes(n_inputs, n_hidden_layers) / 16u;
-    k_pack_weights<<<(pieces + 127u) / 128u, 128, 0, s>>>(params_h, n_inputs, n_hidden_layers, packed);
+    k_pack_weights<<<(pieces + 127u) / 128u, 128, 0, s>>>(params_h, n_inputs, n_hidden_layers, packed, clear0, clear1);
     return cudaGetLastError();
 }
 

@@ -476,6 +476,7 @@ struct TrainTcArgs {
     LossConsts lc;
     __half *dfeat;        // n x n_inputs gradients of the encoded features (emit launches)
     float *grad;          // FP32 gradient vector (network matrices first)
+    float out_scale;      // factor of what is added to it
     float *loss_sum;
     float *sample_loss;   // per row: sum of its output channels' loss values (may be NULL)
     uint32_t *status;     // nonzero when a bounded wait gave up
@@ -784,7 +785,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                 if (tid < nin) {
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
-                        const float x = __uint_as_float(v[c]);
+                        const float x = __uint_as_float(v[c]) * a.out_scale;
                         if (x != 0.f)
                             atomicAdd(g + (size_t)(16u * q + (uint32_t)c) * nin + tid, x);
                     }
@@ -833,7 +834,7 @@ template <bool BF16, uint32_t F>
 __global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_constant__ GridParams grid,
                                                                  const float *__restrict__ positions,
                                                                  const __half *__restrict__ dfeat, uint32_t n,
-                                                                 float *__restrict__ grid_grad)
+                                                                 float *__restrict__ grid_grad, float out_scale)
 {
     constexpr uint32_t FT = kScatterFeatures<F>, parts = F / FT;
     const uint32_t P = grid.n_points, L = grid.n_levels;
@@ -876,8 +877,8 @@ __global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_c
 #pragma unroll
             for (uint32_t q = 0; q < FT / 2u; q++) {
                 const float2 v = MlpPrec<BF16>::unpack(__ldg(gw + q));
-                g[2u * q] = v.x;
-                g[2u * q + 1u] = v.y;
+                g[2u * q] = v.x * out_scale;
+                g[2u * q + 1u] = v.y * out_scale;
                 any |= v.x != 0.f || v.y != 0.f;
             }
             if (!any)
@@ -909,15 +910,15 @@ __global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_c
 
 template <bool BF16>
 cudaError_t scatter_rows(const GridParams &grid, const float *positions, const __half *dfeat, uint32_t n,
-                         float *grid_grad, cudaStream_t s)
+                         float *grid_grad, float out_scale, cudaStream_t s)
 {
     const unsigned blocks = (n + kScatterRows - 1u) / kScatterRows;
     if (grid.n_features == 4u)
-        k_grid_scatter<BF16, 4><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+        k_grid_scatter<BF16, 4><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
     else if (grid.n_features == 8u)
-        k_grid_scatter<BF16, 8><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+        k_grid_scatter<BF16, 8><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
     else
-        k_grid_scatter<BF16, 2><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad);
+        k_grid_scatter<BF16, 2><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
     return cudaGetLastError();
 }
 
@@ -1139,8 +1140,8 @@ cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, u
 
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
-                              __half *features, __half *dfeat, __half *wpacked, float *grad, float *loss_sum,
-                              float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
+                              __half *features, __half *dfeat, __half *wpacked, float *grad, float out_scale,
+                              float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
                               uint64_t wait_ns, bool stall, const cudaEvent_t *marks)
 {
     if (n == 0)
@@ -1154,7 +1155,8 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     const uint32_t *table = reinterpret_cast<const uint32_t *>(params_h + n_network_params);
     e = encode_rows(grid, table, positions, n, features, bf16, num_sms, s);
     if (e == cudaSuccess)
-        e = launch_pack_weights(params_h, n_in, H, wpacked, s);
+        e = launch_pack_weights(params_h, n_in, H, wpacked, s, clear ? status : nullptr,
+                                clear ? reinterpret_cast<uint32_t *>(loss_sum) : nullptr);
     if (e == cudaSuccess && marks)
         e = cudaEventRecord(marks[1], s);
     if (e != cudaSuccess)
@@ -1175,6 +1177,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
         a.lc = lc;
         a.dfeat = dfeat;
         a.grad = grad;
+        a.out_scale = out_scale;
         a.loss_sum = loss_sum;
         a.sample_loss = sample_loss;
         a.status = status;
@@ -1186,8 +1189,8 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     }
     if (marks && (e = cudaEventRecord(marks[2], s)) != cudaSuccess)
         return e;
-    e = bf16 ? scatter_rows<true>(grid, positions, dfeat, n, grad + n_network_params, s)
-             : scatter_rows<false>(grid, positions, dfeat, n, grad + n_network_params, s);
+    e = bf16 ? scatter_rows<true>(grid, positions, dfeat, n, grad + n_network_params, out_scale, s)
+             : scatter_rows<false>(grid, positions, dfeat, n, grad + n_network_params, out_scale, s);
     if (e == cudaSuccess && marks)
         e = cudaEventRecord(marks[3], s);
     return e;

@@ -741,6 +741,8 @@ nbvh_status nbvh_destroy(nbvh_handle *h)
     for (int k = 0; k < 2; k++)
         if (h->ev_drain[k])
             cudaEventDestroy(h->ev_drain[k]);
+    if (h->h_readback)
+        cudaFreeHost(h->h_readback);
     delete h;
     return NBVH_OK;
 }
@@ -1319,6 +1321,30 @@ nbvh_status nbvh_export_tcnn_weights(nbvh_handle *h, const char *path)
     });
 }
 
+} // extern "C"
+
+namespace {
+
+// Reads the kernels' status word (and the loss) back through page-locked words and waits for the
+// stream: a copy to pageable memory is staged by the host, about 10 us each.
+uint32_t read_back(nbvh_handle *h, cudaStream_t s, const float *d_loss = nullptr, float *loss = nullptr)
+{
+    if (!h->h_readback)
+        cuda_check(cudaHostAlloc(reinterpret_cast<void **>(&h->h_readback), 2u * sizeof(uint32_t), cudaHostAllocDefault),
+                   "pinned status");
+    cuda_check(cudaMemcpyAsync(h->h_readback, h->d_status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "status");
+    if (d_loss)
+        cuda_check(cudaMemcpyAsync(h->h_readback + 1, d_loss, sizeof(float), cudaMemcpyDeviceToHost, s), "loss");
+    cuda_check(cudaStreamSynchronize(s), "sync");
+    if (d_loss)
+        std::memcpy(loss, h->h_readback + 1, sizeof(float));
+    return h->h_readback[0];
+}
+
+} // namespace
+
+extern "C" {
+
 nbvh_status nbvh_network_inference(nbvh_handle *h, const float *d_positions, uint32_t n, float *d_outputs,
                                    nbvh_stream stream)
 {
@@ -1339,20 +1365,17 @@ nbvh_status nbvh_network_inference(nbvh_handle *h, const float *d_positions, uin
             cuda_check(h->d_status.resize(1u), "alloc status");
         TensorMapBytes map;
         cuda_check(make_feature_map(h->d_infer_feat.ptr, ni, n, &map), "feature map");
-        cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
         cuda_check(cudaEventRecord(h->ev0, s), "event");
         cuda_check(launch_encode_rows(h->d_params_h.ptr, h->grid, H, d_positions, n, h->d_infer_feat.ptr, mlp_bf16(h),
                                       h->num_sms, s),
                    "encode");
-        cuda_check(launch_pack_weights(h->d_params_h.ptr, ni, H, h->d_wpacked.ptr, s), "pack weights");
+        cuda_check(launch_pack_weights(h->d_params_h.ptr, ni, H, h->d_wpacked.ptr, s, h->d_status.ptr), "pack weights");
         cuda_check(launch_mlp_tc(map, h->d_wpacked.ptr, ni, H, n, nullptr, d_outputs, h->d_status.ptr, mlp_prec(h),
                                  h->num_sms, s, true, h->wait_limit_ns, h->debug_stall),
                    "tensor-core MLP");
         cuda_check(cudaEventRecord(h->ev1, s), "event");
         h->last_launches = 3;
-        uint32_t status = 0;
-        cuda_check(cudaMemcpyAsync(&status, h->d_status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "status");
-        cuda_check(cudaStreamSynchronize(s), "sync");
+        const uint32_t status = read_back(h, s);
         require((status & 2u) == 0u, NBVH_EDEVICE, "tensor-core MLP: shared memory not 1,024-byte aligned");
         require(status == 0u, NBVH_ETIMEOUT, "tensor-core MLP: a bounded wait gave up");
     });
@@ -1372,8 +1395,7 @@ nbvh_status nbvh_mlp_inference(nbvh_handle *h, const uint16_t *d_features, uint3
             cuda_check(h->d_wpacked.resize(wb / 2u), "alloc packed weights");
         if (h->d_status.count < 1u)
             cuda_check(h->d_status.resize(1u), "alloc status");
-        cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
-        cuda_check(launch_pack_weights(h->d_params_h.ptr, ni, H, h->d_wpacked.ptr, s), "pack weights");
+        cuda_check(launch_pack_weights(h->d_params_h.ptr, ni, H, h->d_wpacked.ptr, s, h->d_status.ptr), "pack weights");
         if (n == 0)
             return;
         TensorMapBytes map;
@@ -1384,9 +1406,7 @@ nbvh_status nbvh_mlp_inference(nbvh_handle *h, const uint16_t *d_features, uint3
                    "tensor-core MLP");
         cuda_check(cudaEventRecord(h->ev1, s), "event");
         h->last_launches = 2;
-        uint32_t status = 0;
-        cuda_check(cudaMemcpyAsync(&status, h->d_status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "status");
-        cuda_check(cudaStreamSynchronize(s), "sync");
+        const uint32_t status = read_back(h, s);
         require((status & 2u) == 0u, NBVH_EDEVICE, "tensor-core MLP: shared memory not 1,024-byte aligned");
         require(status == 0u, NBVH_ETIMEOUT, "tensor-core MLP: a bounded wait gave up");
     });
@@ -1425,19 +1445,32 @@ TrainCull train_cull(const nbvh_handle *h)
     return c;
 }
 
-// forward + loss + backward of one batch into h->d_grad (scaled by the loss scale) and loss_sum
-void gradients_into_workspace(nbvh_handle *h, const float *d_pos, const float *d_tgt, uint32_t n, cudaStream_t s,
-                              float *loss_slot, const cudaEvent_t *marks = nullptr)
+// forward + loss + backward of one batch: the gradient times the loss scale times out_scale into grad,
+// the loss into *loss_slot (added; `clear`: it and the status word start from zero)
+void batch_gradients(nbvh_handle *h, const float *d_pos, const float *d_tgt, uint32_t n, cudaStream_t s, float *grad,
+                     float out_scale, float *loss_slot, bool clear, const cudaEvent_t *marks = nullptr)
 {
     ensure_train_workspace(h, n);
     const uint32_t H = (uint32_t)h->cfg.network.n_hidden_layers;
-    cuda_check(cudaMemsetAsync(h->d_grad.ptr, 0, (size_t)h->layout.n_params * sizeof(float), s), "zero grad");
+    cuda_check(cudaMemsetAsync(grad, 0, (size_t)h->layout.n_params * sizeof(float), s), "zero grad");
     cuda_check(launch_train_step(h->d_params_h.ptr, h->grid, H, make_loss_consts(h->cfg, n), d_pos, d_tgt, n,
-                                 h->d_train_feat.ptr, h->d_train_dfeat.ptr, h->d_train_wpacked.ptr, h->d_grad.ptr,
-                                 loss_slot, h->d_train_loss.ptr, h->d_status.ptr, mlp_bf16(h),
+                                 h->d_train_feat.ptr, h->d_train_dfeat.ptr, h->d_train_wpacked.ptr, grad, out_scale,
+                                 loss_slot, clear, h->d_train_loss.ptr, h->d_status.ptr, mlp_bf16(h),
                                  h->cfg.network.precision == NBVH_PRECISION_FP8, h->num_sms, s, h->wait_limit_ns,
                                  h->debug_stall, marks),
                "forward/backward");
+}
+
+// Whether the kernels may add the gradient straight into the caller's buffer: it holds 16-byte
+// atomics, and none of the inputs it would overwrite while they are read.
+bool direct_gradients(const nbvh_handle *h, const float *grad, const float *pos, const float *tgt, uint32_t n)
+{
+    const uintptr_t g0 = reinterpret_cast<uintptr_t>(grad), g1 = g0 + (size_t)h->layout.n_params * sizeof(float);
+    auto apart = [&](const float *p, size_t count) {
+        const uintptr_t p0 = reinterpret_cast<uintptr_t>(p);
+        return p0 + count * sizeof(float) <= g0 || p0 >= g1;
+    };
+    return g0 % 16u == 0u && apart(pos, (size_t)n * h->grid.n_points * 3u) && apart(tgt, (size_t)n * 8u);
 }
 
 } // namespace
@@ -1451,18 +1484,22 @@ nbvh_status nbvh_compute_gradients(nbvh_handle *h, const float *d_positions, con
         require(d_positions && d_targets && d_gradients && n > 0, NBVH_EINVAL, "null buffers");
         cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
         ensure_train_workspace(h, n);
-        cuda_check(cudaMemsetAsync(h->d_loss_sum.ptr, 0, sizeof(float), s), "zero loss");
-        cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
-        gradients_into_workspace(h, d_positions, d_targets, n, s, h->d_loss_sum.ptr);
-        cuda_check(cudaMemcpyAsync(d_gradients, h->d_grad.ptr, (size_t)h->layout.n_params * sizeof(float),
-                                   cudaMemcpyDeviceToDevice, s),
-                   "copy grad");
-        cuda_check(launch_scale(d_gradients, h->layout.n_params, 1.0f / h->cfg.optimizer.loss_scale, s), "unscale");
+        // straight into the caller's buffer where it allows that, without the loss scale where taking it
+        // out of every addend is exact (a power of two); else through the workspace, or one more pass
+        const float scale = h->cfg.optimizer.loss_scale;
+        const bool direct = direct_gradients(h, d_gradients, d_positions, d_targets, n);
+        int exponent = 0;
+        const bool fold = direct && std::frexp(scale, &exponent) == 0.5f;
+        batch_gradients(h, d_positions, d_targets, n, s, direct ? d_gradients : h->d_grad.ptr, fold ? 1.0f / scale : 1.0f,
+                        h->d_loss_sum.ptr, true);
+        if (!direct)
+            cuda_check(cudaMemcpyAsync(d_gradients, h->d_grad.ptr, (size_t)h->layout.n_params * sizeof(float),
+                                       cudaMemcpyDeviceToDevice, s),
+                       "copy grad");
+        if (!fold)
+            cuda_check(launch_scale(d_gradients, h->layout.n_params, 1.0f / scale, s), "unscale");
         float loss = 0.f;
-        uint32_t status = 0;
-        cuda_check(cudaMemcpyAsync(&loss, h->d_loss_sum.ptr, sizeof(float), cudaMemcpyDeviceToHost, s), "loss");
-        cuda_check(cudaMemcpyAsync(&status, h->d_status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "status");
-        cuda_check(cudaStreamSynchronize(s), "sync");
+        const uint32_t status = read_back(h, s, h->d_loss_sum.ptr, &loss);
         require(status == 0u, NBVH_ETIMEOUT, "tensor-core training kernel: a bounded wait gave up");
         if (h_loss)
             *h_loss = loss;
@@ -1534,8 +1571,8 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
                                                h->d_train_nodes.ptr, learned_lod, &survival, h->d_sample_state.ptr,
                                                h->classic_fast_div, train_cull(h), h->num_sms, s),
                        "training samples");
-            gradients_into_workspace(h, h->d_train_pos.ptr, h->d_train_tgt.ptr, n, s, h->d_loss_sum.ptr + i,
-                                     prof ? h->kprof->train_ev + 1 : nullptr);
+            batch_gradients(h, h->d_train_pos.ptr, h->d_train_tgt.ptr, n, s, h->d_grad.ptr, 1.0f,
+                            h->d_loss_sum.ptr + i, false, prof ? h->kprof->train_ev + 1 : nullptr);
             lr_t = adam_step_size(c, h->training_step);
             cuda_check(launch_adam(h->d_params.ptr, h->d_params_h.ptr, h->d_adam_m.ptr, h->d_adam_v.ptr, h->d_grad.ptr,
                                    h->layout.n_params, lr_t, c.optimizer.beta1, c.optimizer.beta2, c.optimizer.epsilon,

@@ -349,6 +349,7 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<__half> d_wpacked;  // network matrices in the tensor-core operand layout
     nbvh::DeviceBuffer<__half> d_infer_feat; // feature rows of nbvh_network_inference
     nbvh::DeviceBuffer<uint32_t> d_status; // error word of kernels with bounded waits
+    uint32_t *h_readback = nullptr; // two page-locked words a call reads its status and loss back into
     nbvh::DeviceBuffer<float> d_adam_m, d_adam_v;
     nbvh::DeviceBuffer<float> d_grad;
     uint32_t training_step = 0;
@@ -583,8 +584,9 @@ cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, u
 // wait inside the kernel gave up. configure = false skips setting the kernel's shared-memory
 // attribute (during stream capture, after an earlier launch set it).
 uint32_t packed_weight_bytes(uint32_t n_inputs, uint32_t n_hidden_layers);
+// (clear0, clear1: words the launch zeroes as well, NULL for none)
 cudaError_t launch_pack_weights(const __half *params_h, uint32_t n_inputs, uint32_t n_hidden_layers, __half *packed,
-                                cudaStream_t s);
+                                cudaStream_t s, uint32_t *clear0 = nullptr, uint32_t *clear1 = nullptr);
 // allow_swizzle = false: always 8-value boxes, so that a 128-row tile lands in shared memory in
 // the unswizzled K-major core-matrix layout (column block c of 8 values at c * 2,048 bytes).
 cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t rows, TensorMapBytes *out,
@@ -657,12 +659,13 @@ cudaError_t launch_training_samples(const float4 *neural_nodes, const float4 *no
 // (packed_weight_bytes), forward + composite loss + backward on the tcgen05 tensor cores (the
 // weight gradients added to grad, the loss sum into *loss_sum, per-row losses into sample_loss
 // when not NULL, the 16-bit feature gradients into dfeat, n x n_inputs), then the hash-grid
-// gradient scattered into grad + n_network_params. grad holds the gradient times the loss scale.
+// gradient scattered into grad + n_network_params. grad (16-byte aligned) receives the gradient
+// times the loss scale times out_scale; with `clear` the loss sum and the status start from zero.
 // status receives a nonzero word if a bounded wait inside the tensor-core kernel gave up.
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
-                              __half *features, __half *dfeat, __half *wpacked, float *grad, float *loss_sum,
-                              float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
+                              __half *features, __half *dfeat, __half *wpacked, float *grad, float out_scale,
+                              float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
                               uint64_t wait_ns = 0, bool stall = false, const cudaEvent_t *marks = nullptr);
 // (marks, when given: 4 events recorded before the encoding, before and after the tensor-core
 // passes, and after the grid scatter)

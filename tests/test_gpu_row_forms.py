@@ -63,3 +63,30 @@ def test_gradients_of_merged_points(built, oracle, grid, n):
                                              h.layout.n_params, loss_scale=h.cfg.optimizer.loss_scale)
         assert abs(loss - rloss) <= 1e-3 * abs(rloss) + 1e-6
         check_gradients(oracle, h, p, pos, tgt, g.cpu().numpy().astype(np.float64), rg.astype(np.float64), 2e-2)
+
+
+@pytest.mark.parametrize("scale", [128.0, 100.0])
+def test_gradient_buffers_and_loss_scales(built, oracle, scale):
+    """A buffer the kernels can add into, one off 16 bytes and one that holds the targets get the same
+    gradient up to the order of its float additions; a loss scale that is no power of two as well."""
+    h0, p = _handle((4, 16, 2))
+    h0.close()
+    h0.cfg.optimizer.loss_scale = scale
+    with nb.NBVH(h0.cfg) as h:
+        h.set_params(p)
+        n = 700
+        pos, rng = _rows(n, 4, 8), np.random.default_rng(8)
+        tgt = rng.random((n, 8)).astype(np.float32)
+        d_pos, d_tgt = torch.from_numpy(pos).cuda(), torch.from_numpy(tgt).cuda()
+        g, loss = h.compute_gradients(d_pos, d_tgt)
+        rg, _ = oracle.compute_gradients(oracle.network(h.cfg, h.layout, p), oracle.loss_consts(h.cfg), pos, tgt,
+                                         h.layout.n_params, loss_scale=scale)
+        check_gradients(oracle, h, p, pos, tgt, g.cpu().numpy().astype(np.float64), rg.astype(np.float64), 2e-2)
+        big = torch.zeros(h.layout.n_params + 1, device="cuda")
+        for off, targets in ((1, d_tgt), (0, big[:n * 8])):
+            if targets is not d_tgt:
+                targets.copy_(d_tgt.view(-1))
+            assert h.lib.nbvh_compute_gradients(h.h, nb._ptr(d_pos), nb._ptr(targets), n, nb._ptr(big[off:]), None,
+                                                nb._stream(None)) == 0
+            # addends of one sign scale, thousands of them at most: far below 1e-4 of the largest
+            assert (big[off:off + g.numel()] - g).abs().max() <= 1e-4 * g.abs().max()
