@@ -84,8 +84,73 @@ __global__ void __launch_bounds__(128) k_encode(const __grid_constant__ GridPara
     }
 }
 
+// One thread per (cell, corner) of the cell copy: the corner's entry, copied bit for bit.
+template <typename T>
+__global__ void __launch_bounds__(256) k_build_cells(const __grid_constant__ GridParams grid,
+                                                     const __grid_constant__ CellParams cp,
+                                                     const T *__restrict__ table, T *__restrict__ cells,
+                                                     uint32_t n_cells)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, ci = i >> 3;
+    if (ci >= n_cells)
+        return;
+    uint32_t l = cp.n_levels - 1u;
+    while (ci < cp.offset[l])
+        l--;
+    const uint32_t n = cp.dim[l], k = ci - cp.offset[l];
+    const LevelCell q = {k % n, k / n % n, k / n / n, 0.f, 0.f, 0.f};
+    cells[i] = __ldg(table + grid.offset[l] +
+                     level_corner_index(grid.hashed[l] != 0u, grid.res[l], grid.size[l], q, i & 7u));
+}
 
 } // namespace
+
+size_t plan_cells(const GridParams &grid, CellParams &cp)
+{
+    cp = CellParams{};
+    size_t total = 0;
+    uint32_t l = 0;
+    for (; l < grid.n_levels; l++) {
+        // cells that positions in [0, 1] reach: floor(scale + 0.5) is the last one
+        const float last = floorf(grid.scale[l] + 0.5f);
+        cp.offset[l] = (uint32_t)total;
+        if (!(last >= 0.f && last < 1024.f))
+            break;
+        const size_t n = (size_t)last + 1u;
+        if ((total + n * n * n) * 16u * grid.n_features > kCellBytes)
+            break;
+        cp.dim[l] = (uint32_t)n;
+        total += n * n * n;
+    }
+    if (grid.n_features == 2u && (l & 3u) != 0u) { // 2-feature encoders take the levels four at a time
+        l &= ~3u;
+        total = cp.offset[l];
+    }
+    cp.n_levels = l;
+    return total;
+}
+
+cudaError_t launch_build_cells(const __half *params_h, const GridParams &grid, const CellParams &cp,
+                               uint32_t n_hidden_layers, uint4 *cells, cudaStream_t s)
+{
+    if (cp.n_levels == 0u)
+        return cudaSuccess;
+    const uint32_t n_network_params = kNeurons * grid.n_inputs + (n_hidden_layers - 1u) * kNeurons * kNeurons +
+                                      kOutputsPadded * kNeurons;
+    const __half *table = params_h + n_network_params;
+    const uint32_t last = cp.n_levels - 1u, n = cp.dim[last];
+    const uint32_t n_cells = cp.offset[last] + n * n * n; // at most kCellBytes / 32
+    const unsigned blocks = (n_cells * 8u + 255u) / 256u;
+    if (grid.n_features == 4u)
+        k_build_cells<<<blocks, 256, 0, s>>>(grid, cp, reinterpret_cast<const uint2 *>(table),
+                                             reinterpret_cast<uint2 *>(cells), n_cells);
+    else if (grid.n_features == 8u)
+        k_build_cells<<<blocks, 256, 0, s>>>(grid, cp, reinterpret_cast<const uint4 *>(table), cells, n_cells);
+    else
+        k_build_cells<<<blocks, 256, 0, s>>>(grid, cp, reinterpret_cast<const uint32_t *>(table),
+                                             reinterpret_cast<uint32_t *>(cells), n_cells);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_segments(const float4 *dilated_nodes, const float4 *bounds, const NeuralConsts &nc,
                             const nbvh_ray *rays, uint32_t n, uint32_t max_segments, nbvh_segment *segs,

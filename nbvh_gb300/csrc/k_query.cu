@@ -64,7 +64,7 @@ constexpr uint32_t kEncodeBlocksPerSm = 4;
 // step 3 on whatever the batch.
 __host__ __device__ constexpr uint32_t tail_step(uint32_t n_cut_nodes, uint32_t n)
 {
-    const uint32_t step = n <= (1u << 14) ? 0u : n <= (1u << 17) ? 2u : n <= (1u << 19) ? 3u : n <= (1u << 20) ? 4u : 5u;
+    const uint32_t step = n <= kTailOnlyRays ? 0u : n <= (1u << 17) ? 2u : n <= (1u << 19) ? 3u : n <= (1u << 20) ? 4u : 5u;
     return n_cut_nodes > kMaxSortNodes && step > 3u ? 3u : step;
 }
 constexpr uint32_t kTailWarps = 8;
@@ -81,6 +81,8 @@ struct WaveArgs {
     const float4 *bounds; // union of dilated leaf boxes per node
     const uint8_t *non_neural;
     const uint32_t *table;
+    const uint4 *cells;    // cell copy of the grid's coarse levels
+    CellParams cp;         // which levels those are (none without a copy)
     const __half *weights; // 16-bit network matrices (network-first parameter layout)
     const nbvh_ray *rays;
     nbvh_neural_hit *hits;
@@ -478,6 +480,13 @@ __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_co
 // negative mint, then encoded into the dilated scene box. The point is computed once for all its
 // levels, so the kernel's instructions go to the gathers and their interpolation; it holds no
 // MLP state; its 4 blocks of 256 threads per SM keep many gathers in flight to hide their latency.
+// The L1 bounds it: it looks up one cache line per cycle, and a (point, level) of the table costs 6
+// lookups (4 pairs of x corners, half of them split). Levels in the cell copy cost one 32-byte read:
+// 1,453 -> 1,250 us per 2^22-ray query with the copy of the 8 coarsest levels (192 MB; dense levels
+// alone, 11 MB: 1,390; 9 levels, 520 MB: no more), 489 -> 455 for 2^20 rays with 4 of the reference's 8
+// levels. Reading the quad of entries where both corners lie in it was slower (1,435 us: the warp then
+// issues three kinds of load). The tail kernel reads the table alone: its lanes hold different levels,
+// and both paths in it cost more registers than the copy saved.
 
 template <uint32_t F>
 __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
@@ -488,6 +497,13 @@ __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
         const uint32_t *src = reinterpret_cast<const uint32_t *>(&a.grid);
         uint32_t *dst = reinterpret_cast<uint32_t *>(&gp);
         for (uint32_t i = threadIdx.x; i < sizeof(GridParams) / 4u; i += blockDim.x)
+            dst[i] = src[i];
+    }
+    __shared__ CellParams cp;
+    {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(&a.cp);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(&cp);
+        for (uint32_t i = threadIdx.x; i < sizeof(CellParams) / 4u; i += blockDim.x)
             dst[i] = src[i];
     }
     __syncthreads();
@@ -551,14 +567,27 @@ __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
             if (vec_store) {
                 for (uint32_t l = lg * LG; l < lg * LG + LG; l += 4u) {
                     uint4 q;
-                    float2 f = encode_level<true>(a.table, gp, l, pos);
-                    q.x = pack16(f.x, f.y);
-                    f = encode_level<true>(a.table, gp, l + 1u, pos);
-                    q.y = pack16(f.x, f.y);
-                    f = encode_level<true>(a.table, gp, l + 2u, pos);
-                    q.z = pack16(f.x, f.y);
-                    f = encode_level<true>(a.table, gp, l + 3u, pos);
-                    q.w = pack16(f.x, f.y);
+                    float2 f[2];
+                    bool two = false;
+                    // four levels per store, two at a time from the cell copy where they are in it (the copy
+                    // holds a multiple of four levels)
+                    if (l < cp.n_levels)
+                        two = encode_cells<2>(a.cells, cp, gp, l, pos, f);
+                    if (!two) {
+                        f[0] = encode_level<true>(a.table, gp, l, pos);
+                        f[1] = encode_level<true>(a.table, gp, l + 1u, pos);
+                    }
+                    q.x = pack16(f[0].x, f[0].y);
+                    q.y = pack16(f[1].x, f[1].y);
+                    two = false;
+                    if (l < cp.n_levels)
+                        two = encode_cells<2>(a.cells, cp, gp, l + 2u, pos, f);
+                    if (!two) {
+                        f[0] = encode_level<true>(a.table, gp, l + 2u, pos);
+                        f[1] = encode_level<true>(a.table, gp, l + 3u, pos);
+                    }
+                    q.z = pack16(f[0].x, f[0].y);
+                    q.w = pack16(f[1].x, f[1].y);
                     *reinterpret_cast<uint4 *>(dst + l) = q;
                 }
             } else {
@@ -571,7 +600,8 @@ __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
             // F = 4: 8 bytes per level; F = 8: 16 bytes per level (always aligned to its size)
             for (uint32_t l = lg * LG; l < lg * LG + LG; l++) {
                 float f[F];
-                encode_level_wide<F>(a.table, gp, l, pos, f);
+                if (l >= cp.n_levels || !encode_cell_wide<F>(a.cells, cp, gp, l, pos, f))
+                    encode_level_wide<F>(a.table, gp, l, pos, f);
                 if constexpr (F == 4u)
                     *reinterpret_cast<uint2 *>(dst + 2u * l) = make_uint2(pack16(f[0], f[1]), pack16(f[2], f[3]));
                 else
@@ -1488,6 +1518,8 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     const uint32_t n_network_params =
         kNeurons * grid.n_inputs + (n_hidden_layers - 1u) * kNeurons * kNeurons + kOutputsPadded * kNeurons;
     a.table = reinterpret_cast<const uint32_t *>(params_h + n_network_params);
+    a.cells = res.cells;
+    a.cp = res.cells ? res.cell_levels : CellParams{};
     a.weights = params_h;
     a.rays = rays;
     a.hits = hits;

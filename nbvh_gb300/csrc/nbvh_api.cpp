@@ -421,9 +421,16 @@ ParamPrecision param_precision(const nbvh_handle *h)
     return pp;
 }
 
+void params_changed(nbvh_handle *h)
+{
+    h->cells_fresh = false;
+    h->cells_rays = 0;
+}
+
 void upload_params(nbvh_handle *h, const float *params, bool reset_adam)
 {
     const uint32_t n = h->layout.n_params;
+    params_changed(h);
     cuda_check(h->d_params.resize(n), "alloc params");
     cuda_check(h->d_params_h.resize(n), "alloc fp16 params");
     cuda_check(cudaMemcpy(h->d_params.ptr, params, (size_t)n * sizeof(float), cudaMemcpyHostToDevice), "upload params");
@@ -480,11 +487,12 @@ void ensure_train_workspace(nbvh_handle *h, uint32_t n)
         cuda_check(h->d_grad.resize(h->layout.n_params), "alloc grad");
 }
 
-void ensure_query_workspace(nbvh_handle *h, uint32_t n, int ctx)
+void ensure_query_workspace(nbvh_handle *h, uint32_t n, int ctx, cudaStream_t s)
 {
     if (h->d_counters.count < 3u)
         cuda_check(h->d_counters.resize(3u), "alloc counters");
     grow_query_context(h, h->qctx[ctx], n);
+    ensure_cells(h, s, n);
 }
 
 // The neural query on the given stream with the given context's buffers (the handle's own
@@ -508,7 +516,7 @@ void neural_query(nbvh_handle *h, const nbvh_ray *d_rays, uint32_t n, uint32_t d
         h->last_rays = 0;
         return;
     }
-    ensure_query_workspace(h, n, ctx);
+    ensure_query_workspace(h, n, ctx, s);
     if (timed)
         cuda_check(cudaEventRecord(h->ev0, s), "event");
     h->last_launches = run_neural_query(h, h->qctx[ctx], h->d_counters.ptr + ctx, d_rays, n, depth, vis_only, d_hits, s);
@@ -574,6 +582,9 @@ void neural_query_noalloc(nbvh_handle *h, const nbvh_ray *d_rays, uint32_t n, ui
         res.stall = h->debug_stall;
         res.sort_key = h->n_sort_bins ? h->d_sort_key.ptr : nullptr;
         res.n_sort_bins = h->n_sort_bins;
+        ensure_cells(h, s, n, false);
+        res.cells = h->cells_fresh ? h->d_cells.ptr : nullptr;
+        res.cell_levels = h->cell_levels;
         cuda_check(make_feature_map(sc.features, h->layout.n_inputs, (uint32_t)kNoallocRays, &res.feature_map),
                    "feature map");
         cuda_check(launch_wave_query(h->d_neural_dilated.ptr, h->d_neural_bounds.ptr,
@@ -711,6 +722,7 @@ nbvh_status nbvh_create(const nbvh_config *cfg, int device, nbvh_handle **out)
         cuda_check(h->d_loss_sum.resize(1u), "alloc loss");
         compute_layout(h->cfg, h->layout, h->grid);
         apply_device_level_scales(h->cfg, h->layout, h->grid);
+        h->n_cells = plan_cells(h->grid, h->cell_levels);
         std::vector<float> p(h->layout.n_params);
         init_params(h->cfg, h->layout, p.data());
         upload_params(h, p.data(), true);
@@ -741,6 +753,8 @@ nbvh_status nbvh_destroy(nbvh_handle *h)
     for (int k = 0; k < 2; k++)
         if (h->ev_drain[k])
             cudaEventDestroy(h->ev_drain[k]);
+    if (h->ev_params)
+        cudaEventDestroy(h->ev_params);
     if (h->h_readback)
         cudaFreeHost(h->h_readback);
     delete h;
@@ -1180,7 +1194,7 @@ bool zero_copy_neural(nbvh_handle *h, const nbvh_ray *h_rays, uint32_t n, uint32
     reserve_stat_chunks(h, n, chunk);
     for (uint32_t c0 = 0, ci = 0; c0 < n; c0 += chunk, ci++) {
         const uint32_t cnt = (n - c0) < chunk ? (n - c0) : chunk;
-        ensure_query_workspace(h, cnt, 1);
+        ensure_query_workspace(h, cnt, 1, s);
         if (h->d_drain_hits.count < cnt)
             cuda_check(h->d_drain_hits.resize(cnt), "alloc records");
         if (h->d_late.count < (size_t)cnt + 1u)
@@ -1512,11 +1526,21 @@ nbvh_status nbvh_adam_step(nbvh_handle *h, const float *d_gradients, nbvh_stream
     return guarded(h, [&]() {
         require(d_gradients != nullptr, NBVH_EINVAL, "null gradient");
         const nbvh_config &c = h->cfg;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &capture), "capture status");
+        params_changed(h);
+        if (capture != cudaStreamCaptureStatusNone)
+            h->cells_off = true; // replays will change the parameters unseen
         cuda_check(launch_adam(h->d_params.ptr, h->d_params_h.ptr, h->d_adam_m.ptr, h->d_adam_v.ptr, d_gradients,
                                h->layout.n_params, adam_step_size(c, h->training_step), c.optimizer.beta1,
                                c.optimizer.beta2, c.optimizer.epsilon, c.optimizer.l2_reg, 1.0f, param_precision(h),
                                reinterpret_cast<cudaStream_t>(stream)),
                    "adam");
+        if (!h->cells_off) { // the cell copy is built after this step, whatever stream builds it
+            if (!h->ev_params)
+                cuda_check(cudaEventCreateWithFlags(&h->ev_params, cudaEventDisableTiming), "event");
+            cuda_check(cudaEventRecord(h->ev_params, reinterpret_cast<cudaStream_t>(stream)), "event");
+        }
         h->training_step++;
         h->last_launches = 1;
     });
@@ -1552,6 +1576,7 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
         cudaStream_t s = h->pipe_stream[0];
         cuda_check(cudaMemsetAsync(h->d_loss_sum.ptr, 0, ((size_t)steps + 1u) * sizeof(float), s), "zero loss");
         cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
+        params_changed(h);
         const NeuralConsts nc = make_neural_consts(h, 1u, false);
         const uint32_t first = h->training_step;
         float lr_t = 0.f;
@@ -1704,6 +1729,9 @@ nbvh_status nbvh_render_path(nbvh_handle *h, const nbvh_path_request *req, float
         if (h->d_counters.count < 3u)
             cuda_check(h->d_counters.resize(3u), "alloc counters");
         require(req != nullptr, NBVH_EINVAL, "null request");
+        const uint64_t paths = (uint64_t)req->camera.width * req->camera.height * req->spp;
+        ensure_cells(h, reinterpret_cast<cudaStream_t>(stream),
+                     paths < kCellsAfterRays ? (uint32_t)paths : kCellsAfterRays);
         const uint64_t traced = render_path_core(h, h->qctx[0], h->d_counters.ptr, h->path, req, d_image,
                                                  reinterpret_cast<cudaStream_t>(stream),
                                                  req->camera.sample_idx * req->spp);
@@ -1977,6 +2005,8 @@ nbvh_status nbvh_load(nbvh_handle *h, const char *path)
         h->cfg = cfg;
         h->layout = L;
         h->grid = g;
+        h->n_cells = plan_cells(h->grid, h->cell_levels);
+        params_changed(h);
         h->vertices.swap(verts);
         h->indices.swap(idx);
         h->albedo.swap(albedo);
@@ -2150,6 +2180,35 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
         q.generation++;
 }
 
+void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
+{
+    std::lock_guard<std::mutex> lock(h->cells_mu);
+    if (h->cells_fresh || h->cells_off || h->n_cells == 0u || !uses_cells(n))
+        return;
+    if (h->cells_rays + n < kCellsAfterRays) { // a program may train again before its next query
+        h->cells_rays += n;
+        return;
+    }
+    const size_t words = h->n_cells * h->layout.n_features_per_level;
+    if (h->d_cells.count < words) {
+        if (!may_allocate)
+            return;
+        h->model_version++; // captured graphs hold the address
+        if (h->d_cells.resize(words) != cudaSuccess) { // no room: the table alone serves the queries
+            cudaGetLastError();
+            h->cells_off = true;
+            return;
+        }
+    }
+    if (h->ev_params) // an Adam step on another stream may still be writing the parameters
+        cuda_check(cudaStreamWaitEvent(s, h->ev_params, 0), "wait for parameters");
+    cuda_check(launch_build_cells(h->d_params_h.ptr, h->grid, h->cell_levels, (uint32_t)h->cfg.network.n_hidden_layers,
+                                  h->d_cells.ptr, s),
+               "cell copy");
+    cuda_check(cudaStreamSynchronize(s), "sync");
+    h->cells_fresh = true;
+}
+
 // The neural query itself on explicit per-call buffers (context q, counters): reads only the
 // handle's scene, cut and parameters, so several contexts may run it at once on different
 // streams. Returns the number of kernels launched.
@@ -2189,6 +2248,8 @@ uint32_t run_neural_query(const nbvh_handle *h, QueryContext &q, QueryCounters *
     res.ev = q.ev;
     res.wait_ns = h->wait_limit_ns;
     res.stall = h->debug_stall;
+    res.cells = h->cells_fresh ? h->d_cells.ptr : nullptr;
+    res.cell_levels = h->cell_levels;
     if (tune) {
         res.visits_per_round = tune->visits_per_round;
         res.encode_blocks_per_sm = tune->encode_blocks_per_sm;

@@ -84,6 +84,15 @@ static_assert(sizeof(GridParams) % 16 == 0, "GridParams must keep 16-byte alignm
 // bytes a shared-memory copy of GridParams takes before the 16-byte aligned data that follows it
 constexpr size_t kGridParamsSmem = (sizeof(GridParams) + 15u) & ~size_t(15);
 
+// Levels of the grid's cell copy (launch_build_cells): the first n_levels ones, with their cells per
+// axis and first cell. Apart from GridParams: two blocks of the tail kernel fill an SM's shared
+// memory to within 200 bytes.
+struct CellParams {
+    uint32_t n_levels;
+    uint32_t dim[kMaxLevels];
+    uint32_t offset[kMaxLevels];
+};
+
 // Constants of the neural traversal and decode (NeuralBVHRendererConstants /
 // PathTracingOutputConstants subsets).
 struct NeuralConsts {
@@ -349,6 +358,15 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<__half> d_wpacked;  // network matrices in the tensor-core operand layout
     nbvh::DeviceBuffer<__half> d_infer_feat; // feature rows of nbvh_network_inference
     nbvh::DeviceBuffer<uint32_t> d_status; // error word of kernels with bounded waits
+    // cell copy of the coarse hash-grid levels, built for the first query after the parameters changed
+    nbvh::DeviceBuffer<uint4> d_cells;
+    nbvh::CellParams cell_levels{};
+    size_t n_cells = 0;       // cells of the layout (0: none)
+    bool cells_fresh = false; // d_cells holds the current parameters' entries
+    uint64_t cells_rays = 0;  // rays queried without it since the parameters changed
+    bool cells_off = false;   // never: no memory for it, or Adam steps captured into a graph
+    cudaEvent_t ev_params = nullptr; // after the last nbvh_adam_step, on its stream
+    std::mutex cells_mu;      // serving slots may find them stale at the same time
     uint32_t *h_readback = nullptr; // two page-locked words a call reads its status and loss back into
     nbvh::DeviceBuffer<float> d_adam_m, d_adam_v;
     nbvh::DeviceBuffer<float> d_grad;
@@ -513,6 +531,8 @@ struct StepResources {
     // read by the sort (nullptr: the sort recomputes the bins); may be the ray-order key buffer,
     // which is free once the first pass has taken the rays
     uint16_t *row_keys = nullptr;
+    const uint4 *cells = nullptr;  // cell copy of the coarse grid levels (nullptr: the table alone)
+    CellParams cell_levels{};
     bool stall = false;            // failure-path tests: the MLP kernels wait on a barrier nothing arrives at
 };
 
@@ -576,6 +596,18 @@ cudaError_t launch_segments(const float4 *dilated_nodes, const float4 *bounds, c
 cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                                const float *positions, uint32_t n, __half *features, bool bf16, int num_sms,
                                cudaStream_t s);
+
+constexpr uint32_t kTailOnlyRays = 1u << 14; // batches up to this size run the tail kernel alone (k_query.cu)
+
+// Cell copy of the coarse levels of a hash grid: for every cell of such a level the entries of its 8
+// corners side by side (corner c at c * F halves), so that a point's lookup on the level is one 16F-byte
+// read instead of 8 entries in 4 to 8 sectors. plan_cells picks the levels (as many of the coarsest as
+// kCellBytes holds) and returns the number of cells; launch_build_cells fills the copy from the
+// 16-bit parameters.
+constexpr size_t kCellBytes = (size_t)192 << 20;
+size_t plan_cells(const GridParams &grid, CellParams &cp);
+cudaError_t launch_build_cells(const __half *params_h, const GridParams &grid, const CellParams &cp,
+                               uint32_t n_hidden_layers, uint4 *cells, cudaStream_t s);
 
 // tcgen05 fully fused MLP (k_mlp_tc.cu): weights packed into the tensor-core operand layout, then
 // 128-row tiles of FP16 inputs (row-major [rows][n_inputs], 16-byte aligned) fed by TMA through
@@ -726,6 +758,14 @@ namespace nbvh {
 // Grows a query context to n rays for the handle's cut and network (allocates device and pinned
 // memory; no kernel runs).
 void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n);
+// Brings the handle's cell copy up to date on stream s for a query of n rays and waits for it; called
+// before the queries that may use it (one that finds it stale, or not allocated, reads the table
+// instead). It is built once kCellsAfterRays rays have been queried since the parameters changed:
+// building it takes 150 us, which it saves over 2 to 3 million rays (2^22: 2,880 -> 2,700 us, 2^18: 655
+// -> 620), and a program that trains between its frames never pays for it.
+constexpr uint32_t kCellsAfterRays = 1u << 21;
+constexpr bool uses_cells(uint32_t n) { return n > kTailOnlyRays; }
+void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate = true);
 
 // The neural query on explicit per-call buffers (context q, counters): reads only the handle's
 // scene, cut and parameters, so several contexts may run it at once on different streams.

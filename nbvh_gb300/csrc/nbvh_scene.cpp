@@ -190,6 +190,7 @@ void scene_query(nbvh_scene *sc, const nbvh_ray *d_rays, uint32_t n, uint32_t de
             continue;
         nbvh_handle *model = sc->groups[gi]->model;
         ModelContext &mc = context_of(sc, model, m);
+        ensure_cells(model, s, m);
         run_neural_query(model, mc.q, mc.counters.ptr, sc->obj_rays.ptr + start[gi], m, depth, false,
                          sc->obj_hits.ptr + start[gi], s);
     }

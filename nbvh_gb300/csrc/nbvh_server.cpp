@@ -241,6 +241,7 @@ void slot_query(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t n, uint3
                    "pad batch");
     const StepResources tune = tuning_of(m, bucket);
     nbvh_handle *h = m.h;
+    ensure_cells(h, sl.stream, kCellsAfterRays); // the model may have been trained since its last request
     // a model whose device arrays were reallocated since its graphs were captured (a new cut, a
     // grown learned cut, a new mesh) drops them; the context is resized for the new cut first
     auto ver = sl.model_versions.find(model_id);
@@ -643,6 +644,7 @@ nbvh_status nbvh_server_add_model(nbvh_server *srv, nbvh_handle *h, uint32_t *mo
                 sl->graphs.clear();
             }
         }
+        ensure_cells(h, srv->slots[0]->stream, kCellsAfterRays);
         if (srv->cfg.autotune) {
             autotune(srv, id);
         } else { // one direct query sets the kernels' attributes before any capture

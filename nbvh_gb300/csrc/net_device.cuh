@@ -294,6 +294,124 @@ __device__ __forceinline__ void encode_level_wide(const void *__restrict__ table
     }
 }
 
+// A point's cell at one level (its lowest corner's grid coordinates) and position inside it.
+struct LevelCell {
+    uint32_t gx, gy, gz;
+    float rx, ry, rz;
+};
+__device__ __forceinline__ LevelCell level_cell(const GridParams &gp, uint32_t l, V3 p)
+{
+    const float s = gp.scale[l];
+    const float px = __fmaf_rn(p.x, s, 0.5f), py = __fmaf_rn(p.y, s, 0.5f), pz = __fmaf_rn(p.z, s, 0.5f);
+    const float flx = floorf(px), fly = floorf(py), flz = floorf(pz);
+    LevelCell c;
+    c.gx = (uint32_t)(int32_t)flx, c.gy = (uint32_t)(int32_t)fly, c.gz = (uint32_t)(int32_t)flz;
+    c.rx = __fsub_rn(px, flx), c.ry = __fsub_rn(py, fly), c.rz = __fsub_rn(pz, flz);
+    return c;
+}
+
+// Index of corner c (bit d of c selects the upper corner along axis d) in its level's table.
+__device__ __forceinline__ uint32_t level_corner_index(bool hashed, uint32_t res, uint32_t size, const LevelCell &q,
+                                                       uint32_t c)
+{
+    const uint32_t x = q.gx + (c & 1u), y = q.gy + ((c >> 1) & 1u), z = q.gz + ((c >> 2) & 1u);
+    if (hashed)
+        return (x ^ (y * 2654435761u) ^ (z * 805459861u)) & (size - 1u);
+    const uint32_t i = x + y * res + z * res * res;
+    return i >= size ? i % size : i;
+}
+
+// Whether cell q of level l is in the cell copy (positions outside the unit cube may not be), and
+// which cell it is there.
+__device__ __forceinline__ bool cell_index(const CellParams &cp, uint32_t l, const LevelCell &q, uint32_t &i)
+{
+    const uint32_t n = cp.dim[l];
+    i = cp.offset[l] + q.gx + n * (q.gy + n * q.gz);
+    return q.gx < n && q.gy < n && q.gz < n;
+}
+
+__device__ __forceinline__ float corner_weight(const LevelCell &q, uint32_t c)
+{
+    return __fmul_rn(__fmul_rn((c & 1u) ? q.rx : __fsub_rn(1.0f, q.rx), (c & 2u) ? q.ry : __fsub_rn(1.0f, q.ry)),
+                     (c & 4u) ? q.rz : __fsub_rn(1.0f, q.rz));
+}
+
+// 32 bytes (32-byte aligned, read-only) in one load
+__device__ __forceinline__ void load32(const void *p, uint32_t (&v)[8])
+{
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
+
+// Features of one point at levels l .. l + N - 1, all in the cell copy: the reads first, so that they are
+// in flight together. False (and nothing done) if the point lies outside the copy on any of them.
+template <uint32_t N>
+__device__ __forceinline__ bool encode_cells(const uint4 *__restrict__ cells, const CellParams &cp,
+                                             const GridParams &gp, uint32_t l, V3 p, float2 (&f)[N])
+{
+    LevelCell q[N];
+    uint32_t ci[N];
+    bool inside = true;
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) {
+        q[k] = level_cell(gp, l + k, p);
+        inside = cell_index(cp, l + k, q[k], ci[k]) && inside;
+    }
+    if (!inside)
+        return false;
+    uint32_t v[N][8];
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++)
+        load32(cells + 2u * (size_t)ci[k], v[k]);
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) {
+        f[k] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (uint32_t c = 0; c < 8; c++) {
+            const float w = corner_weight(q[k], c);
+            const float2 e = unpack_half2(v[k][c]);
+            f[k].x = __fmaf_rn(w, e.x, f[k].x);
+            f[k].y = __fmaf_rn(w, e.y, f[k].y);
+        }
+    }
+    return true;
+}
+
+// The same for one level of 4 or 8 features per entry (the order of encode_level_wide).
+template <uint32_t F>
+__device__ __forceinline__ bool encode_cell_wide(const uint4 *__restrict__ cells, const CellParams &cp,
+                                                 const GridParams &gp, uint32_t l, V3 p, float (&acc)[F])
+{
+    const LevelCell q = level_cell(gp, l, p);
+    uint32_t ci;
+    if (!cell_index(cp, l, q, ci))
+        return false;
+#pragma unroll
+    for (uint32_t k = 0; k < F; k++)
+        acc[k] = 0.0f;
+    const uint4 *src = cells + (size_t)F * ci;
+#pragma unroll
+    for (uint32_t c0 = 0; c0 < 8u; c0 += 4u) { // four corners: F / 4 loads of 32 bytes
+        uint32_t h[F / 4u][8];
+#pragma unroll
+        for (uint32_t k = 0; k < F / 4u; k++)
+            load32(src + (F / 2u) * (c0 / 4u) + 2u * k, h[k]);
+#pragma unroll
+        for (uint32_t cc = 0; cc < 4u; cc++) {
+            const float w = corner_weight(q, c0 + cc);
+#pragma unroll
+            for (uint32_t k = 0; k < F / 2u; k++) {
+                const uint32_t i = cc * (F / 2u) + k;
+                const float2 e = unpack_half2(h[i / 8u][i % 8u]);
+                acc[2 * k] = __fmaf_rn(w, e.x, acc[2 * k]);
+                acc[2 * k + 1] = __fmaf_rn(w, e.y, acc[2 * k + 1]);
+            }
+        }
+    }
+    return true;
+}
+
 // FP8 activations of a pair packed as FP16 (lo in the low half): e4m3(max(x, 0) * 2^7) / 2^7 per
 // value, through the hardware conversions to and from E4M3 (nearest even, saturating at 448,
 // subnormals on the 2^-9 grid: the rounding e4m3_round states); the 2^-7 scale is exact in FP16.
