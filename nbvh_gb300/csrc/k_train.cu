@@ -445,7 +445,7 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 //             transposed from the same shared-memory tiles), then dZ_j = dX_j * (X_j > 0);
 //             dX_0, rounded to the MLP precision, goes to global memory for the grid scatter.
 // The weight gradients stay in tensor memory, accumulated over all the CTA's tiles, and are
-// added to the FP32 gradient once per CTA at the end. Every [128 rows][C columns] tile lives in
+// written out once per CTA at the end; the scatter kernel's last blocks sum them. Every [128 rows][C columns] tile lives in
 // shared memory in the K-major core-matrix layout (8-column block c at c * 2,048 bytes, row r at
 // r * 16 within it): with M = rows it is a K-major operand (LBO 2,048, SBO 128), with K = rows an
 // MN-major one (LBO 128, SBO 2,048). The input tile is copied into that layout 16 bytes at a time.
@@ -475,8 +475,8 @@ struct TrainTcArgs {
     const float *targets; // n x 8
     LossConsts lc;
     __half *dfeat;        // n x n_inputs gradients of the encoded features (emit launches)
-    float *grad;          // FP32 gradient vector (network matrices first)
-    float out_scale;      // factor of what is added to it
+    float *wpart;         // [gridDim.x][n_network] each CTA's weight gradients
+    uint32_t n_network;
     float *loss_sum;
     float *sample_loss;   // per row: sum of its output channels' loss values (may be NULL)
     uint32_t *status;     // nonzero when a bounded wait gave up
@@ -764,6 +764,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     if (!ok) {
         // a wait ran out: record it, give copies and MMAs still in flight one more bounded wait
         tc::copy_async_wait();
+        for (uint32_t i = threadIdx.x; i < a.n_network; i += kTcThreads) // no gradient of this CTA
+            a.wpart[(size_t)blockIdx.x * a.n_network + i] = 0.f;
         if (mma_warp && tc::elect_one()) {
             atomicOr(a.status, 1u);
             if (mma_pending)
@@ -777,18 +779,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
             if (!((a.wg_mask >> j) & 1u))
                 continue;
             const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
-            float *g = a.grad + tc_param_off(j, K0);
+            float *g = a.wpart + (size_t)blockIdx.x * a.n_network + tc_param_off(j, K0);
             for (uint32_t q = half; q < nout / 16u; q += 2u) {
                 uint32_t v[16];
                 tc::tmem_ld16(tmem + lane_off + a.wg_col[j] + 16u * q, v);
                 tc::tmem_wait_ld();
                 if (tid < nin) {
 #pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        const float x = __uint_as_float(v[c]) * a.out_scale;
-                        if (x != 0.f)
-                            atomicAdd(g + (size_t)(16u * q + (uint32_t)c) * nin + tid, x);
-                    }
+                    for (int c = 0; c < 16; c++)
+                        g[(size_t)(16u * q + (uint32_t)c) * nin + tid] = __uint_as_float(v[c]);
                 }
             }
         }
@@ -830,16 +829,38 @@ constexpr uint32_t kScatterThreads = 256, kScatterRows = 32; // rows of a block
 template <uint32_t F>
 constexpr uint32_t kScatterFeatures = F < 4u ? F : 4u;
 
+// The weight gradients of k_train_tc's CTAs, which the launch's first blocks sum while the others scatter:
+// in FP64 and in CTA order, so that the matrices' gradient is the same in every run (as FP32 atomics of
+// 152 CTAs its last bits changed from run to run, and they cost the same time).
+struct WeightSum {
+    const float *part; // [n_part][n]
+    uint32_t n_part, n;
+    float *grad;
+    uint32_t blocks; // of this launch
+};
+
 template <bool BF16, uint32_t F>
 __global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_constant__ GridParams grid,
+                                                                 const __grid_constant__ WeightSum ws,
                                                                  const float *__restrict__ positions,
                                                                  const __half *__restrict__ dfeat, uint32_t n,
                                                                  float *__restrict__ grid_grad, float out_scale)
 {
+    if (blockIdx.x < ws.blocks) {
+        const uint32_t i = blockIdx.x * kScatterThreads + threadIdx.x;
+        if (i < ws.n) {
+            double sum = 0.0;
+#pragma unroll 8
+            for (uint32_t k = 0; k < ws.n_part; k++)
+                sum += (double)__ldg(ws.part + (size_t)k * ws.n + i);
+            ws.grad[i] = (float)sum * out_scale;
+        }
+        return;
+    }
     constexpr uint32_t FT = kScatterFeatures<F>, parts = F / FT;
     const uint32_t P = grid.n_points, L = grid.n_levels;
     for (uint32_t k = threadIdx.x; k < 2u * kScatterRows * L * parts; k += kScatterThreads) {
-        const uint32_t up = k & 1u, row = blockIdx.x * kScatterRows + ((k >> 1) & (kScatterRows - 1u));
+        const uint32_t up = k & 1u, row = (blockIdx.x - ws.blocks) * kScatterRows + ((k >> 1) & (kScatterRows - 1u));
         const uint32_t lp = k / (2u * kScatterRows), l = lp / parts, part = lp % parts;
         if (row >= n)
             continue;
@@ -909,16 +930,16 @@ __global__ void __launch_bounds__(kScatterThreads) k_grid_scatter(const __grid_c
 }
 
 template <bool BF16>
-cudaError_t scatter_rows(const GridParams &grid, const float *positions, const __half *dfeat, uint32_t n,
-                         float *grid_grad, float out_scale, cudaStream_t s)
+cudaError_t scatter_rows(const GridParams &grid, const WeightSum &ws, const float *positions, const __half *dfeat,
+                         uint32_t n, float *grid_grad, float out_scale, cudaStream_t s)
 {
-    const unsigned blocks = (n + kScatterRows - 1u) / kScatterRows;
+    const unsigned blocks = ws.blocks + (n + kScatterRows - 1u) / kScatterRows;
     if (grid.n_features == 4u)
-        k_grid_scatter<BF16, 4><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
+        k_grid_scatter<BF16, 4><<<blocks, kScatterThreads, 0, s>>>(grid, ws, positions, dfeat, n, grid_grad, out_scale);
     else if (grid.n_features == 8u)
-        k_grid_scatter<BF16, 8><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
+        k_grid_scatter<BF16, 8><<<blocks, kScatterThreads, 0, s>>>(grid, ws, positions, dfeat, n, grid_grad, out_scale);
     else
-        k_grid_scatter<BF16, 2><<<blocks, kScatterThreads, 0, s>>>(grid, positions, dfeat, n, grid_grad, out_scale);
+        k_grid_scatter<BF16, 2><<<blocks, kScatterThreads, 0, s>>>(grid, ws, positions, dfeat, n, grid_grad, out_scale);
     return cudaGetLastError();
 }
 
@@ -1140,8 +1161,8 @@ cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, u
 
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
-                              __half *features, __half *dfeat, __half *wpacked, float *grad, float out_scale,
-                              float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
+                              __half *features, __half *dfeat, __half *wpacked, float *wpart, float *grad,
+                              float out_scale, float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
                               uint64_t wait_ns, bool stall, const cudaEvent_t *marks)
 {
     if (n == 0)
@@ -1176,8 +1197,8 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
         a.targets = targets;
         a.lc = lc;
         a.dfeat = dfeat;
-        a.grad = grad;
-        a.out_scale = out_scale;
+        a.wpart = wpart;
+        a.n_network = n_network_params;
         a.loss_sum = loss_sum;
         a.sample_loss = sample_loss;
         a.status = status;
@@ -1189,8 +1210,9 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     }
     if (marks && (e = cudaEventRecord(marks[2], s)) != cudaSuccess)
         return e;
-    e = bf16 ? scatter_rows<true>(grid, positions, dfeat, n, grad + n_network_params, out_scale, s)
-             : scatter_rows<false>(grid, positions, dfeat, n, grad + n_network_params, out_scale, s);
+    const WeightSum ws = {wpart, blocks, n_network_params, grad, (n_network_params + kScatterThreads - 1u) / kScatterThreads};
+    e = bf16 ? scatter_rows<true>(grid, ws, positions, dfeat, n, grad + n_network_params, out_scale, s)
+             : scatter_rows<false>(grid, ws, positions, dfeat, n, grad + n_network_params, out_scale, s);
     if (e == cudaSuccess && marks)
         e = cudaEventRecord(marks[3], s);
     return e;

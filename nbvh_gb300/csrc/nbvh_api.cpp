@@ -479,6 +479,8 @@ void ensure_train_workspace(nbvh_handle *h, uint32_t n)
         cuda_check(h->d_train_dfeat.resize((size_t)n * ni), "alloc feature gradients");
     if (h->d_train_wpacked.count < packed_weight_bytes(ni, H) / 2u)
         cuda_check(h->d_train_wpacked.resize(packed_weight_bytes(ni, H) / 2u), "alloc packed weights");
+    if (h->d_train_wpart.count < (size_t)h->num_sms * h->layout.n_network_params)
+        cuda_check(h->d_train_wpart.resize((size_t)h->num_sms * h->layout.n_network_params), "alloc weight gradients");
     if (h->d_status.count < 1u) {
         cuda_check(h->d_status.resize(1u), "alloc status");
         cuda_check(cudaMemset(h->d_status.ptr, 0, sizeof(uint32_t)), "reset status");
@@ -1468,7 +1470,8 @@ void batch_gradients(nbvh_handle *h, const float *d_pos, const float *d_tgt, uin
     const uint32_t H = (uint32_t)h->cfg.network.n_hidden_layers;
     cuda_check(cudaMemsetAsync(grad, 0, (size_t)h->layout.n_params * sizeof(float), s), "zero grad");
     cuda_check(launch_train_step(h->d_params_h.ptr, h->grid, H, make_loss_consts(h->cfg, n), d_pos, d_tgt, n,
-                                 h->d_train_feat.ptr, h->d_train_dfeat.ptr, h->d_train_wpacked.ptr, grad, out_scale,
+                                 h->d_train_feat.ptr, h->d_train_dfeat.ptr, h->d_train_wpacked.ptr,
+                                 h->d_train_wpart.ptr, grad, out_scale,
                                  loss_slot, clear, h->d_train_loss.ptr, h->d_status.ptr, mlp_bf16(h),
                                  h->cfg.network.precision == NBVH_PRECISION_FP8, h->num_sms, s, h->wait_limit_ns,
                                  h->debug_stall, marks),

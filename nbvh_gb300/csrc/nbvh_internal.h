@@ -378,6 +378,7 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<uint32_t> d_train_nodes;
     nbvh::DeviceBuffer<__half> d_train_feat;    // n x n_inputs encoded features (16-bit)
     nbvh::DeviceBuffer<__half> d_train_dfeat;   // n x n_inputs gradients of the features (16-bit)
+    nbvh::DeviceBuffer<float> d_train_wpart;    // num_sms x network parameters: weight gradients per CTA
     nbvh::DeviceBuffer<__half> d_train_wpacked; // network matrices in the tensor-core operand layout
     nbvh::DeviceBuffer<float> d_train_loss;  // per row loss (sum over output channels)
     nbvh::DeviceBuffer<float> d_loss_sum;
@@ -688,16 +689,17 @@ cudaError_t launch_training_samples(const float4 *neural_nodes, const float4 *no
 
 // One training pass over n rows (positions n x points x 3, targets n x 8): the hash-grid features
 // into `features` (n x n_inputs, 16-bit), the network matrices packed into `wpacked`
-// (packed_weight_bytes), forward + composite loss + backward on the tcgen05 tensor cores (the
-// weight gradients added to grad, the loss sum into *loss_sum, per-row losses into sample_loss
-// when not NULL, the 16-bit feature gradients into dfeat, n x n_inputs), then the hash-grid
-// gradient scattered into grad + n_network_params. grad (16-byte aligned) receives the gradient
+// (packed_weight_bytes), forward + composite loss + backward on the tcgen05 tensor cores (each CTA's
+// weight gradients into wpart, num_sms x n_network_params, the loss added to *loss_sum, per-row
+// losses into sample_loss when not NULL, the 16-bit feature gradients into dfeat, n x n_inputs), then
+// the sum of the weight gradients written to grad and the hash-grid gradient added to grad +
+// n_network_params. grad (16-byte aligned) receives the gradient
 // times the loss scale times out_scale; with `clear` the loss sum and the status start from zero.
 // status receives a nonzero word if a bounded wait inside the tensor-core kernel gave up.
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
-                              __half *features, __half *dfeat, __half *wpacked, float *grad, float out_scale,
-                              float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
+                              __half *features, __half *dfeat, __half *wpacked, float *wpart, float *grad,
+                              float out_scale, float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
                               uint64_t wait_ns = 0, bool stall = false, const cudaEvent_t *marks = nullptr);
 // (marks, when given: 4 events recorded before the encoding, before and after the tensor-core
 // passes, and after the grid scatter)
