@@ -989,6 +989,11 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
     const WaveList &in = a.lists[it & 1u];
     uint32_t *head = &a.wave_counts[4u + it % 3u];
     const bool sorted = a.perm != nullptr && count_in >= kSortMinRows;
+    // place on the segment of the point this lane encodes (encode_tile_to_smem)
+    uint32_t no_rng = 0;
+    const float point_t = a.grid.segment_distribution == NBVH_SEGMENT_UNIFORM
+                              ? 0.f
+                              : segment_t((uint32_t)lane % P, P, a.grid.segment_distribution, no_rng);
     const bool ahead_ok = a.grid.segment_distribution != NBVH_SEGMENT_UNIFORM && a.non_neural == nullptr;
     uint32_t st_segments = 0, st_capped = 0, st_overflow = 0, st_fallback = 0;
 
@@ -1117,14 +1122,11 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
             const uint32_t n_t = min(16u, rows - tile * 16u);
             auto pos = [&](uint32_t r, uint32_t p) -> V3 {
                 const float4 e0 = ends[2u * (16u * tile + r)], e1 = ends[2u * (16u * tile + r) + 1u];
-                float t;
+                float t = point_t;
                 if (gp.segment_distribution == NBVH_SEGMENT_UNIFORM) {
                     uint32_t rng = __float_as_uint(e0.w);
                     for (uint32_t k = 0; k <= p; k++)
                         t = lcg_randomf(rng);
-                } else {
-                    uint32_t unused = 0;
-                    t = segment_t(p, P, gp.segment_distribution, unused);
                 }
                 return segment_point(mk3(e0.x, e0.y, e0.z), mk3(e1.x, e1.y, e1.z), t);
             };

@@ -543,58 +543,42 @@ __device__ __forceinline__ void mlp_forward_tile(const __half *sw, uint32_t n_in
 
 // Encode phase of a tile of `rows` (at most 16) rows: the 16-bit features of every (row, point, level)
 // written to the warp's feature tile feat[16][ld] (ld = n_inputs + 8 halves); the rows past them keep
-// whatever they hold (an MLP row depends on its own features alone). The warp's lanes take the
-// (row, level, point) items in turn, points fastest (a row's points are neighbours, so their corners
-// share cache lines on the coarser levels), kTileItems at a time: the positions first, then the
-// gathers of all of them without branches in between, so that they are in flight together. A lane
-// past the last item repeats its first one. No MLP accumulator is live here.
-//
-// The gathers bound this phase: a lane's 8 corners lie in as many cache lines, and the L1 takes one
-// line per cycle, so work for rows that do not exist costs as much as work for rows that do (the
-// form before this one rounded up to 4 rows and put 32 (point, level) pairs of one row in a warp).
-// Two items at once: 700 us per 512 x 512 frame and 2,925 per 2^22-ray query against 707 and 2,970
-// with four, which spill.
-constexpr uint32_t kTileItems = 2;
-
+// whatever they hold (an MLP row depends on its own features alone). Row by row: a lane takes one
+// point of the row and every (32 / points)-th level. Neighbouring lanes hold a row's points, which
+// are neighbours in space, so their corners share cache lines on the coarser levels; the point's place
+// on the segment is the same for every row (the caller keeps it), and no item needs a division. No MLP
+// accumulator is live here.
+// Address arithmetic and the gathers' latency bound this phase, at 16 warps per SM. Dealing a tile's
+// (row, level, point) items over the lanes fills all of them, but finds row, level, point and place
+// anew for each: 632 us per 512 x 512 frame, 2,002 per 960 x 540 path, 186 per 16,384-ray query
+// against 611, 1,924 and 165 so. Two levels in flight per lane: 615, 1,948 and 174.
 template <bool BF16, uint32_t F, typename PosFn>
 __device__ __forceinline__ void encode_tile_to_smem(const uint32_t *__restrict__ table, const GridParams &gp,
                                                     PosFn &&pos, uint32_t rows, __half *feat, uint32_t ld)
 {
-    constexpr uint32_t N = F == 2u ? kTileItems : 8u / F; // the same number of gathered words in flight
-    const uint32_t lane = threadIdx.x & 31u, P = gp.n_points, L = gp.n_levels, PL = P * L, total = rows * PL;
-    for (uint32_t i0 = lane; i0 < total; i0 += 32u * N) {
-        V3 q[N];
-        uint32_t lev[N], dst[N];
+    const uint32_t lane = threadIdx.x & 31u, P = gp.n_points, L = gp.n_levels;
+    const uint32_t slots = 32u / P, slot = lane / P, p = lane - slot * P; // P <= 32: at least one slot
+    if (slot < slots) {
+        for (uint32_t r = 0; r < rows; r++) {
+            const V3 q = pos(r, p);
+            __half *dst = feat + r * ld + p * L * F;
+            for (uint32_t l = slot; l < L; l += slots) { // one 4-, 8- or 16-byte store per level
+                if constexpr (F == 2u) {
+                    const float2 f = encode_level<false>(table, gp, l, q);
+                    *reinterpret_cast<uint32_t *>(dst + l * F) = MlpPrec<BF16>::pack(f.x, f.y);
+                } else {
+                    float f[F];
+                    encode_level_wide<F>(table, gp, l, q, f);
+                    uint32_t w[F / 2u];
 #pragma unroll
-        for (uint32_t k = 0; k < N; k++) {
-            const uint32_t i = i0 + 32u * k < total ? i0 + 32u * k : i0;
-            const uint32_t r = i / PL, j = i - r * PL, l = j / P, p = j - l * P;
-            q[k] = pos(r, p);
-            lev[k] = l;
-            dst[k] = r * ld + (p * L + l) * F;
-        }
-        uint32_t w[N][F / 2u];
-#pragma unroll
-        for (uint32_t k = 0; k < N; k++) {
-            if constexpr (F == 2u) {
-                const float2 f = encode_level<false>(table, gp, lev[k], q[k]);
-                w[k][0] = MlpPrec<BF16>::pack(f.x, f.y);
-            } else {
-                float f[F];
-                encode_level_wide<F>(table, gp, lev[k], q[k], f);
-#pragma unroll
-                for (uint32_t c = 0; c < F / 2u; c++)
-                    w[k][c] = MlpPrec<BF16>::pack(f[2u * c], f[2u * c + 1u]);
+                    for (uint32_t c = 0; c < F / 2u; c++)
+                        w[c] = MlpPrec<BF16>::pack(f[2u * c], f[2u * c + 1u]);
+                    if constexpr (F == 4u)
+                        *reinterpret_cast<uint2 *>(dst + l * F) = make_uint2(w[0], w[1]);
+                    else
+                        *reinterpret_cast<uint4 *>(dst + l * F) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
             }
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < N; k++) { // one 4-, 8- or 16-byte store (a repeated item writes the same bits)
-            if constexpr (F == 2u)
-                *reinterpret_cast<uint32_t *>(feat + dst[k]) = w[k][0];
-            else if constexpr (F == 4u)
-                *reinterpret_cast<uint2 *>(feat + dst[k]) = make_uint2(w[k][0], w[k][1]);
-            else
-                *reinterpret_cast<uint4 *>(feat + dst[k]) = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
         }
     }
     __syncwarp();

@@ -15,7 +15,8 @@ from nbvh_gb300 import scenes
 pytestmark = pytest.mark.gpu
 
 # (points, levels, features, precision, hidden layers): a row of a tile is points x levels items of the encoder
-NETS = [(4, 16, 2, 0, 4), (3, 8, 4, 1, 4), (2, 4, 8, 2, 4), (1, 8, 2, 0, 1), (4, 16, 2, 1, 8), (4, 8, 4, 2, 3)]
+NETS = [(4, 16, 2, 0, 4), (3, 8, 4, 1, 4), (2, 4, 8, 2, 4), (1, 8, 2, 0, 1), (4, 16, 2, 1, 8), (4, 8, 4, 2, 3),
+        (4, 12, 2, 0, 2), (16, 4, 2, 0, 2), (6, 8, 2, 1, 2)]
 
 
 @pytest.mark.parametrize("net", NETS)
