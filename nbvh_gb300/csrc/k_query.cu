@@ -234,6 +234,18 @@ __device__ __forceinline__ uint32_t listed_row_bin(const WaveArgs &a, const Wave
     return row_bin(a, m.y, mk3(od0.x, od0.y, od0.z), mk3(od1.x, od1.y, od1.z), od1.w, __uint_as_float(m.x));
 }
 
+// Word of the sort's shared-memory scan for bin k: a word of padding per 32, so that threads that walk
+// neighbouring runs of a few bins meet in no bank.
+__host__ __device__ constexpr uint32_t sort_scan_index(uint32_t k)
+{
+    return k + (k >> 5);
+}
+// scan and per-block counts
+__host__ __device__ constexpr uint32_t sort_smem_bytes(uint32_t n_bins)
+{
+    return (sort_scan_index(n_bins) + n_bins) * (uint32_t)sizeof(uint32_t);
+}
+
 // Counts the rows a warp appends per sort bin (one atomic per distinct bin in the warp); all 32
 // lanes take part.
 __device__ __forceinline__ void count_nodes(uint32_t *bins, bool want, uint32_t node)
@@ -613,17 +625,23 @@ __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
 }
 
 // Counting sort of the listed rays by their current leaf node (the per-node compaction of the
-// segments). The per-node counts were gathered when the list was written. Each block takes one
-// contiguous chunk of the list: it scans the counts in shared memory, counts its own rows per node
-// with shared-memory atomics, reserves one range per non-empty node with a global atomic, then
-// places its rows. The encoder, MLP and decoder then walk the list in node order, so rays of the
-// same leaf region are encoded together and the grid cells of the coarser levels are served from
-// L1. Also clears the next step's counts and cursors.
+// segments). The per-node counts were gathered when the list was written. Every block scans them in
+// shared memory, then places one contiguous chunk of the list. The encoder, MLP and decoder then walk
+// the list in node order, so rays of the same leaf region are encoded together and the grid cells of
+// the coarser levels are served from L1. Also clears the next step's counts and cursors.
+//
+// Chains of dependent accesses bound it, not bytes: 23 us for 150,000 rows and 16,376 bins when every
+// thread reserved its bins' ranges one after the other and scanned runs that met in the same banks;
+// 18 with eight reservations in flight and the padded scan (123 to 81 for the sorts of 2^22 rays). A chunk
+// with at most half as many rows as there are bins has about one row per bin and
+// takes its places straight from the bins' cursors, one atomic for the lanes of a warp that share a bin:
+// 16 us, and 574 instead of 589 per 512 x 512 frame. With few bins many blocks would meet on
+// each cursor: 54 us instead of 34 for the lists of 2^20 visibility rays in 2,047 bins.
 __global__ void __launch_bounds__(kSortThreads) k_wave_sort(const __grid_constant__ WaveArgs a, uint32_t it)
 {
-    extern __shared__ uint32_t sort_smem[];
+    extern __shared__ uint32_t scan[]; // [sort_scan_index(NB)]
     const uint32_t NB = a.n_sort_nodes;
-    uint32_t *scan = sort_smem, *cnt = sort_smem + NB, *base = sort_smem + 2u * NB;
+    uint32_t *cnt = scan + sort_scan_index(NB); // [NB]
     const uint32_t *bins = a.node_bins + (it & 1u) * NB;
     uint32_t *cursor = a.node_cursor + (it & 1u) * NB;
     {
@@ -640,13 +658,17 @@ __global__ void __launch_bounds__(kSortThreads) k_wave_sort(const __grid_constan
     if (count_in < kSortMinRows || r0 >= r1)
         return;
     // exclusive scan of the node counts: contiguous runs per thread, then a scan of the run sums
+#pragma unroll 4
+    for (uint32_t k = threadIdx.x; k < NB; k += blockDim.x) {
+        scan[sort_scan_index(k)] = bins[k];
+        cnt[k] = 0u;
+    }
+    __syncthreads();
     const uint32_t per = (NB + blockDim.x - 1u) / blockDim.x;
     const uint32_t k0 = min(NB, threadIdx.x * per), k1 = min(NB, k0 + per);
     uint32_t run = 0;
-    for (uint32_t k = k0; k < k1; k++) {
-        run += bins[k];
-        cnt[k] = 0u;
-    }
+    for (uint32_t k = k0; k < k1; k++)
+        run += scan[sort_scan_index(k)];
     __shared__ uint32_t warp_sums[kSortThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl = run;
@@ -663,23 +685,47 @@ __global__ void __launch_bounds__(kSortThreads) k_wave_sort(const __grid_constan
     for (int w = 0; w < warp; w++)
         acc += warp_sums[w];
     for (uint32_t k = k0; k < k1; k++) {
-        scan[k] = acc;
-        acc += bins[k];
+        const uint32_t c = scan[sort_scan_index(k)];
+        scan[sort_scan_index(k)] = acc;
+        acc += c;
     }
+    __syncthreads();
     const WaveList &in = a.lists[it & 1u];
+    if (2u * (r1 - r0) <= NB) {
+        for (uint32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+            const uint32_t node = listed_row_bin(a, in, r);
+            const unsigned same = __match_any_sync(__activemask(), node);
+            const int leader = __ffs(same) - 1;
+            uint32_t slot = 0;
+            if (lane == leader)
+                slot = scan[sort_scan_index(node)] + atomicAdd(&cursor[node], (uint32_t)__popc(same));
+            slot = __shfl_sync(same, slot, leader) + __popc(same & ((1u << lane) - 1u));
+            if (slot < count_in) // the counts match the list; the check only keeps a stray row in bounds
+                a.perm[slot] = r;
+        }
+        return;
+    }
     for (uint32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)
         atomicAdd(&cnt[listed_row_bin(a, in, r)], 1u);
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < NB; k += blockDim.x) {
-        const uint32_t c = cnt[k];
-        base[k] = c ? atomicAdd(&cursor[k], c) : 0u;
-        cnt[k] = 0u;
+    for (uint32_t k = threadIdx.x; k < NB; k += 8u * blockDim.x) { // a range per bin that the chunk has rows of
+        uint32_t at[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; j++) {
+            const uint32_t i = k + j * blockDim.x, c = i < NB ? cnt[i] : 0u;
+            at[j] = c ? atomicAdd(&cursor[i], c) : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8u; j++) {
+            const uint32_t i = k + j * blockDim.x;
+            if (i < NB)
+                cnt[i] = scan[sort_scan_index(i)] + at[j];
+        }
     }
     __syncthreads();
     for (uint32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-        const uint32_t node = listed_row_bin(a, in, r);
-        const uint32_t slot = scan[node] + base[node] + atomicAdd(&cnt[node], 1u);
-        if (slot < count_in) // the counts match the list; the check only keeps a stray row in bounds
+        const uint32_t slot = atomicAdd(&cnt[listed_row_bin(a, in, r)], 1u);
+        if (slot < count_in)
             a.perm[slot] = r;
     }
 }
@@ -1317,7 +1363,7 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
             // the rest of the query in one launch; in a captured graph the list counters are cleared
             // after it, so that the copy the graph ends with reads an empty list
             if (a.perm) {
-                k_wave_sort<<<(uint32_t)num_sms, kSortThreads, 3u * a.n_sort_nodes * 4u, s>>>(a, it);
+                k_wave_sort<<<(uint32_t)num_sms, kSortThreads, sort_smem_bytes(a.n_sort_nodes), s>>>(a, it);
                 e = cudaGetLastError();
                 if (e != cudaSuccess)
                     return e;
@@ -1332,7 +1378,7 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
             return cudaSuccess;
         }
         if (a.perm) {
-            k_wave_sort<<<(uint32_t)num_sms, kSortThreads, 3u * a.n_sort_nodes * 4u, s>>>(a, it);
+            k_wave_sort<<<(uint32_t)num_sms, kSortThreads, sort_smem_bytes(a.n_sort_nodes), s>>>(a, it);
             e = cudaGetLastError();
             if (e != cudaSuccess)
                 return e;
@@ -1535,8 +1581,8 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     const bool keyed = res.sort_key != nullptr && res.n_sort_bins > 0u;
     const uint32_t n_bins = keyed ? res.n_sort_bins : n_cut_nodes;
     a.sort_key = keyed ? res.sort_key : nullptr;
-    // octant sub-bins where the caller sized the count buffers for them, the sort's three
-    // shared-memory arrays of 8 x n_bins words fit, and each row has enough point-levels to gather
+    // octant sub-bins where the caller sized the count buffers for them, the sort's
+    // shared memory (of the form that kept three words per bin) fits, and each row has enough point-levels to gather
     // for the encoder's better locality to outweigh the sort's extra reads (measured on GB300: 4
     // points x 16 levels 3.35 -> 3.31 ms per 2^22-ray query; 3 points x 8 levels 2.32 -> 2.37 ms)
     a.sub_bins = (res.sub_bins && (size_t)3u * 4u * kSubBins * n_bins <= (size_t)kMaxDynamicSmem &&
