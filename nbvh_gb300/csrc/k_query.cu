@@ -287,13 +287,14 @@ struct RayBinArgs {
     uint32_t n;
     V3 lo, scale;
     uint16_t *keys;
-    uint32_t *bins;  // kRayBins counts (zeroed before), then the cursors
+    uint32_t *bins;  // kRayBins counts, then kRayBins cursors (both zeroed before)
     uint32_t *order; // n ray ids, bin by bin
 };
 
 // Counts the rays per bin and keeps every ray's bin. Each block takes one contiguous chunk of the
 // batch and adds its shared-memory counts to the global ones (one atomic per non-empty bin).
 constexpr uint32_t kRayBinThreads = 1024;
+constexpr uint32_t kRaysAtOnce = 2, kKeysAtOnce = 4;
 
 __device__ __forceinline__ void ray_chunk(uint32_t n, uint32_t &r0, uint32_t &r1)
 {
@@ -310,10 +311,17 @@ __global__ void __launch_bounds__(kRayBinThreads) k_ray_bins(const __grid_consta
     __syncthreads();
     uint32_t r0, r1;
     ray_chunk(a.n, r0, r1);
-    for (uint32_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-        const uint32_t b = ray_bin(a.rays, i, a.lo, a.scale);
-        a.keys[i] = (uint16_t)b;
-        atomicAdd(&cnt[b], 1u);
+    for (uint32_t i = r0 + threadIdx.x; i < r1; i += kRaysAtOnce * blockDim.x) {
+        uint32_t b[kRaysAtOnce];
+#pragma unroll
+        for (uint32_t j = 0; j < kRaysAtOnce; j++) // past the chunk: the first ray again
+            b[j] = ray_bin(a.rays, i + j * blockDim.x < r1 ? i + j * blockDim.x : i, a.lo, a.scale);
+#pragma unroll
+        for (uint32_t j = 0; j < kRaysAtOnce; j++)
+            if (i + j * blockDim.x < r1) {
+                a.keys[i + j * blockDim.x] = (uint16_t)b[j];
+                atomicAdd(&cnt[b[j]], 1u);
+            }
     }
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < kRayBins; b += blockDim.x)
@@ -321,19 +329,44 @@ __global__ void __launch_bounds__(kRayBinThreads) k_ray_bins(const __grid_consta
             atomicAdd(&a.bins[b], cnt[b]);
 }
 
-// Exclusive scan of the bin counts into placement cursors (one block of 1,024 threads,
-// kRayBins / 1,024 bins each).
-constexpr uint32_t kRayBinsPerThread = kRayBins / 1024u;
-static_assert(kRayBins % 1024u == 0u, "whole bins per scan thread");
-__global__ void __launch_bounds__(1024) k_ray_bin_scan(uint32_t *bins)
+// Places the ray ids bin by bin: each block takes the same chunk as k_ray_bins, counts it per bin
+// again in shared memory, reserves one range per non-empty bin, then places its rays with
+// shared-memory atomics (the order inside a bin does not matter). A thread's kRayBinsPerThread bins are
+// neighbours, so that it also holds their share of the scan of the batch's counts, which every block
+// makes for itself (as a kernel of one block it took 9 us).
+//
+// Dependent accesses bound both kernels, so a thread has kRaysAtOnce / kKeysAtOnce rays and all its
+// reservations in flight: 2^22 rays take 26 us to bin and 43 to place (29 and 45, and 9 for the scan, one
+// by one), 2^20 rays 10 and 14 (10, 16 and 9). Four rays or eight keys at once: 29 and 43.
+constexpr uint32_t kRayBinsPerThread = kRayBins / kRayBinThreads;
+static_assert(kRayBins % (4u * kRayBinThreads) == 0u, "whole groups of four bins per thread");
+__global__ void __launch_bounds__(kRayBinThreads) k_ray_bin_place(const __grid_constant__ RayBinArgs a)
 {
-    __shared__ uint32_t warp_sums[32];
+    __shared__ __align__(16) uint32_t cnt[kRayBins];
+    for (uint32_t b = threadIdx.x; b < kRayBins; b += blockDim.x)
+        cnt[b] = 0u;
+    __syncthreads();
+    uint32_t r0, r1;
+    ray_chunk(a.n, r0, r1);
+    for (uint32_t i = r0 + threadIdx.x; i < r1; i += kKeysAtOnce * blockDim.x) {
+        uint32_t b[kKeysAtOnce];
+#pragma unroll
+        for (uint32_t j = 0; j < kKeysAtOnce; j++)
+            b[j] = i + j * blockDim.x < r1 ? a.keys[i + j * blockDim.x] : kRayBins;
+#pragma unroll
+        for (uint32_t j = 0; j < kKeysAtOnce; j++)
+            if (b[j] < kRayBins)
+                atomicAdd(&cnt[b[j]], 1u);
+    }
+    // first place of each of this thread's bins: an exclusive scan over the threads
+    __shared__ uint32_t warp_sums[kRayBinThreads / 32u];
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     uint32_t v[kRayBinsPerThread], run = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < kRayBinsPerThread; k++) {
-        v[k] = bins[kRayBinsPerThread * t + k];
-        run += v[k];
+    for (uint32_t k = 0; k < kRayBinsPerThread; k += 4u) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(a.bins + kRayBinsPerThread * t + k);
+        v[k] = q.x, v[k + 1u] = q.y, v[k + 2u] = q.z, v[k + 3u] = q.w;
+        run += q.x + q.y + q.z + q.w;
     }
     uint32_t incl = run;
 #pragma unroll
@@ -344,37 +377,39 @@ __global__ void __launch_bounds__(1024) k_ray_bin_scan(uint32_t *bins)
     }
     if (lane == 31u)
         warp_sums[warp] = incl;
-    __syncthreads();
-    uint32_t base = incl - run;
+    __syncthreads(); // the block's counts are complete, too
+    uint32_t first = incl - run;
     for (uint32_t w = 0; w < warp; w++)
-        base += warp_sums[w];
+        first += warp_sums[w];
+    uint32_t *cursor = a.bins + kRayBins + kRayBinsPerThread * t, *mine = cnt + kRayBinsPerThread * t;
+    uint32_t at[kRayBinsPerThread];
 #pragma unroll
     for (uint32_t k = 0; k < kRayBinsPerThread; k++) {
-        bins[kRayBinsPerThread * t + k] = base;
-        base += v[k];
+        const uint32_t c = mine[k];
+        at[k] = c ? atomicAdd(&cursor[k], c) : 0u;
     }
-}
-
-// Places the ray ids bin by bin: each block takes the same chunk as k_ray_bins, counts it per bin
-// again in shared memory, reserves one range per non-empty bin from the global cursors, then
-// places its rays with shared-memory atomics (the order inside a bin does not matter).
-__global__ void __launch_bounds__(kRayBinThreads) k_ray_bin_place(const __grid_constant__ RayBinArgs a)
-{
-    __shared__ uint32_t cnt[kRayBins];
-    for (uint32_t b = threadIdx.x; b < kRayBins; b += blockDim.x)
-        cnt[b] = 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kRayBinsPerThread; k++) { // now this block's next position in the bin
+        mine[k] = first + at[k];
+        first += v[k];
+    }
     __syncthreads();
-    uint32_t r0, r1;
-    ray_chunk(a.n, r0, r1);
-    for (uint32_t i = r0 + threadIdx.x; i < r1; i += blockDim.x)
-        atomicAdd(&cnt[a.keys[i]], 1u);
-    __syncthreads();
-    for (uint32_t b = threadIdx.x; b < kRayBins; b += blockDim.x)
-        if (cnt[b])
-            cnt[b] = atomicAdd(&a.bins[b], cnt[b]); // now this block's next position in bin b
-    __syncthreads();
-    for (uint32_t i = r0 + threadIdx.x; i < r1; i += blockDim.x)
-        a.order[atomicAdd(&cnt[a.keys[i]], 1u)] = i;
+    for (uint32_t i = r0 + threadIdx.x; i < r1; i += kKeysAtOnce * blockDim.x) {
+        uint32_t b[kKeysAtOnce];
+#pragma unroll
+        for (uint32_t j = 0; j < kKeysAtOnce; j++)
+            b[j] = i + j * blockDim.x < r1 ? a.keys[i + j * blockDim.x] : kRayBins;
+#pragma unroll
+        for (uint32_t j = 0; j < kKeysAtOnce; j++)
+            if (b[j] < kRayBins)
+                b[j] = atomicAdd(&cnt[b[j]], 1u);
+            else
+                b[j] = kInvalid;
+#pragma unroll
+        for (uint32_t j = 0; j < kKeysAtOnce; j++)
+            if (b[j] != kInvalid)
+                a.order[b[j]] = i + j * blockDim.x;
+    }
 }
 
 // What a query needs before its first pass, in one launch (it was four memsets and a launch): its
@@ -1524,11 +1559,10 @@ cudaError_t launch_ray_order(const nbvh_ray *rays, uint32_t n, const float scene
     rb.bins = bins;
     rb.order = order;
     const uint32_t blocks = (uint32_t)num_sms;
-    cudaError_t e = cudaMemsetAsync(bins, 0, kRayBins * sizeof(uint32_t), s);
+    cudaError_t e = cudaMemsetAsync(bins, 0, kRayBinWords * sizeof(uint32_t), s);
     if (e != cudaSuccess)
         return e;
     k_ray_bins<<<blocks, kRayBinThreads, 0, s>>>(rb);
-    k_ray_bin_scan<<<1, 1024, 0, s>>>(bins);
     k_ray_bin_place<<<blocks, kRayBinThreads, 0, s>>>(rb);
     return cudaGetLastError();
 }

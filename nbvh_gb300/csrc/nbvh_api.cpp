@@ -1007,8 +1007,8 @@ const uint32_t *classic_order(nbvh_handle *h, uint32_t n)
         cuda_check(h->d_classic_order.resize(n), "alloc ray order");
         cuda_check(h->d_classic_keys.resize(n), "alloc ray bins");
     }
-    if (h->d_classic_bins.count < kRayBins)
-        cuda_check(h->d_classic_bins.resize(kRayBins), "alloc ray bin counts");
+    if (h->d_classic_bins.count < kRayBinWords)
+        cuda_check(h->d_classic_bins.resize(kRayBinWords), "alloc ray bin counts");
     return h->d_classic_order.ptr;
 }
 
@@ -2156,8 +2156,8 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
     const uint32_t wb = packed_weight_bytes(h->layout.n_inputs, (uint32_t)h->cfg.network.n_hidden_layers);
     if (q.wpacked.count < wb / 2u)
         cuda_check(q.wpacked.resize(wb / 2u), "alloc packed weights");
-    if (q.ray_bins.count < kRayBins)
-        cuda_check(q.ray_bins.resize(kRayBins), "alloc ray bin counts");
+    if (q.ray_bins.count < kRayBinWords)
+        cuda_check(q.ray_bins.resize(kRayBinWords), "alloc ray bin counts");
     if (!q.ev)
         cuda_check(cudaEventCreateWithFlags(&q.ev, cudaEventDisableTiming), "event");
     if (q.capacity < n || q.features.count < (size_t)n * h->layout.n_inputs) {

@@ -203,7 +203,7 @@ struct QueryContext {
     DeviceBuffer<__half> wpacked;
     DeviceBuffer<uint32_t> perm;                   // [capacity]
     DeviceBuffer<uint16_t> ray_keys;               // [capacity] coherence bin of each ray
-    DeviceBuffer<uint32_t> ray_bins;               // [kRayBins]
+    DeviceBuffer<uint32_t> ray_bins;               // [kRayBinWords]
     DeviceBuffer<uint32_t> node_bins, node_cursor; // [2][cut nodes]
     uint32_t capacity = 0;
     uint64_t generation = 0;     // incremented whenever a buffer is reallocated
@@ -458,12 +458,13 @@ inline cudaError_t allow_max_dynamic_smem(K kernel)
 }
 
 // Coherence bins of the rays of a query (24 direction classes, octant x dominant axis, x 8^3 origin
-// cells of the scene box grown by half its size on every side): the first pass and the classic kernel take the rays bin
-// by bin, so that the rays of a warp start near one another in the same direction. Batches below
-// kRaySortMin rays are taken in batch order: the ordering's three launches (about 50 us) pay only
-// on larger batches (measured: 2^22 uniform rays, classic 1.49 -> 1.09 ms; a 389K-ray camera batch,
-// already coherent, 0.174 -> 0.213 ms).
+// cells of the scene box grown by half its size on every side): the first pass and the classic kernel
+// take the rays bin by bin, so that the rays of a warp start near one another in the same direction.
+// Batches below kRaySortMin rays are taken in batch order: the ordering pays only on larger batches
+// (measured when it took three launches and about 50 us: 2^22 uniform rays, classic 1.49 -> 1.09 ms; a
+// 389K-ray camera batch, already coherent, 0.174 -> 0.213 ms; it now takes 15 to 70 us).
 constexpr uint32_t kRayBins = 12288; // 24 direction classes x 8^3 origin cells
+constexpr uint32_t kRayBinWords = 2u * kRayBins; // a count and a placement cursor per bin
 constexpr uint32_t kRaySortMin = 1u << 19;
 
 // Cuts with more nodes than this are not sorted by node between steps (the sort scans the node
@@ -494,7 +495,7 @@ struct StepResources {
     uint32_t *perm;        // [capacity] rows in leaf-node order (nullptr: no sorting); before the first
                            // step, the order in which the first pass takes the rays
     uint16_t *ray_keys = nullptr; // [capacity] coherence bins of the rays (nullptr: rays in batch order)
-    uint32_t *ray_bins = nullptr; // [kRayBins] counts, then placement cursors, of those bins
+    uint32_t *ray_bins = nullptr; // [kRayBinWords] counts and placement cursors of those bins
     uint32_t *node_bins;   // [2][n_cut_nodes]
     uint32_t *node_cursor; // [2][n_cut_nodes]
     TensorMapBytes feature_map;
@@ -584,7 +585,8 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
 cudaError_t configure_query_kernels();
 
 // order[0..n) = the ray ids bin by bin (coherence bins over the scene box, kRayBins of them);
-// keys: n, bins: kRayBins device words of scratch. Three kernels and a memset on the stream.
+// keys: n, bins: kRayBinWords device words of scratch (16-byte aligned). Two kernels and a memset on the
+// stream.
 cudaError_t launch_ray_order(const nbvh_ray *rays, uint32_t n, const float scene_min[3], const float scene_max[3],
                              uint16_t *keys, uint32_t *bins, uint32_t *order, int num_sms, cudaStream_t s);
 
