@@ -436,7 +436,11 @@ __global__ void __launch_bounds__(128) k_query_begin(const __grid_constant__ Beg
 // current_maxt, include/cuda/neural/neural_bvh_module_common.cuh:332-343). Rays that enter none
 // are answered at once; the others are appended to state list 0. Persistent warps take rays from
 // a work counter and refill lanes between rounds of a.visits node visits, as the decode
-// kernel does, so the warp's lanes stay busy while the traversal lengths differ.
+// kernel does, so the warp's lanes stay busy while the traversal lengths differ. The smallest
+// batches (SPREAD) are spread over the grid's warps, ceil(n / warps) lanes in each: lanes of one warp that take
+// different branches run one after the other (a 64-ray query takes 86 us so, 98 with the rays in two
+// warps; 512 rays 97 and 103; 65,536 rays 277 and 272, so larger batches fill their warps).
+template <bool SPREAD>
 __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_constant__ WaveArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -447,8 +451,10 @@ __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_co
     bool cull_ok = false, active = false, exhausted = false;
     float tmax = 0.f;
     const GlobalCut cut{a.nodes, a.bounds};
+    const uint32_t n_warps = gridDim.x * (kFirstThreads / 32u);
+    const bool takes = !SPREAD || (uint32_t)lane < (a.n + n_warps - 1u) / n_warps; // this lane has rays at all
     for (;;) {
-        const unsigned idle = __ballot_sync(kFull, !active);
+        const unsigned idle = __ballot_sync(kFull, !active && takes);
         if (idle != 0u && !exhausted) {
             const int leader = __ffs(idle) - 1;
             uint32_t base = 0;
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_co
             base = __shfl_sync(kFull, base, leader);
             exhausted = base + (uint32_t)__popc(idle) >= a.n;
             const uint32_t i = base + __popc(idle & ((1u << lane) - 1u));
-            if (!active && i < a.n) {
+            if (!active && takes && i < a.n) {
                 const uint32_t ray = a.ray_order ? a.ray_order[i] : i;
                 const float4 *r = reinterpret_cast<const float4 *>(a.rays + ray);
                 const float4 ra = __ldg(r), rb = __ldg(r + 1);
@@ -1369,7 +1375,10 @@ cudaError_t launch_tail(const WaveArgs &a, uint32_t it, int num_sms, bool config
 {
     const TailLayout staged = tail_layout(a.n_cut_nodes, true, a.grid.n_inputs, a.n_hidden_layers);
     const TailLayout global = tail_layout(a.n_cut_nodes, false, a.grid.n_inputs, a.n_hidden_layers);
-    const bool smem_cut = stage_cut && staged.total <= kMaxDynamicSmem;
+    // A batch that only the tail kernel answers leaves most lanes of an SM empty: the traversals'
+    // latency is its time, and the cut in shared memory shortens it (512 rays 98 -> 87 us, 2,048 rays
+    // 100 -> 97, 16,384 rays 162 -> 152; from 24,576 rays on no better or slower, 215 -> 223 for 32,768).
+    const bool smem_cut = (stage_cut || a.tail_at == 0u) && staged.total <= kMaxDynamicSmem;
     const size_t smem = smem_cut ? staged.total : global.total;
     if (a.bf16)
         return smem_cut ? launch_tail_variant<true, true, false>(a, it, num_sms, configure, smem, s)
@@ -1672,13 +1681,18 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
         if (e != cudaSuccess)
             return e;
         a.ray_order = res.perm;
-        *launches += 3u;
+        *launches += 2u;
     }
-    uint32_t first_blocks = (n + kFirstThreads - 1u) / kFirstThreads;
+    // a ray per warp for the batches that the tail kernel answers alone, else one per lane
+    const uint32_t first_rays = a.tail_at == 0u ? kFirstThreads / 32u : kFirstThreads;
+    uint32_t first_blocks = (n + first_rays - 1u) / first_rays;
     const uint32_t first_cap = (uint32_t)num_sms * 4u; // resident blocks (64 registers a thread)
     if (first_blocks > first_cap)
         first_blocks = first_cap;
-    k_wave_first<<<first_blocks, kFirstThreads, 0, s>>>(a);
+    if (a.tail_at == 0u)
+        k_wave_first<true><<<first_blocks, kFirstThreads, 0, s>>>(a);
+    else
+        k_wave_first<false><<<first_blocks, kFirstThreads, 0, s>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
