@@ -435,8 +435,8 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 // ---------------------------------------------------------------------------------------------
 // Training forward + composite loss + backward on the tensor cores (K3/K4 backward).
 //
-// k_encode_rows writes each row's FP16 features; then one CTA per SM (256 threads, two per tile row
-// and TMEM lane) runs 128-row tiles through
+// k_encode_rows writes each row's FP16 features; then one CTA per SM (two threads per tile row and
+// TMEM lane, a warp that issues the MMAs and one that copies the next tile) runs 128-row tiles through
 //   forward   Z_{j+1} = X_j W_j^T for every matrix j (tcgen05, M = 128 rows), the ReLU'd 16-bit
 //             activations X_{j+1} written back to shared memory (and their ReLU masks kept in
 //             registers), then the sigmoid, the composite loss and dZ_out = dL/dZ_out;
@@ -452,13 +452,19 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 // ---------------------------------------------------------------------------------------------
 
 constexpr uint32_t kTcRows = 128;
-// Two threads per tile row, each with half of its columns: the step is bound by the chain MMA ->
-// accumulator read -> rounding -> shared-memory tile -> next MMA, ten times per tile, and the half
-// rows shorten its epilogues. With that, the input tiles by cp.async, the weight-gradient MMAs under
-// the next epilogue and the MMAs issued from uniform registers (tc::elect_one) a pass over 2^18 rows
-// went from 218 to 188 us; only the last of the four shows alone (215 us without it), since the chain
-// waited for the MMAs to be issued.
-constexpr uint32_t kTcThreads = 256;
+// The chain MMA -> accumulator read -> rounding -> shared-memory tile -> next MMA bounds the kernel, ten
+// times per tile (20,000 cycles; the tensor cores need some 5,500 of them). What shortens it, us per 2^18
+// rows, 128 inputs, 4 hidden layers: two threads per row with half of its columns, input tiles by cp.async
+// and the weight-gradient MMAs under the next epilogue 218 -> 215; MMAs issued from uniform registers
+// (tc::elect_one) 188 (waiting for them to be issued hid the rest before); a warp of their own for the
+// MMAs, every warp waiting for itself, one barrier per step, the next tile's layer 0 under dX_0's
+// epilogue and the targets read ahead 155; a second warp that copies the next tile apart from the steps
+// 145 (the MMA warp spent 100 cycles on each 512-byte copy, which the next barrier waited for); the next step's
+// descriptors made before the barrier 142. The row warps' stores of dX_0 through shared memory, 64 bytes of 8 rows
+// at a time instead of 16 bytes of 32, changed nothing.
+constexpr uint32_t kTcRowThreads = 256;               // two per tile row
+constexpr uint32_t kTcStepThreads = kTcRowThreads + 32u; // and the warp that issues the MMAs
+constexpr uint32_t kTcThreads = kTcStepThreads + 32u;    // and the one that copies the next tile
 constexpr uint32_t kColBlock = kTcRows * 16u; // bytes between 8-column blocks of a row tile
 constexpr uint32_t kTcAccCols = 128;          // TMEM columns of the current layer's accumulator
 constexpr uint32_t kTcTmemCols = 512;
@@ -489,6 +495,7 @@ struct TrainTcArgs {
     uint32_t dz_off[2], dzo_off, bar_off; // dZ_j alternates between two tiles (one where only one fits)
     uint32_t loss_off;                    // [kTcRows] loss of each row's upper four channels
     uint32_t wg_col[kTcMaxMatrices];      // TMEM column of the dW_j^T accumulator
+    uint32_t acc0_col;                    // layer 0's accumulator (0: that of the other layers and dX_j)
     uint64_t wait_ns;                     // time limit of the phase waits
     uint32_t stall;                       // failure-path test: wait on an mbarrier nothing arrives at
 };
@@ -517,6 +524,13 @@ __device__ __forceinline__ void store_row_chunks(unsigned char *tile, uint32_t r
             make_uint4(words[4u * c], words[4u * c + 1u], words[4u * c + 2u], words[4u * c + 3u]);
 }
 
+// The operands of one chain of MMAs (tc::mma_chain): D, A and B with their steps, the instruction
+// descriptor and the number of MMAs (0: no chain).
+struct TcChain {
+    uint64_t a_desc, b_desc;
+    uint32_t d, a_step, b_step, idesc, count;
+};
+
 template <bool BF16, bool FP8>
 __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constant__ TrainTcArgs a)
 {
@@ -526,17 +540,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     const uint32_t n_tiles = (a.n + kTcRows - 1u) / kTcRows;
     if (blockIdx.x >= n_tiles)
         return;
-    // this thread's tile row (= TMEM lane) and half of its columns
+    // this thread's tile row (= TMEM lane) and half of its columns; the last two warps have none
     const uint32_t tid = threadIdx.x & (kTcRows - 1u), half = threadIdx.x / kTcRows, warp = tid >> 5;
     const bool issuer = threadIdx.x == 0u;
-    const bool mma_warp = __shfl_sync(kFull, threadIdx.x >> 5, 0) == 0u; // allocates TMEM, issues the MMAs
-    // weights, mma, one nothing arrives at (failure-path test), end
+    const uint32_t role = __shfl_sync(kFull, threadIdx.x >> 5, 0);
+    const bool mma_warp = role == kTcRowThreads / 32u; // allocates TMEM, issues the MMAs
+    const bool copy_warp = role == kTcStepThreads / 32u;
+    // weights, layers 1 to H and backward, one nothing arrives at (failure-path test), end, layer 0, next tile
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + a.bar_off);
-    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 4);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(bars + 6);
     float *upper_loss = reinterpret_cast<float *>(smem + a.loss_off);
     const uint32_t base = tc::smem_addr(smem);
     const uint32_t bar_w = tc::smem_addr(&bars[0]), bar_mma = tc::smem_addr(&bars[1]),
-                   bar_end = tc::smem_addr(&bars[3]);
+                   bar_end = tc::smem_addr(&bars[3]), bar_0 = tc::smem_addr(&bars[4]), bar_x = tc::smem_addr(&bars[5]);
     const uint32_t x0_bytes = K0 * kTcRows * 2u;
 
     if (mma_warp) {
@@ -544,7 +560,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
         tc::tmem_relinquish();
     }
     if (issuer) {
-        for (uint32_t b = 0; b < 4u; b++)
+        for (uint32_t b = 0; b < 6u; b++)
             tc::mbar_init(tc::smem_addr(&bars[b]), 1u);
         tc::mbar_init_fence();
     }
@@ -554,15 +570,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     const uint32_t tmem = *slot;
     const uint32_t lane_off = (32u * warp) << 16; // this warp's TMEM lanes
 
-    // This thread's 16-byte pieces of tile t's input rows (zeros past the batch), K0 / 16 of them:
-    // neighbouring lanes take the two halves of a 32-byte sector. (As sixteen TMA boxes of 128 x 16
-    // bytes the tile took 9,000 of the 34,000 cycles a tile needs, and its issuing thread with it.)
-    auto load_tile = [&](uint32_t t, uint32_t buf) {
-        const uint32_t r = (threadIdx.x >> 1) & (kTcRows - 1u), row = t * kTcRows + r, odd = threadIdx.x & 1u;
-        const __half *src = a.features + (size_t)(row < a.n ? row : 0u) * K0 + 8u * odd;
-        const uint32_t dst = base + a.x0_off + buf * x0_bytes + odd * kColBlock + r * 16u;
-        for (uint32_t c = 0; c < K0 / 16u; c++)
-            tc::copy16_async(dst + 2u * c * kColBlock, src + 16u * c, row < a.n);
+    // Pieces q0 to q1 of tile t's input rows, 512 bytes each by one warp (zeros past the batch): 8 rows and
+    // 4 chunks of 16 bytes, which meet in no shared-memory bank. (As sixteen TMA boxes of 128 x 16 bytes
+    // the tile took 9,000 of the 34,000 cycles a tile needed, and its issuing thread with it.)
+    const uint32_t chunks = K0 / 8u, pieces = (kTcRows / 8u) * ((chunks + 3u) / 4u);
+    auto load_tile = [&](uint32_t t, uint32_t buf, uint32_t q0, uint32_t q1) {
+        const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll 4
+        for (uint32_t q = q0; q < q1; q++) {
+            const uint32_t r = 8u * (q & 15u) + (lane >> 2), c = 4u * (q >> 4) + (lane & 3u), row = t * kTcRows + r;
+            if (c < chunks)
+                tc::copy16_async(base + a.x0_off + buf * x0_bytes + c * kColBlock + r * 16u,
+                                 a.features + (size_t)(row < a.n ? row : 0u) * K0 + 8u * c, row < a.n);
+        }
     };
     uint32_t t = blockIdx.x;
     if (issuer) {
@@ -571,58 +591,123 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
             tc::bulk_load(base + o, reinterpret_cast<const unsigned char *>(a.wpacked) + o,
                           a.wbytes - o < 16384u ? a.wbytes - o : 16384u, bar_w);
     }
-    load_tile(t, 0u);
+    for (uint32_t q = threadIdx.x >> 5; q < pieces; q += kTcThreads / 32u)
+        load_tile(t, 0u, q, q + 1u);
+    tc::copy_async_wait();
+    tc::fence_async_shared(); // the tile's pieces are read by the MMAs
     bool ok = issuer ? tc::mbar_wait(bar_w, 0u, a.wait_ns) : true;
     if (a.stall && issuer) // nothing ever arrives at this barrier: the wait runs out
         ok = ok && tc::mbar_wait(tc::smem_addr(&bars[2]), 0u, a.wait_ns);
     ok = __syncthreads_and(ok);
 
-    uint32_t ph_mma = 0u, buf = 0u;
-    bool mma_pending = false, first_tile = true;
+    uint32_t ph_mma = 0u, ph_0 = 0u, ph_x = 0u, buf = 0u;
+    bool first_tile = true;
     float loss_acc = 0.f;
-    // waits for the MMAs committed so far; false (everyone) if the wait gave up
-    auto mma_done = [&]() -> bool {
-        bool r = issuer ? tc::mbar_wait(bar_mma, ph_mma, a.wait_ns) : true;
-        r = __syncthreads_and(r);
-        if (r) {
-            ph_mma ^= 1u;
-            mma_pending = false;
-            tc::fence_after_sync();
-        }
+    // Per step one warp issues the MMAs; the row warps wait for those that the epilogue reads, each thread
+    // for itself, and write the tiles of the next step. One barrier ends the step and tells everyone if a
+    // wait gave up. The last warp keeps out of the steps: it copies the next tile into the other buffer.
+    auto mma_done = [&](uint32_t bar, uint32_t &phase) -> bool {
+        const bool r = __all_sync(kFull, tc::mbar_wait(bar, phase, a.wait_ns));
+        phase ^= 1u;
+        tc::fence_after_sync();
         return r;
     };
+    bool fine = ok; // this warp's waits; ok is the block's, from the last barrier
+    if (copy_warp) {
+        for (; fine && t + gridDim.x < n_tiles; t += gridDim.x, buf ^= 1u) {
+            // layer 0's commit covers the MMAs of the tile before, the other buffer's last readers
+            if (!(fine = mma_done(bar_0, ph_0)))
+                break;
+            load_tile(t + gridDim.x, buf ^ 1u, 0u, pieces);
+            tc::copy_async_wait();
+            tc::fence_async_shared();
+            __syncwarp();
+            if (tc::elect_one())
+                tc::mbar_arrive(bar_x);
+        }
+        first_tile = !ok; // as for the warps below, which run at least one tile
+        t = n_tiles;
+    }
     for (; ok && t < n_tiles; t += gridDim.x, buf ^= 1u) {
-        tc::copy_async_wait();
-        tc::fence_async_shared(); // the tile's pieces are read by the MMAs
-        __syncthreads();
         const uint32_t x0_addr = base + a.x0_off + buf * x0_bytes;
         auto x_addr = [&](uint32_t j) { return j == 0u ? x0_addr : base + a.x_off[j]; };
+        // the MMAs of a step, described before the barrier that starts it
+        auto forward_chain = [&](uint32_t j) { // Z_{j+1} = X_j W_j^T
+            const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
+            TcChain c;
+            c.d = tmem + (j == 0u ? a.acc0_col : 0u);
+            c.a_desc = tc::smem_desc(x_addr(j), kColBlock, 128u);
+            c.a_step = kColBlock / 8u;
+            c.b_desc = tc::smem_desc(base + tc_w_off(j, K0), nout * 16u, 128u);
+            c.b_step = 2u * nout;
+            c.idesc = tc::idesc_f16(kTcRows, nout, BF16);
+            c.count = nin / 16u;
+            return c;
+        };
+        auto dz_addr = [&](uint32_t j) { return base + (j > H ? a.dzo_off : a.dz_off[j & 1u]); };
+        auto dgrad_chain = [&](uint32_t j) { // dX_j (128 x nin) = dZ_{j+1} (128 x nout) . W_j (nout x nin), W_j MN-major
+            const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
+            TcChain c;
+            c.d = tmem;
+            c.a_desc = tc::smem_desc(dz_addr(j + 1u), kColBlock, 128u);
+            c.a_step = kColBlock / 8u;
+            c.b_desc = tc::smem_desc(base + tc_w_off(j, K0), 128u, nout * 16u);
+            c.b_step = 16u;
+            c.idesc = tc::idesc_f16_major(kTcRows, nin, BF16, false, true);
+            c.count = j > a.min_matrix || (j == 0u && a.emit) ? nout / 16u : 0u;
+            return c;
+        };
+        auto wgrad_chain = [&](uint32_t j) { // dW_j^T (128 x nout; rows >= nin unused) += X_j^T . dZ_{j+1}, K = the 128 rows
+            const uint32_t nout = tc_n_out(j, H);
+            TcChain c;
+            c.d = tmem + a.wg_col[j];
+            c.a_desc = tc::smem_desc(x_addr(j), 128u, kColBlock);
+            c.a_step = 16u;
+            c.b_desc = tc::smem_desc(dz_addr(j + 1u), 128u, kColBlock);
+            c.b_step = 16u;
+            c.idesc = tc::idesc_f16_major(kTcRows, nout, BF16, true, true);
+            c.count = ((a.wg_mask >> j) & 1u) ? kTcRows / 16u : 0u;
+            return c;
+        };
+        auto issue = [&](const TcChain &c, uint32_t accumulate) {
+            tc::mma_chain(c.d, c.a_desc, c.a_step, c.b_desc, c.b_step, c.idesc, c.count, accumulate);
+        };
+        TcChain next = forward_chain(0u), next_w = {};
         const uint32_t row = t * kTcRows + tid;
         const bool valid = row < a.n;
-        uint32_t relu_mask[kTcMaxMatrices]; // bit c: column 32 * half + c of X_j's row
+        float4 tgt = make_float4(0.f, 0.f, 0.f, 0.f);
+        float target_vis = 0.f;
+        if (valid && !mma_warp) { // read here, under the forward layers
+            tgt = __ldg(reinterpret_cast<const float4 *>(a.targets + (size_t)row * 8u) + half);
+            target_vis = __ldg(a.targets + (size_t)row * 8u);
+        }
+        uint32_t relu_mask[kTcMaxMatrices]; // bits c and 16 + c: columns 32 * half + 2 c and + 2 c + 1 of X_j's row
         float row_loss = 0.f;
         // ---------------- forward ----------------
         for (uint32_t j = 0; j <= H && ok; j++) {
-            const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
-            if (mma_warp && tc::elect_one()) {
-                tc::fence_after_sync();
-                const uint32_t idesc = tc::idesc_f16(kTcRows, nout, BF16);
-                const uint32_t w_addr = base + tc_w_off(j, K0), a_addr = x_addr(j);
-                tc::mma_chain(tmem, tc::smem_desc(a_addr, kColBlock, 128u), kColBlock / 8u,
-                              tc::smem_desc(w_addr, nout * 16u, 128u), 2u * nout, idesc, nin / 16u, 0u);
-                tc::mma_commit(bar_mma);
-            }
-            mma_pending = true;
-            if (!(ok = mma_done()))
-                break;
-            // the other buffer's last readers, the previous tile's MMAs, are done as well
-            if (j == 0u && t + gridDim.x < n_tiles)
-                load_tile(t + gridDim.x, buf ^ 1u);
-            if (j < H) { // X_{j+1} = relu(Z_{j+1}) in the MLP precision (FP8 mode: E4M3 into hidden matrices)
+            const uint32_t acc = tmem + (j == 0u ? a.acc0_col : 0u);
+            if (mma_warp) {
+                if (j == 0u && !first_tile) // the copy of this tile
+                    fine = fine && mma_done(bar_x, ph_x);
+                if (fine && tc::elect_one()) {
+                    tc::fence_after_sync();
+                    issue(next, 0u);
+                    tc::mma_commit(j == 0u ? bar_0 : bar_mma);
+                }
+                __syncwarp();
+                if (j < H) {
+                    next = forward_chain(j + 1u);
+                } else {
+                    next = dgrad_chain(H);
+                    next_w = wgrad_chain(H);
+                }
+            } else if (!(fine = fine && (j == 0u ? mma_done(bar_0, ph_0) : mma_done(bar_mma, ph_mma)))) {
+                // nothing to read
+            } else if (j < H) { // X_{j+1} = relu(Z_{j+1}) in the MLP precision (FP8 mode: E4M3 into hidden matrices)
                 uint32_t v[2][16];
 #pragma unroll
                 for (int q = 0; q < 2; q++)
-                    tc::tmem_ld16(tmem + lane_off + 32u * half + 16u * q, v[q]);
+                    tc::tmem_ld16(acc + lane_off + 32u * half + 16u * q, v[q]);
                 tc::tmem_wait_ld();
                 uint32_t packed[16];
                 const bool quant = FP8 && j + 1u < H;
@@ -633,7 +718,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                     const float hi = __uint_as_float(v[c >> 3][(2 * c + 1) & 15]);
                     const uint32_t p = quant ? fp8_act_relu_half2(lo, hi) : pack_relu<BF16>(lo, hi);
                     packed[c] = p;
-                    m |= (((p & 0xFFFFu) != 0u ? 1u : 0u) | ((p >> 16) != 0u ? 2u : 0u)) << (2 * c);
+                    m |= tc::nonzero_halves<BF16>(p) & (0x00010001u << c);
                 }
                 relu_mask[j + 1u] = m;
                 store_row_chunks(smem + a.x_off[j + 1u] + 4u * half * kColBlock, tid, packed, 4u);
@@ -641,12 +726,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                 uint32_t v[8];
                 tc::tmem_ld8(tmem + lane_off, v);
                 tc::tmem_wait_ld();
-                float4 tgt = make_float4(0.f, 0.f, 0.f, 0.f);
-                float target_vis = 0.f;
-                if (valid) {
-                    tgt = __ldg(reinterpret_cast<const float4 *>(a.targets + (size_t)row * 8u) + half);
-                    target_vis = __ldg(a.targets + (size_t)row * 8u);
-                }
                 const float t4[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
                 float dz[4], val[4];
 #pragma unroll
@@ -669,7 +748,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
             }
             tc::fence_async_shared(); // the tile rows written above are read by the next MMAs
             tc::fence_before_sync();
-            __syncthreads();
+            ok = fine = tc::barrier_and(1u, kTcStepThreads, fine);
         }
         if (ok && half == 0u) {
             row_loss += upper_loss[tid];
@@ -680,38 +759,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
         // ---------------- backward ----------------
         for (int jj = (int)H; jj >= (int)a.min_matrix && ok; jj--) {
             const uint32_t j = (uint32_t)jj;
-            const uint32_t nout = tc_n_out(j, H), nin = tc_n_in(j, K0);
-            const uint32_t dz_addr = base + (j == H ? a.dzo_off : a.dz_off[(j + 1u) & 1u]);
             const bool dgrad = j > a.min_matrix || (j == 0u && a.emit);
-            const bool wgrad = (a.wg_mask >> j) & 1u;
             // With two dZ tiles the epilogue only waits for dX_j; dW_j's MMAs run under it. A later commit
             // covers them, so they are done before the next step writes the tile they read (its own
             // commit comes after them), before the next tile overwrites X_j, and at the end.
             const bool overlap = dgrad && a.dz_off[0] != a.dz_off[1];
-            if (mma_warp && tc::elect_one()) {
-                tc::fence_after_sync();
-                if (dgrad) { // dX_j (128 x nin) = dZ_{j+1} (128 x nout) . W_j (nout x nin), W_j MN-major
-                    const uint32_t idesc = tc::idesc_f16_major(kTcRows, nin, BF16, false, true);
-                    const uint32_t w_addr = base + tc_w_off(j, K0);
-                    tc::mma_chain(tmem, tc::smem_desc(dz_addr, kColBlock, 128u), kColBlock / 8u,
-                                  tc::smem_desc(w_addr, 128u, nout * 16u), 16u, idesc, nout / 16u, 0u);
+            const bool last = j == a.min_matrix;
+            if (mma_warp) {
+                if (tc::elect_one()) {
+                    tc::fence_after_sync();
+                    issue(next, 0u);
                     if (overlap)
                         tc::mma_commit(bar_mma);
+                    issue(next_w, first_tile ? 0u : 1u);
+                    if (dgrad && !overlap)
+                        tc::mma_commit(bar_mma);
                 }
-                if (wgrad) { // dW_j^T (128 x nout; rows >= nin unused) += X_j^T . dZ_{j+1}, K = the 128 rows
-                    const uint32_t idesc = tc::idesc_f16_major(kTcRows, nout, BF16, true, true);
-                    const uint32_t xa = x_addr(j);
-                    static_assert(kTcRows / 16u == 8u, "one chain");
-                    tc::mma_chain(tmem + a.wg_col[j], tc::smem_desc(xa, 128u, kColBlock), 16u,
-                                  tc::smem_desc(dz_addr, 128u, kColBlock), 16u, idesc, 8u, first_tile ? 0u : 1u);
+                __syncwarp();
+                if (!last) {
+                    next = dgrad_chain(j - 1u);
+                    next_w = wgrad_chain(j - 1u);
                 }
-                if (!overlap)
-                    tc::mma_commit(bar_mma);
-            }
-            mma_pending = true;
-            if (!(ok = mma_done()))
-                break;
-            if (j >= 1u && j > a.min_matrix) { // dZ_j = dX_j * (X_j > 0), 16-bit
+            } else if (dgrad && !(fine = fine && mma_done(bar_mma, ph_mma))) {
+                // nothing to read
+            } else if (j >= 1u && j > a.min_matrix) { // dZ_j = dX_j * (X_j > 0), 16-bit
                 uint32_t v[2][16];
 #pragma unroll
                 for (int q = 0; q < 2; q++)
@@ -721,10 +792,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                 uint32_t packed[16];
 #pragma unroll
                 for (int c = 0; c < 16; c++) {
-                    const uint32_t bits = (m >> (2 * c)) & 3u;
-                    const float lo = (bits & 1u) ? __uint_as_float(v[c >> 3][(2 * c) & 15]) : 0.f;
-                    const float hi = (bits & 2u) ? __uint_as_float(v[c >> 3][(2 * c + 1) & 15]) : 0.f;
-                    packed[c] = Pr::pack(lo, hi);
+                    const uint32_t p = Pr::pack(__uint_as_float(v[c >> 3][(2 * c) & 15]),
+                                                __uint_as_float(v[c >> 3][(2 * c + 1) & 15]));
+                    packed[c] = p & tc::fill_halves(m << (15 - c));
                 }
                 store_row_chunks(smem + a.dz_off[j & 1u] + 4u * half * kColBlock, tid, packed, 4u);
             } else if (j == 0u && a.emit) { // dX_0, rounded to the MLP precision, for the grid scatter
@@ -748,18 +818,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
                     }
                 }
             }
+            // With an accumulator of its own the next tile's layer 0 runs under dX_0's epilogue; its commit
+            // covers this tile's last MMAs.
+            if (last && a.acc0_col != 0u)
+                break;
             tc::fence_async_shared();
             tc::fence_before_sync();
-            __syncthreads();
+            ok = fine = tc::barrier_and(1u, kTcStepThreads, fine);
         }
         first_tile = false;
     }
-    if (ok && !first_tile) { // the last weight-gradient MMAs
-        if (mma_warp && tc::elect_one())
-            tc::mma_commit(bar_end);
-        ok = issuer ? tc::mbar_wait(bar_end, 0u, a.wait_ns) : true;
-        ok = __syncthreads_and(ok);
-        tc::fence_after_sync();
+    if (!first_tile) { // the last weight-gradient MMAs
+        tc::fence_before_sync();
+        ok = __syncthreads_and(fine);
+        if (ok) {
+            if (mma_warp && tc::elect_one())
+                tc::mma_commit(bar_end);
+            ok = tc::mbar_wait(bar_end, 0u, a.wait_ns);
+            ok = __syncthreads_and(ok);
+            tc::fence_after_sync();
+        }
     }
     if (!ok) {
         // a wait ran out: record it, give copies and MMAs still in flight one more bounded wait
@@ -768,12 +846,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
             a.wpart[(size_t)blockIdx.x * a.n_network + i] = 0.f;
         if (mma_warp && tc::elect_one()) {
             atomicOr(a.status, 1u);
-            if (mma_pending)
-                tc::mbar_wait(bar_mma, ph_mma);
-            tc::mma_commit(bar_end); // MMAs without a commit of their own
+            tc::mma_commit(bar_end); // covers every MMA issued
             tc::mbar_wait(bar_end, 0u);
         }
-    } else if (!first_tile) {
+    } else if (!first_tile && !mma_warp && !copy_warp) {
         // the CTA's weight gradients: lane m of the dW_j^T accumulator holds column m of dW_j
         for (uint32_t j = 0; j <= H; j++) {
             if (!((a.wg_mask >> j) & 1u))
@@ -1053,6 +1129,7 @@ bool plan_train_pass(uint32_t n_in, uint32_t H, uint32_t mask, bool emit, TrainT
         a.wg_col[j] = col;
         col += tc_n_out(j, H);
     }
+    a.acc0_col = col + kNeurons <= kTcTmemCols ? col : 0u;
     if (col > kTcTmemCols || off > kTcSmemLimit)
         return false;
     uint32_t lo = H;

@@ -74,6 +74,27 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+
+// __syncthreads_and over the first `threads` threads of the block (whole warps), on barrier `id`
+__device__ __forceinline__ bool barrier_and(uint32_t id, uint32_t threads, bool v)
+{
+    uint32_t r;
+    asm volatile("{\n"
+                 ".reg .pred p, q;\n"
+                 "setp.ne.u32 p, %3, 0;\n"
+                 "barrier.cta.red.and.pred q, %1, %2, p;\n"
+                 "selp.u32 %0, 1, 0, q;\n"
+                 "}\n"
+                 : "=r"(r)
+                 : "r"(id), "r"(threads), "r"(v ? 1u : 0u)
+                 : "memory");
+    return r != 0u;
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
@@ -155,6 +176,24 @@ __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fenc
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 // Makes generic-proxy shared-memory writes visible to the tensor core (async proxy).
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
+// 0xFFFF in each half of a pair of FP16 or BF16 values that is not zero (NaN is not)
+template <bool BF16>
+__device__ __forceinline__ uint32_t nonzero_halves(uint32_t p)
+{
+    if constexpr (BF16)
+        return __hneu2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&p), __floats2bfloat162_rn(0.f, 0.f));
+    else
+        return __hneu2_mask(*reinterpret_cast<const __half2 *>(&p), __floats2half2_rn(0.f, 0.f));
+}
+
+// each half filled with its top bit
+__device__ __forceinline__ uint32_t fill_halves(uint32_t v)
+{
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, 0xBB99;\n" : "=r"(r) : "r"(v)); // bytes 1 and 3, their sign bit replicated
+    return r;
+}
 
 // One lane of a fully converged warp (always the same one). MMAs are issued inside
 // `if (warp index, made uniform by a shuffle) if (elect_one())`: the compiler then keeps their
