@@ -329,6 +329,57 @@ __global__ void __launch_bounds__(kRayBinThreads) k_ray_bins(const __grid_consta
             atomicAdd(&a.bins[b], cnt[b]);
 }
 
+// The same for rows of points (launch_row_order): the bin is the Morton code of the row's middle point's cell
+// in a 32 x 16 x 16 grid over the unit cube.
+constexpr uint32_t kRowBins = 8192;
+static_assert(kRowBins <= kRayBins, "k_ray_bin_place serves both");
+struct RowBinArgs {
+    const float *positions; // n x n_points x 3
+    uint32_t n, n_points;
+    uint16_t *keys;
+    uint32_t *bins;
+};
+__device__ __forceinline__ uint32_t row_cell(const float *__restrict__ p)
+{
+    auto axis = [](float x, float s) { // NaN -> 0
+        const float c = x * s;
+        return c >= s - 1.0f ? (uint32_t)s - 1u : (c > 0.0f ? (uint32_t)c : 0u);
+    };
+    const uint32_t x = axis(__ldg(p), 32.0f), y = axis(__ldg(p + 1), 16.0f), z = axis(__ldg(p + 2), 16.0f);
+    uint32_t m = x & 1u; // the fifth bit of x is the lowest of the code
+#pragma unroll
+    for (uint32_t b = 0; b < 4u; b++)
+        m |= (((x >> (b + 1u)) & 1u) | (((y >> b) & 1u) << 1) | (((z >> b) & 1u) << 2)) << (3u * b + 1u);
+    return m;
+}
+__global__ void __launch_bounds__(kRayBinThreads) k_row_bins(const __grid_constant__ RowBinArgs a)
+{
+    __shared__ uint32_t cnt[kRowBins];
+    for (uint32_t b = threadIdx.x; b < kRowBins; b += blockDim.x)
+        cnt[b] = 0u;
+    __syncthreads();
+    uint32_t r0, r1;
+    ray_chunk(a.n, r0, r1);
+    for (uint32_t i = r0 + threadIdx.x; i < r1; i += kRaysAtOnce * blockDim.x) {
+        uint32_t b[kRaysAtOnce];
+#pragma unroll
+        for (uint32_t j = 0; j < kRaysAtOnce; j++) { // past the chunk: the first row again
+            const uint32_t r = i + j * blockDim.x < r1 ? i + j * blockDim.x : i;
+            b[j] = row_cell(a.positions + ((size_t)r * a.n_points + a.n_points / 2u) * 3u);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kRaysAtOnce; j++)
+            if (i + j * blockDim.x < r1) {
+                a.keys[i + j * blockDim.x] = (uint16_t)b[j];
+                atomicAdd(&cnt[b[j]], 1u);
+            }
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < kRowBins; b += blockDim.x)
+        if (cnt[b])
+            atomicAdd(&a.bins[b], cnt[b]);
+}
+
 // Places the ray ids bin by bin: each block takes the same chunk as k_ray_bins, counts it per bin
 // again in shared memory, reserves one range per non-empty bin, then places its rays with
 // shared-memory atomics (the order inside a bin does not matter). A thread's kRayBinsPerThread bins are
@@ -1573,6 +1624,25 @@ cudaError_t launch_ray_order(const nbvh_ray *rays, uint32_t n, const float scene
         return e;
     k_ray_bins<<<blocks, kRayBinThreads, 0, s>>>(rb);
     k_ray_bin_place<<<blocks, kRayBinThreads, 0, s>>>(rb);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_row_order(const float *positions, uint32_t n, uint32_t n_points, uint16_t *keys, uint32_t *bins,
+                             uint32_t *order, int num_sms, cudaStream_t s)
+{
+    if (n == 0)
+        return cudaSuccess;
+    const RowBinArgs a = {positions, n, n_points, keys, bins};
+    RayBinArgs place = {};
+    place.n = n;
+    place.keys = keys;
+    place.bins = bins;
+    place.order = order;
+    cudaError_t e = cudaMemsetAsync(bins, 0, kRayBinWords * sizeof(uint32_t), s);
+    if (e != cudaSuccess)
+        return e;
+    k_row_bins<<<(uint32_t)num_sms, kRayBinThreads, 0, s>>>(a);
+    k_ray_bin_place<<<(uint32_t)num_sms, kRayBinThreads, 0, s>>>(place);
     return cudaGetLastError();
 }
 

@@ -362,21 +362,27 @@ __device__ __forceinline__ void composite_loss(const LossConsts &lc, uint32_t ch
 // L / LPS threads instead, one store each; batches too small to fill the GPU otherwise are bound by
 // the latency of one thread's gathers, level after level (3,001 rows: 37 -> 15 us). Large batches are
 // bound by the L1's misses to L2 (ncu: L1 88%, L2 68%); 4-byte stores, sixteen partial sectors a
-// point, were the rest of 289 us per 2^18 rows, 222 now (264 -> 206 in a training step).
+// point, were the rest of 289 us per 2^18 rows, 222 now; large training batches come in an order that
+// brings neighbours together (kRowOrderMin).
 // ---------------------------------------------------------------------------------------------
 template <uint32_t F>
 __global__ void __launch_bounds__(256, 4) k_encode_rows(const __grid_constant__ GridParams grid,
                                                      const uint32_t *__restrict__ table,
                                                      const float *__restrict__ positions, uint32_t n,
-                                                     __half *__restrict__ feat, uint32_t bf16_, uint32_t split)
+                                                     __half *__restrict__ feat, uint32_t bf16_, uint32_t split,
+                                                     const uint32_t *__restrict__ order)
 {
     constexpr uint32_t LPS = 8u / F;
     const uint32_t P = grid.n_points, L = grid.n_levels, G = split ? L / LPS : 1u, LG = L / G;
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= (uint64_t)n * P * G)
         return;
-    const uint64_t i = w / G; // (row, point)
+    uint64_t i = w / G; // (row, point)
     const uint32_t l0 = (uint32_t)(w - i * G) * LG;
+    if (order) {
+        const uint64_t r = i / P;
+        i = (uint64_t)__ldg(order + r) * P + (i - r * P);
+    }
     const float *src = positions + i * 3u;
     const V3 pos = mk3(__ldg(src), __ldg(src + 1), __ldg(src + 2));
     const bool bf16 = bf16_ != 0u;
@@ -415,7 +421,7 @@ __global__ void __launch_bounds__(256, 4) k_encode_rows(const __grid_constant__ 
 }
 
 cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const float *positions, uint32_t n,
-                        __half *features, bool bf16, int num_sms, cudaStream_t s)
+                        __half *features, bool bf16, int num_sms, cudaStream_t s, const uint32_t *order = nullptr)
 {
     const uint32_t lps = 8u / grid.n_features, groups = grid.n_levels / lps;
     const uint64_t points = (uint64_t)n * grid.n_points, lanes = (uint64_t)num_sms * 2048u;
@@ -424,11 +430,11 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
     const unsigned blocks = (unsigned)((threads + 255u) / 256u);
     const uint32_t b = bf16 ? 1u : 0u, sp = split ? 1u : 0u;
     if (grid.n_features == 4u)
-        k_encode_rows<4><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+        k_encode_rows<4><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp, order);
     else if (grid.n_features == 8u)
-        k_encode_rows<8><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+        k_encode_rows<8><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp, order);
     else
-        k_encode_rows<2><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp);
+        k_encode_rows<2><<<blocks, 256, 0, s>>>(grid, table, positions, n, features, b, sp, order);
     return cudaGetLastError();
 }
 
@@ -1236,6 +1242,15 @@ cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, u
     return encode_rows(grid, table, positions, n, features, bf16, num_sms, s);
 }
 
+// Batches of at least this many rows are encoded in the order of launch_row_order: rows of one place share
+// entries of the coarser levels in the L1 (encoding 2^18 random rows 224 -> 172 us). Their gradients are
+// scattered in batch order, where neighbours rarely meet on an entry (344 us, 530 in place order). The ordering
+// costs some 30 us whatever the batch: gradients of 65,536 rows 286 -> 297 us, 131,072 437 -> 437, 196,608
+// 619 -> 608, 262,144 776 -> 754.
+constexpr uint32_t kRowOrderMin = 3u << 16;
+// order, bins and keys in the buffer of at least 16 halves per row
+static_assert((size_t)kRowOrderMin * 32u >= (size_t)kRowOrderMin * 6u + 4u * (kRayBinWords + 4u), "the order fits");
+
 cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
                               __half *features, __half *dfeat, __half *wpacked, float *wpart, float *grad,
@@ -1251,7 +1266,17 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
     const uint32_t n_network_params =
         kNeurons * n_in + (H - 1u) * kNeurons * kNeurons + kOutputsPadded * kNeurons;
     const uint32_t *table = reinterpret_cast<const uint32_t *>(params_h + n_network_params);
-    e = encode_rows(grid, table, positions, n, features, bf16, num_sms, s);
+    const uint32_t *order = nullptr;
+    if (n >= kRowOrderMin) { // the feature gradients are written after the encoding: their buffer holds the order
+        uint32_t *words = reinterpret_cast<uint32_t *>(dfeat);
+        uint32_t *bins = words + ((size_t)n + 3u) / 4u * 4u;
+        e = launch_row_order(positions, n, grid.n_points, reinterpret_cast<uint16_t *>(bins + kRayBinWords), bins, words,
+                             num_sms, s);
+        if (e != cudaSuccess)
+            return e;
+        order = words;
+    }
+    e = encode_rows(grid, table, positions, n, features, bf16, num_sms, s, order);
     if (e == cudaSuccess)
         e = launch_pack_weights(params_h, n_in, H, wpacked, s, clear ? status : nullptr,
                                 clear ? reinterpret_cast<uint32_t *>(loss_sum) : nullptr);

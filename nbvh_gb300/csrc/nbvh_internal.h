@@ -584,6 +584,11 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
 // variants it launches; a stream capture cannot, so the serving loop calls this before capturing.
 cudaError_t configure_query_kernels();
 
+// order[0..n) = the rows of points by the cell of the unit cube that their middle point lies in; scratch as for
+// launch_ray_order.
+cudaError_t launch_row_order(const float *positions, uint32_t n, uint32_t n_points, uint16_t *keys, uint32_t *bins,
+                             uint32_t *order, int num_sms, cudaStream_t s);
+
 // order[0..n) = the ray ids bin by bin (coherence bins over the scene box, kRayBins of them);
 // keys: n, bins: kRayBinWords device words of scratch (16-byte aligned). Two kernels and a memset on the
 // stream.

@@ -14,8 +14,9 @@ from helpers import check_gradients
 pytestmark = pytest.mark.gpu
 
 
-def _handle(points, hidden, precision):
-    cfg = nb.default_config(**{"hashgrid.n_levels": 8, "hashgrid.n_features_per_level": 2, "hashgrid.base_resolution": 4,
+def _handle(points, hidden, precision, levels=8, features=2):
+    cfg = nb.default_config(**{"hashgrid.n_levels": levels, "hashgrid.n_features_per_level": features,
+                               "hashgrid.base_resolution": 4,
                                "hashgrid.per_level_scale": 1.5, "hashgrid.log2_hashmap_size": 12,
                                "module.input_segment_points": points, "network.precision": precision,
                                "network.n_hidden_layers": hidden})
@@ -43,6 +44,24 @@ def test_batch_equals_its_halves(built, points, hidden):
     with h:
         m = 19391  # 151 tiles and a ragged one; twice that: two tiles for every block
         pos, tgt = (torch.from_numpy(x).cuda() for x in _batch(2 * m, points, points * 10 + hidden))
+        g, loss = h.compute_gradients(pos, tgt)
+        parts = [h.compute_gradients(pos[a:a + m].contiguous(), tgt[a:a + m].contiguous()) for a in (0, m)]
+        want = (parts[0][0].double() + parts[1][0].double()) / 2
+        assert torch.isfinite(g).all() and (want != 0).any()
+        assert (g.double() - want).abs().max() <= 1e-4 * want.abs().max()
+        assert abs(loss - (parts[0][1] + parts[1][1]) / 2) <= 1e-4 * abs(loss)
+
+
+@pytest.mark.parametrize("points,levels,features", [(4, 16, 2), (3, 8, 4), (1, 2, 8)])
+def test_ordered_batch_equals_its_halves(built, points, levels, features):
+    """From 196,608 rows on a batch is encoded in the order of its rows' places, its halves in batch order."""
+    h, _ = _handle(points, 2, 1, levels, features)
+    with h:
+        m = 98305
+        pos, tgt = _batch(2 * m, points, points)
+        pos[: m // 4] = np.round(pos[: m // 4])  # the cube's border
+        pos[m:m + 50] = 0.25  # more rows in one place than a warp has lanes
+        pos, tgt = torch.from_numpy(pos).cuda(), torch.from_numpy(tgt).cuda()
         g, loss = h.compute_gradients(pos, tgt)
         parts = [h.compute_gradients(pos[a:a + m].contiguous(), tgt[a:a + m].contiguous()) for a in (0, m)]
         want = (parts[0][0].double() + parts[1][0].double()) / 2
