@@ -54,17 +54,25 @@ constexpr uint32_t kEncodeBlocksPerSm = 4;
 // size of the batch and of the cut; which kernel evaluates a segment does not show in its record,
 // since mma.sync and tcgen05 give the same bits on the same FP16 or BF16 rows (a test holds both to
 // that). Each wavefront step costs a batch of n rays about 30 us + what its kernels take; the tail
-// kernel costs no fixed time but about four times as much per segment. Measured on GB300 with the
-// tail from step 0 / 1 / 2 / 3 / 4 / 5 on, us per call (1,024-leaf cut, uniform rays; secondary and
-// camera rays cross at the same sizes within a factor of two):
-//   n =     2,048   110 / 148 / 187 / 210 / 248 / 280     n =   131,072   400 / 383 / 366 / 373 / 388 / 425
-//   n =    16,384   184 / 190 / 203 / 236 / 269 / 299     n =   524,288  1062 / 891 / 771 / 739 / 743 / 760
-//   n =    32,768   238 / 229 / 226 / 252 / 279 / 310     n = 1,048,576  1827 / 1389 / 1145 / 1081 / 1056 / 1072
+// kernel costs no fixed time but three to four times as much per segment. Measured on GB300 with the
+// tail from step 0 / 1 / 2 / 3 / 4 / 5 on, us per call (1,024-leaf cut, uniform rays; "s": rays that start
+// on the surface, which meet more leaves):
+//   n =     2,048    90 / 145 / 183 / 208 / 244 / 280     n = s  49,152   293 / 253 / 254 / 272 / 307 / 335
+//   n =    16,384   157 / 180 / 204 / 233 / 263 / 298     n =    65,536   296 / 268 / 276 / 300 / 332 / 372
+//   n =    24,576   187 / 196 / 210 / 239 / 270 / 302     n = s  65,536   373 / 300 / 288 / 306 / 343 / 385
+//   n = s  24,576   197 / 184 / 214 / 232 / 272 / 296     n =   131,072   358 / 353 / 341 / 353 / 374 / 413
+//   n =    32,768   213 / 211 / 219 / 246 / 277 / 313     n =   524,288   939 / 781 / 689 / 652 / 663 / 680
+//   n =    49,152   249 / 244 / 245 / 270 / 303 / 334     n = 1,048,576  1619 / 1233 / 1024 / 974 / 946 / 961
 // Larger learned cuts (long runs of small leaves, lists that stay short for 20-30 steps) gain from
 // step 3 on whatever the batch.
 __host__ __device__ constexpr uint32_t tail_step(uint32_t n_cut_nodes, uint32_t n)
 {
-    const uint32_t step = n <= kTailOnlyRays ? 0u : n <= (1u << 17) ? 2u : n <= (1u << 19) ? 3u : n <= (1u << 20) ? 4u : 5u;
+    const uint32_t step = n <= kTailOnlyRays  ? 0u
+                          : n <= (3u << 14)   ? 1u
+                          : n <= (1u << 17)   ? 2u
+                          : n <= (1u << 19)   ? 3u
+                          : n <= (1u << 20)   ? 4u
+                                              : 5u;
     return n_cut_nodes > kMaxSortNodes && step > 3u ? 3u : step;
 }
 constexpr uint32_t kTailWarps = 8;
