@@ -4,19 +4,23 @@
 // 54-137) runs, per traversal step, an encode kernel, tcnn inference, a process kernel and a
 // compaction kernel, then copies the active count to the host and synchronises. Here:
 //
-//   k_wave_first   one thread per ray: the first entered leaf (K2). Rays that enter none are
-//                  answered at once; the others are appended (warp-aggregated) to state list 0.
-//   then per step, over the rays listed by the previous step:
-//   k_wave_encode  K3: segment points and hash-grid features, one thread per (ray, point, level),
+//   k_query_begin  counters cleared, weights packed;
+//   k_ray_bins, k_ray_bin_place (2^19 rays or more): a coherence order of the rays;
+//   k_wave_first   the first entered leaf of every ray (K2). Rays that enter none are answered
+//                  at once; the others are appended (warp-aggregated) to state list 0.
+//   then per step up to the tail's (tail_step), over the rays listed by the previous step:
+//   k_wave_sort    (lists of 2^16 rays or more) the listed rays in leaf order;
+//   k_wave_encode  K3: segment points and hash-grid features, one thread per (ray, point),
 //                  FP16 rows written in the layout the tensor-core MLP loads by TMA;
 //   k_mlp_tc       K4: the fused MLP on tcgen05 tensor cores (k_mlp_tc.cu), 128-row tiles;
 //   k_wave_decode  K2: LocalT decode and closest-hit update, then the next entered leaf for the
-//                  rays that continue, appended to the other list.
+//                  rays that continue, appended to the other list;
+//   k_wave_tail    the rays left, in one launch.
 //
-// Splitting the step lets each phase run at the occupancy it needs: the gathers of K3 with 48
+// Splitting the step lets each phase run at the occupancy it needs: the gathers of K3 with 32
 // warps per SM, the MLP with its accumulators in tensor memory, the divergent traversal with the
-// cut read through L1 (or staged in shared memory: StepResources::stage_cut). Every kernel reads the list length from device memory, so the host
-// checks it only once per batch of steps (one 16-byte copy).
+// cut read through L1 (or staged in shared memory: StepResources::stage_cut). Every kernel reads the
+// list length from device memory; the host reads it once, after the tail kernel (one 16-byte copy).
 #include <type_traits>
 
 #include "device_math.cuh"
@@ -595,11 +599,10 @@ __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_co
 // The L1 bounds it: it looks up one cache line per cycle, and a (point, level) of the table costs 6
 // lookups (4 pairs of x corners, half of them split). Levels in the cell copy cost one 32-byte read:
 // 1,453 -> 1,250 us per 2^22-ray query with the copy of the 8 coarsest levels (192 MB; dense levels
-// alone, 11 MB: 1,390; 9 levels, 520 MB: no more), 489 -> 455 for 2^20 rays with 4 of the reference's 8
+// alone, 11 MB: 1,390; 9 levels, 520 MB: no more), 489 -> 455 for 2^20 rays with 5 of the reference's 8
 // levels. Reading the quad of entries where both corners lie in it was slower (1,435 us: the warp then
 // issues three kinds of load). The tail kernel reads the table alone: its lanes hold different levels,
 // and both paths in it cost more registers than the copy saved.
-
 template <uint32_t F>
 __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
     k_wave_encode(const __grid_constant__ WaveArgs a, uint32_t it)
@@ -1702,9 +1705,9 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     const bool keyed = res.sort_key != nullptr && res.n_sort_bins > 0u;
     const uint32_t n_bins = keyed ? res.n_sort_bins : n_cut_nodes;
     a.sort_key = keyed ? res.sort_key : nullptr;
-    // octant sub-bins where the caller sized the count buffers for them, the sort's
-    // shared memory (of the form that kept three words per bin) fits, and each row has enough point-levels to gather
-    // for the encoder's better locality to outweigh the sort's extra reads (measured on GB300: 4
+    // octant sub-bins where the caller sized the count buffers for them, the sort's shared memory (of the
+    // form that kept three words per bin) fits, and each row has enough point-levels to gather for the
+    // encoder's better locality to outweigh the sort's extra reads (measured on GB300: 4
     // points x 16 levels 3.35 -> 3.31 ms per 2^22-ray query; 3 points x 8 levels 2.32 -> 2.37 ms)
     a.sub_bins = (res.sub_bins && (size_t)3u * 4u * kSubBins * n_bins <= (size_t)kMaxDynamicSmem &&
                   grid.n_points * grid.n_levels >= kSubBinMinPointLevels)
