@@ -3,8 +3,8 @@
 // tcnn's FullyFusedMLP (configured at src/cuda/neural/neural_bvh_module.cu:232-238: 64 neurons,
 // ReLU hidden layers, Sigmoid output, no biases, output padded to 16) evaluated on 128-row tiles:
 //
-//   TMA        one 2-D tensor copy per 8-column slice moves the tile's FP16 inputs from HBM into
-//              shared memory, already in the tensor core's K-major core-matrix layout;
+//   TMA        one 2-D tensor copy per column block (64, 32 or 16 values) moves the tile's 16-bit inputs
+//              from HBM into shared memory, already in a swizzled K-major layout of the tensor core;
 //   tcgen05    one thread issues each layer as M=128 x N=64 (N=16 for the output layer) MMAs over
 //              K in steps of 16; the FP32 accumulator lives in tensor memory (columns 0-63);
 //   epilogue   each of the 4 warps reads its 32 TMEM lanes (= its 32 rows), applies ReLU, rounds to
@@ -49,9 +49,14 @@ __host__ __device__ constexpr uint32_t tmem_alloc_cols(uint32_t groups)
 // The input tiles follow the weights on a 1,024-byte boundary (the swizzle atoms of the tiles).
 __host__ __device__ constexpr uint32_t tile_offset(uint32_t wbytes) { return (wbytes + 1023u) & ~1023u; }
 
-// Feature rows of a multiple of 64 values are copied in 128-byte swizzled boxes (one TMA request
-// per 128-byte row segment); other widths in 16-byte boxes (eight times the requests).
-__host__ __device__ constexpr bool feature_map_swizzled(uint32_t n_inputs) { return n_inputs % 64u == 0u; }
+// Feature rows are copied in swizzled boxes, one TMA request per row of a box: 128 bytes (64 values) where the
+// width is a multiple of that, else 64 or 32 bytes. (Widths that are no multiple of 64 came in unswizzled boxes
+// of 16 bytes before, two to eight times the requests, which the TMA unit takes one by one: 2^21 rows of 96
+// inputs 162 -> 135 us per call, of 112 171 -> 145, of 48 139 -> 130, of 16 131 -> 122.)
+__host__ __device__ constexpr uint32_t feature_box_bytes(uint32_t n_inputs)
+{
+    return n_inputs % 64u == 0u ? 128u : (n_inputs % 32u == 0u ? 64u : 32u);
+}
 
 __host__ __device__ inline uint32_t w0_bytes(uint32_t n_inputs) { return kNeurons * n_inputs * 2u; }
 __host__ __device__ inline uint32_t hidden_w_bytes() { return kNeurons * kNeurons * 2u; }
@@ -85,27 +90,15 @@ struct MlpTcArgs {
     uint32_t stall;   // failure-path test: wait on an mbarrier nothing arrives at (it runs out)
 };
 
-// D = A * W^T for the 128-row tile: A (128 x K) at a_addr, W (N x K) at w_addr, both in the
-// operand layout; one MMA per 16 values of K.
-__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_addr, uint32_t w_addr, uint32_t k_dim,
-                                            uint32_t n_dim, uint32_t idesc)
+// Layer 0 from an input tile in the swizzled layout: A (128 x K) as column blocks of 128 rows x row_bytes, W
+// (N x K) in the unswizzled operand layout.
+__device__ __forceinline__ void issue_layer_swizzled(uint32_t tmem, uint32_t a_addr, uint32_t row_bytes, uint32_t w_addr,
+                                                     uint32_t k_dim, uint32_t n_dim, uint32_t idesc)
 {
-    const uint32_t a_lbo = kTileRows * 16u, b_lbo = n_dim * 16u;
+    const uint32_t b_lbo = n_dim * 16u, shift = row_bytes == 128u ? 2u : (row_bytes == 64u ? 1u : 0u);
     for (uint32_t k = 0; k < k_dim / 16u; k++) {
-        const uint64_t ad = tc::smem_desc(a_addr + 2u * k * a_lbo, a_lbo, 128u);
-        const uint64_t bd = tc::smem_desc(w_addr + 2u * k * b_lbo, b_lbo, 128u);
-        tc::mma_f16(tmem, ad, bd, idesc, k > 0u ? 1u : 0u);
-    }
-}
-
-// Layer 0 from an input tile in the 128-byte swizzled layout (inputs a multiple of 64): A (128 x K)
-// as K / 64 column blocks of 16 KB, W (N x K) in the unswizzled operand layout.
-__device__ __forceinline__ void issue_layer_sw128(uint32_t tmem, uint32_t a_addr, uint32_t w_addr, uint32_t k_dim,
-                                                  uint32_t n_dim, uint32_t idesc)
-{
-    const uint32_t b_lbo = n_dim * 16u;
-    for (uint32_t k = 0; k < k_dim / 16u; k++) {
-        const uint64_t ad = tc::smem_desc_sw128(a_addr + (k >> 2) * (kTileRows * 128u) + (k & 3u) * 32u);
+        const uint32_t block = k >> shift, step = k - (block << shift);
+        const uint64_t ad = tc::smem_desc_swizzled(a_addr + block * (kTileRows * row_bytes) + step * 32u, row_bytes);
         const uint64_t bd = tc::smem_desc(w_addr + 2u * k * b_lbo, b_lbo, 128u);
         tc::mma_f16(tmem, ad, bd, idesc, k > 0u ? 1u : 0u);
     }
@@ -193,7 +186,7 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
     if (blockIdx.x >= n_tiles)
         return; // no tile for this CTA: skip TMEM and the weight copy
     const uint32_t tile_bytes = kTileRows * K * 2u;
-    const bool sw128 = feature_map_swizzled(K);
+    const uint32_t box = feature_box_bytes(K);
     if ((tc::smem_addr(smem) & 1023u) != 0u) { // the swizzled tiles need 1,024-byte aligned atoms
         if (threadIdx.x == 0)
             atomicOr(a.status, 2u);
@@ -234,15 +227,9 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
 
     auto load_tile = [&](uint32_t t) {
         tc::mbar_expect_tx(bar_load, tile_bytes);
-        if (sw128) { // boxes of 64 values (128-byte rows), swizzled
-            for (uint32_t c = 0; c < K / 64u; c++)
-                tc::tma_load_2d(t_addr + c * kTileRows * 128u, &fmap, (int32_t)(64u * c), (int32_t)(t * kTileRows),
-                                bar_load);
-        } else { // boxes of 8 values (16-byte rows)
-            for (uint32_t c = 0; c < K / 8u; c++)
-                tc::tma_load_2d(t_addr + c * kTileRows * 16u, &fmap, (int32_t)(8u * c), (int32_t)(t * kTileRows),
-                                bar_load);
-        }
+        for (uint32_t c = 0; c * box < 2u * K; c++)
+            tc::tma_load_2d(t_addr + c * kTileRows * box, &fmap, (int32_t)(c * (box / 2u)), (int32_t)(t * kTileRows),
+                            bar_load);
     };
     uint32_t ph_load = 0, ph_mma = 0;
     bool load_pending = false, mma_pending = false;
@@ -274,10 +261,8 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
         for (uint32_t layer = 0; layer <= H; layer++) {
             if (mma_warp && tc::elect_one()) {
                 tc::fence_after_sync();
-                if (layer == 0 && sw128)
-                    issue_layer_sw128(tmem, t_addr, w_addr, K, kNeurons, id_hidden);
-                else if (layer == 0)
-                    issue_layer(tmem, t_addr, w_addr, K, kNeurons, id_hidden);
+                if (layer == 0)
+                    issue_layer_swizzled(tmem, t_addr, box, w_addr, K, kNeurons, id_hidden);
                 else if (layer < H)
                     issue_layer_ta(tmem, kActCol, w_addr + w0_bytes(K) + (layer - 1u) * hidden_w_bytes(), kNeurons,
                                    kNeurons, id_hidden);
@@ -374,8 +359,7 @@ cudaError_t launch_pack_weights(const __half *params_h, uint32_t n_inputs, uint3
     return cudaGetLastError();
 }
 
-cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t rows, TensorMapBytes *out,
-                             bool allow_swizzle)
+cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t rows, TensorMapBytes *out)
 {
     static_assert(sizeof(CUtensorMap) == sizeof(TensorMapBytes), "tensor map size");
     if ((reinterpret_cast<uintptr_t>(features) & 15u) != 0u || n_inputs % 16u != 0u || n_inputs > 128u || rows == 0u)
@@ -386,14 +370,16 @@ cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t
     CUtensorMap fmap;
     const cuuint64_t dims[2] = {n_inputs, rows};
     const cuuint64_t strides[1] = {(cuuint64_t)n_inputs * 2u};
-    // 64 values x 128 rows, 128-byte swizzle (one atom column of the K-major swizzled layout), or
-    // 8 values x 128 rows unswizzled (one K column of core matrices)
-    const bool sw = allow_swizzle && feature_map_swizzled(n_inputs);
-    const cuuint32_t box[2] = {sw ? 64u : 8u, kTileRows};
+    // row_bytes x 128 rows with the swizzle of that width (one atom column of the K-major swizzled layout)
+    const uint32_t row_bytes = feature_box_bytes(n_inputs);
+    const CUtensorMapSwizzle swizzle = row_bytes == 128u  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                       : row_bytes == 64u ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                          : CU_TENSOR_MAP_SWIZZLE_32B;
+    const cuuint32_t box[2] = {row_bytes / 2u, kTileRows};
     const cuuint32_t estr[2] = {1u, 1u};
     // 16-bit rows; the element type of the map only sizes the copy (FP16 and BF16 move the same bits)
     if (encode(&fmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(features), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, sw ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     memcpy(out->bytes, &fmap, sizeof(fmap));

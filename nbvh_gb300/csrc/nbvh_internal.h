@@ -627,10 +627,7 @@ uint32_t packed_weight_bytes(uint32_t n_inputs, uint32_t n_hidden_layers);
 // (clear0, clear1: words the launch zeroes as well, NULL for none)
 cudaError_t launch_pack_weights(const __half *params_h, uint32_t n_inputs, uint32_t n_hidden_layers, __half *packed,
                                 cudaStream_t s, uint32_t *clear0 = nullptr, uint32_t *clear1 = nullptr);
-// allow_swizzle = false: always 8-value boxes, so that a 128-row tile lands in shared memory in
-// the unswizzled K-major core-matrix layout (column block c of 8 values at c * 2,048 bytes).
-cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t rows, TensorMapBytes *out,
-                             bool allow_swizzle = true);
+cudaError_t make_feature_map(const __half *features, uint32_t n_inputs, uint32_t rows, TensorMapBytes *out);
 // wait_ns: time limit of the kernel's phase waits (0: the default of one second). stall (failure-path
 // tests): one wait on an mbarrier that nothing arrives at, which runs out after wait_ns.
 // MaxDynamicSharedMemorySize of the tensor-core MLP's variants (FP16, BF16, FP8) on the current device.

@@ -2,14 +2,14 @@
 // tensor memory (TMEM), TMA bulk / tensor copies into shared memory, and mbarrier waits that give up
 // after a time limit instead of spinning forever.
 //
-// Shared-memory operand layout used throughout (K-major, no swizzle): the matrix is cut into "core
+// Shared-memory operand layout (K-major, no swizzle; the MLP's input tiles are swizzled, see
+// smem_desc_swizzled): the matrix is cut into "core
 // matrices" of 8 rows x 16 bytes (8 FP16 values), each stored as 128 contiguous bytes (row i of the
 // core matrix at byte 16 * i). A descriptor gives two strides: LBO, the byte distance between core
 // matrices adjacent along K, and SBO, the distance between core matrices adjacent along M (or N).
 // Here every operand uses SBO = 128 (the 8-row groups of one K column of core matrices are
 // contiguous) and LBO = rows * 16, so element (r, k) of an R-row operand lives at
 //     (k / 8) * (R * 16) + r * 16 + (k % 8) * 2.
-// This is also exactly what a 2-D TMA box of 8 values x R rows writes, so tiles arrive ready to use.
 #pragma once
 
 #include <cstdint>
@@ -288,15 +288,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// Shared-memory matrix descriptor of a K-major operand in the 128-byte swizzled layout: atoms of
-// 8 rows x 128 bytes (64 16-bit values of K), rows 128 bytes apart with their 16-byte chunks XORed
-// by the row index (what a TMA box of 64 values x R rows with SWIZZLE_128B writes), atoms along
-// M/N 1,024 bytes apart. addr = atom-aligned base (1,024-byte aligned) + 32 bytes per 16 values of
-// K inside the atom.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
+// Shared-memory matrix descriptor of a K-major operand in a swizzled layout with rows of row_bytes = 128, 64
+// or 32: atoms of 8 rows, rows row_bytes apart with their 16-byte chunks XORed by address bits 7 and up
+// (what a TMA box of row_bytes x R rows with that swizzle writes), atoms along M/N next to each
+// other. addr = atom-aligned base + 32 bytes per 16 values of K inside the atom.
+__device__ __forceinline__ uint64_t smem_desc_swizzled(uint32_t addr, uint32_t row_bytes)
 {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
+    const uint64_t layout = row_bytes == 128u ? 2u : (row_bytes == 64u ? 4u : 6u);
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(row_bytes >> 1) << 32) | (1ull << 46) |
+           (layout << 61);
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator, A and B both FP16 (or both BF16),
