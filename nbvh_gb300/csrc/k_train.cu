@@ -450,10 +450,10 @@ cudaError_t encode_rows(const GridParams &grid, const uint32_t *table, const flo
 //             and dW_j^T += X_j^T dZ_{j+1} over the tile's 128 rows (both operands read
 //             transposed from the same shared-memory tiles), then dZ_j = dX_j * (X_j > 0);
 //             dX_0, rounded to the MLP precision, goes to global memory for the grid scatter.
-// The weight gradients stay in tensor memory, accumulated over all the CTA's tiles, and are
-// written out once per CTA at the end; the scatter kernel's last blocks sum them. Every [128 rows][C columns] tile lives in
-// shared memory in the K-major core-matrix layout (8-column block c at c * 2,048 bytes, row r at
-// r * 16 within it): with M = rows it is a K-major operand (LBO 2,048, SBO 128), with K = rows an
+// The weight gradients stay in tensor memory, accumulated over all the CTA's tiles, and are written out
+// once per CTA at the end; the scatter kernel's first blocks sum them. Every [128 rows][C columns] tile
+// lives in shared memory in the K-major core-matrix layout (8-column block c at c * 2,048 bytes, row r
+// at r * 16 within it): with M = rows it is a K-major operand (LBO 2,048, SBO 128), with K = rows an
 // MN-major one (LBO 128, SBO 2,048). The input tile is copied into that layout 16 bytes at a time.
 // ---------------------------------------------------------------------------------------------
 
