@@ -9,7 +9,7 @@
 //   k_wave_first   the first entered leaf of every ray (K2). Rays that enter none are answered
 //                  at once; the others are appended (warp-aggregated) to state list 0.
 //   then per step up to the tail's (tail_step), over the rays listed by the previous step:
-//   k_wave_sort    (lists of 2^16 rays or more) the listed rays in leaf order;
+//   k_wave_sort    (batches of 2^19 rays or more) the listed rays in leaf order;
 //   k_wave_encode  K3: segment points and hash-grid features, one thread per (ray, point),
 //                  FP16 rows written in the layout the tensor-core MLP loads by TMA;
 //   k_mlp_tc       K4: the fused MLP on tcgen05 tensor cores (k_mlp_tc.cu), 128-row tiles;
@@ -37,8 +37,14 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr uint32_t kEncodeThreads = 256;
 constexpr uint32_t kFirstThreads = 256;
 constexpr uint32_t kSortThreads = 1024;
-// Lists shorter than this are walked in list order: the sort would cost more than the locality it buys.
-constexpr uint32_t kSortMinRows = 1u << 16;
+// Lists shorter than kSortMinRows are walked in list order: the sort would cost more than the locality it buys.
+// Batches below kSortMinRays have no list sorted: besides the sorts' launches, which every step has whatever its
+// list, the first pass and the decode then count no rows per bin. us per call with lists sorted from 2^16 rows on /
+// not at all: 131,072 uniform rays 333 / 317, 262,144 459 / 432, a 512 x 512 frame 580 / 545, a 960 x 540 path
+// 1,864 / 1,785, 524,288 uniform rays 654 / 650. Larger batches gain from it: 2^20 rays 947 sorted, 963 with lists
+// below 2^19 left as they are; of 2^16, 2^17 and 2^18 none is better for them (2^22 rays 2,622, 2,613, 2,616).
+constexpr uint32_t kSortMinRays = 1u << 19;
+constexpr uint32_t kSortMinRows = 1u << 17;
 // Rows with at least this many (point, level) pairs to encode are sorted by octant within a leaf.
 constexpr uint32_t kSubBinMinPointLevels = 32;
 // node visits of a traversal between lane refills (measured on GB300, 2^22 uniform rays: 4 -> 3.29,
@@ -738,7 +744,7 @@ __global__ void __launch_bounds__(kEncodeThreads, kEncodeBlocksPerSm)
 // 18 with eight reservations in flight and the padded scan (123 to 81 for the sorts of 2^22 rays). A chunk
 // with at most half as many rows as there are bins has about one row per bin and
 // takes its places straight from the bins' cursors, one atomic for the lanes of a warp that share a bin:
-// 16 us, and 574 instead of 589 per 512 x 512 frame. With few bins many blocks would meet on
+// 16 us for lists of that size. With few bins many blocks would meet on
 // each cursor: 54 us instead of 34 for the lists of 2^20 visibility rays in 2,047 bins.
 __global__ void __launch_bounds__(kSortThreads) k_wave_sort(const __grid_constant__ WaveArgs a, uint32_t it)
 {
@@ -1716,8 +1722,7 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     a.n_sort_nodes = a.sub_bins ? kSubBins * n_bins : n_bins;
     a.bf16 = prec == NBVH_PRECISION_BF16 ? 1u : 0u;
     a.prec = prec;
-    // (no list of a batch below kSortMinRows rays is long enough to be sorted)
-    const bool sort = res.perm != nullptr && n_bins <= kMaxSortNodes && n >= kSortMinRows;
+    const bool sort = res.perm != nullptr && n_bins <= kMaxSortNodes && n >= kSortMinRays;
     // a stalled wait (failure-path test) needs the tensor-core kernels to run
     a.tail_at = tail_step(n_cut_nodes, res.stall ? 0xFFFFFFFFu : n);
     a.perm = sort ? res.perm : nullptr;

@@ -35,3 +35,22 @@ def test_sorted_lists_against_unsorted(built, points, levels, features, depth):
         for a in range(0, n, 65535):
             part = h.query_closest_neural(rays[a:a + 65535].contiguous())
             assert torch.equal(part, whole[a:a + 65535]), a
+
+
+@pytest.mark.parametrize("depth", [4, 10])
+def test_sorted_batch_with_octant_bins(built, depth):
+    """600,001 rays: a list of some 4,000 rows per block, fewer than half the bins of the deep cut (places
+    straight from the cursors) and more than those of the shallow one (ranges per block)."""
+    cfg = nb.default_config(**{"hashgrid.base_resolution": 8, "hashgrid.log2_hashmap_size": 12})
+    h, s = handle(cfg, kind="soup64k", seed=4, depth=depth)
+    with h:
+        rng = np.random.default_rng(3)
+        p = h.params()
+        nn = h.layout.n_network_params
+        p[nn:] = rng.uniform(-0.5, 0.5, p.size - nn).astype(np.float32)
+        h.set_params(p)
+        n = 600001
+        rays = torch.from_numpy(scenes.uniform_rays(n, s["bbox"][:3], s["bbox"][3:], seed=6, scaling=1.0)).cuda()
+        whole = h.query_closest_neural(rays)
+        for a in range(0, n, 65535):
+            assert torch.equal(h.query_closest_neural(rays[a:a + 65535].contiguous()), whole[a:a + 65535]), a
