@@ -67,12 +67,14 @@ constexpr uint32_t kEncodeBlocksPerSm = 4;
 // kernel costs no fixed time but three to four times as much per segment. Measured on GB300 with the
 // tail from step 0 / 1 / 2 / 3 / 4 / 5 on, us per call (1,024-leaf cut, uniform rays; "s": rays that start
 // on the surface, which meet more leaves):
-//   n =     2,048    90 / 145 / 183 / 208 / 244 / 280     n = s  49,152   293 / 253 / 254 / 272 / 307 / 335
-//   n =    16,384   157 / 180 / 204 / 233 / 263 / 298     n =    65,536   296 / 268 / 276 / 300 / 332 / 372
-//   n =    24,576   187 / 196 / 210 / 239 / 270 / 302     n = s  65,536   373 / 300 / 288 / 306 / 343 / 385
-//   n = s  24,576   197 / 184 / 214 / 232 / 272 / 296     n =   131,072   358 / 353 / 341 / 353 / 374 / 413
-//   n =    32,768   213 / 211 / 219 / 246 / 277 / 313     n =   524,288   939 / 781 / 689 / 652 / 663 / 680
-//   n =    49,152   249 / 244 / 245 / 270 / 303 / 334     n = 1,048,576  1619 / 1233 / 1024 / 974 / 946 / 961
+//   n =     2,048    90 / 145 / 183 / 208 / 244 / 280     n = s  65,536   373 / 291 / 267 / 284 / 315 / 350
+//   n =    16,384   157 / 180 / 204 / 233 / 263 / 298     n =   131,072   358 / 339 / 320 / 327 / 347 / 381
+//   n =    24,576   187 / 196 / 210 / 239 / 270 / 302     n = s 131,072     - / 452 / 377 / 392 / 414 / 451
+//   n = s  24,576   197 / 184 / 214 / 232 / 272 / 296     n =   262,144     - / 464 / 439 / 428 / 445 / 466
+//   n =    32,768   213 / 216 / 217 / 246 / 281 / 311     n = s 262,144     - / 747 / 619 / 579 / 599 / 630
+//   n =    49,152   249 / 243 / 240 / 261 / 290 / 331     n =   524,288   939 / 771 / 676 / 651 / 655 / 678
+//   n = s  49,152   293 / 248 / 250 / 270 / 299 / 334     n = 1,048,576  1619 / 1233 / 1024 / 974 / 946 / 961
+//   n =    65,536   296 / 254 / 254 / 269 / 304 / 343
 // Larger learned cuts (long runs of small leaves, lists that stay short for 20-30 steps) gain from
 // step 3 on whatever the batch.
 __host__ __device__ constexpr uint32_t tail_step(uint32_t n_cut_nodes, uint32_t n)
