@@ -1037,7 +1037,7 @@ nbvh_status nbvh_query_closest_classic(nbvh_handle *h, const nbvh_ray *d_rays, u
         cuda_check(launch_classic(h->d_nodes.ptr, h->d_tris.ptr, d_rays, n, d_hits, false, order, h->classic_fast_div, s),
                    "classic");
         cuda_check(cudaEventRecord(h->ev1, s), "event");
-        h->last_launches = order ? 4u : 1u;
+        h->last_launches = order ? 3u : 1u;
         h->last_rays = n;
     });
 }
