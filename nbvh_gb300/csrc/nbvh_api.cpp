@@ -1532,8 +1532,10 @@ nbvh_status nbvh_adam_step(nbvh_handle *h, const float *d_gradients, nbvh_stream
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         cuda_check(cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &capture), "capture status");
         params_changed(h);
-        if (capture != cudaStreamCaptureStatusNone)
+        if (capture != cudaStreamCaptureStatusNone && !h->cells_off) {
             h->cells_off = true; // replays will change the parameters unseen
+            h->model_version++;  // captured query graphs may hold the cell copy: they are made anew
+        }
         cuda_check(launch_adam(h->d_params.ptr, h->d_params_h.ptr, h->d_adam_m.ptr, h->d_adam_v.ptr, d_gradients,
                                h->layout.n_params, adam_step_size(c, h->training_step), c.optimizer.beta1,
                                c.optimizer.beta2, c.optimizer.epsilon, c.optimizer.l2_reg, 1.0f, param_precision(h),

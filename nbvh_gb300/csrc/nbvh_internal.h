@@ -383,7 +383,7 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<float> d_train_loss;  // per row loss (sum over output channels)
     nbvh::DeviceBuffer<float> d_loss_sum;
     nbvh::TreeCutSession cut;
-    uint64_t model_version = 0; // bumped whenever a device array that queries read is reallocated
+    uint64_t model_version = 0; // bumped whenever a device array that queries read is reallocated or given up
 
     // path-tracing workspace
     nbvh::PathBuffers path;
