@@ -427,7 +427,9 @@ __device__ __forceinline__ uint32_t fp8_act_relu_half2(float lo, float hi)
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// Two FP32 values -> ReLU -> 16-bit pair (lo in the low half), one cvt.rn.relu instruction.
+// Two FP32 values -> ReLU -> 16-bit pair (lo in the low half), one cvt.rn.relu instruction. NaN stays
+// NaN (fmaxf would make it 0): every path of the network has to treat the sums of overflowed
+// activations alike, since the size of a batch decides which one evaluates a segment.
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack_relu(float lo, float hi)
 {
@@ -446,7 +448,6 @@ __device__ __forceinline__ uint32_t pack_relu(float lo, float hi)
 template <bool BF16, bool FP8 = false>
 __device__ __forceinline__ void relu_pack(const float (&acc)[8][4], uint32_t (&a)[4][4], bool quant = false)
 {
-    using Pr = MlpPrec<BF16>;
     static_assert(!(FP8 && BF16), "FP8 hidden layers run on the FP16 tensor-core path");
     if (FP8 && quant) {
 #pragma unroll
@@ -458,13 +459,12 @@ __device__ __forceinline__ void relu_pack(const float (&acc)[8][4], uint32_t (&a
         }
         return;
     }
-    auto act = [](float x) { return fmaxf(x, 0.f); };
 #pragma unroll
     for (int kb = 0; kb < 4; kb++) {
-        a[kb][0] = Pr::pack(act(acc[2 * kb][0]), act(acc[2 * kb][1]));
-        a[kb][1] = Pr::pack(act(acc[2 * kb][2]), act(acc[2 * kb][3]));
-        a[kb][2] = Pr::pack(act(acc[2 * kb + 1][0]), act(acc[2 * kb + 1][1]));
-        a[kb][3] = Pr::pack(act(acc[2 * kb + 1][2]), act(acc[2 * kb + 1][3]));
+        a[kb][0] = pack_relu<BF16>(acc[2 * kb][0], acc[2 * kb][1]);
+        a[kb][1] = pack_relu<BF16>(acc[2 * kb][2], acc[2 * kb][3]);
+        a[kb][2] = pack_relu<BF16>(acc[2 * kb + 1][0], acc[2 * kb + 1][1]);
+        a[kb][3] = pack_relu<BF16>(acc[2 * kb + 1][2], acc[2 * kb + 1][3]);
     }
 }
 
