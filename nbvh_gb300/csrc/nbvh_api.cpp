@@ -423,14 +423,26 @@ ParamPrecision param_precision(const nbvh_handle *h)
 
 void params_changed(nbvh_handle *h)
 {
+    std::lock_guard<std::mutex> lock(h->cells_mu);
     h->cells_fresh = false;
     h->cells_rays = 0;
 }
 
+// Around every write of the parameters. A scene or serving query does not hold the handle's lock and may
+// build the cell copy while they are written, from values before, between or after: what is built up to
+// the write's end is dropped.
+struct ParamsWrite {
+    nbvh_handle *h;
+    explicit ParamsWrite(nbvh_handle *handle) : h(handle) { params_changed(h); }
+    ~ParamsWrite() { params_changed(h); }
+    ParamsWrite(const ParamsWrite &) = delete;
+    ParamsWrite &operator=(const ParamsWrite &) = delete;
+};
+
 void upload_params(nbvh_handle *h, const float *params, bool reset_adam)
 {
     const uint32_t n = h->layout.n_params;
-    params_changed(h);
+    const ParamsWrite write(h);
     cuda_check(h->d_params.resize(n), "alloc params");
     cuda_check(h->d_params_h.resize(n), "alloc fp16 params");
     cuda_check(cudaMemcpy(h->d_params.ptr, params, (size_t)n * sizeof(float), cudaMemcpyHostToDevice), "upload params");
@@ -1531,20 +1543,26 @@ nbvh_status nbvh_adam_step(nbvh_handle *h, const float *d_gradients, nbvh_stream
         const nbvh_config &c = h->cfg;
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         cuda_check(cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &capture), "capture status");
-        params_changed(h);
-        if (capture != cudaStreamCaptureStatusNone && !h->cells_off) {
-            h->cells_off = true; // replays will change the parameters unseen
-            h->model_version++;  // captured query graphs may hold the cell copy: they are made anew
+        const ParamsWrite write(h);
+        if (capture != cudaStreamCaptureStatusNone) {
+            std::lock_guard<std::mutex> lock(h->cells_mu);
+            if (!h->cells_off) {
+                h->cells_off = true; // replays will change the parameters unseen
+                h->model_version++;  // captured query graphs may hold the cell copy: they are made anew
+            }
         }
         cuda_check(launch_adam(h->d_params.ptr, h->d_params_h.ptr, h->d_adam_m.ptr, h->d_adam_v.ptr, d_gradients,
                                h->layout.n_params, adam_step_size(c, h->training_step), c.optimizer.beta1,
                                c.optimizer.beta2, c.optimizer.epsilon, c.optimizer.l2_reg, 1.0f, param_precision(h),
                                reinterpret_cast<cudaStream_t>(stream)),
                    "adam");
-        if (!h->cells_off) { // the cell copy is built after this step, whatever stream builds it
-            if (!h->ev_params)
-                cuda_check(cudaEventCreateWithFlags(&h->ev_params, cudaEventDisableTiming), "event");
-            cuda_check(cudaEventRecord(h->ev_params, reinterpret_cast<cudaStream_t>(stream)), "event");
+        {
+            std::lock_guard<std::mutex> lock(h->cells_mu);
+            if (!h->cells_off) { // the cell copy is built after this step, whatever stream builds it
+                if (!h->ev_params)
+                    cuda_check(cudaEventCreateWithFlags(&h->ev_params, cudaEventDisableTiming), "event");
+                cuda_check(cudaEventRecord(h->ev_params, reinterpret_cast<cudaStream_t>(stream)), "event");
+            }
         }
         h->training_step++;
         h->last_launches = 1;
@@ -1581,7 +1599,7 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
         cudaStream_t s = h->pipe_stream[0];
         cuda_check(cudaMemsetAsync(h->d_loss_sum.ptr, 0, ((size_t)steps + 1u) * sizeof(float), s), "zero loss");
         cuda_check(cudaMemsetAsync(h->d_status.ptr, 0, sizeof(uint32_t), s), "reset status");
-        params_changed(h);
+        const ParamsWrite write(h);
         const NeuralConsts nc = make_neural_consts(h, 1u, false);
         const uint32_t first = h->training_step;
         float lr_t = 0.f;

@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -362,11 +363,11 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<uint4> d_cells;
     nbvh::CellParams cell_levels{};
     size_t n_cells = 0;       // cells of the layout (0: none)
-    bool cells_fresh = false; // d_cells holds the current parameters' entries
+    std::atomic<bool> cells_fresh{false}; // d_cells holds the current parameters' entries
     uint64_t cells_rays = 0;  // rays queried without it since the parameters changed
     bool cells_off = false;   // never: no memory for it, or Adam steps captured into a graph
     cudaEvent_t ev_params = nullptr; // after the last nbvh_adam_step, on its stream
-    std::mutex cells_mu;      // serving slots may find them stale at the same time
+    std::mutex cells_mu;      // guards the six above (cells_fresh is also read without it)
     uint32_t *h_readback = nullptr; // two page-locked words a call reads its status and loss back into
     nbvh::DeviceBuffer<float> d_adam_m, d_adam_v;
     nbvh::DeviceBuffer<float> d_grad;
