@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(256) k_build_cells(const __grid_constant__ Gri
 size_t plan_cells(const GridParams &grid, CellParams &cp)
 {
     cp = CellParams{};
+    if (grid.n_features == 2u && (grid.n_levels & 3u) != 0u)
+        return 0; // their encoder stores level by level and reads the table alone
     size_t total = 0;
     uint32_t l = 0;
     for (; l < grid.n_levels; l++) {

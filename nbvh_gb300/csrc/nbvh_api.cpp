@@ -2206,7 +2206,9 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
 void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
 {
     std::lock_guard<std::mutex> lock(h->cells_mu);
-    if (h->cells_fresh || h->cells_off || h->n_cells == 0u || !uses_cells(n))
+    if (h->cells_off)
+        h->d_cells.release();
+    if (h->cells_fresh || h->cells_off || h->n_cells == 0u || h->cfg.bvh.ignore_neural_blas || !uses_cells(n))
         return;
     if (h->cells_rays + n < kCellsAfterRays) { // a program may train again before its next query
         h->cells_rays += n;
@@ -2217,9 +2219,9 @@ void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
         if (!may_allocate)
             return;
         h->model_version++; // captured graphs hold the address
-        if (h->d_cells.resize(words) != cudaSuccess) { // no room: the table alone serves the queries
+        if (h->d_cells.resize(words) != cudaSuccess) { // no room now: as many rays on the table alone
             cudaGetLastError();
-            h->cells_off = true;
+            h->cells_rays = 0;
             return;
         }
     }

@@ -359,13 +359,13 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<__half> d_wpacked;  // network matrices in the tensor-core operand layout
     nbvh::DeviceBuffer<__half> d_infer_feat; // feature rows of nbvh_network_inference
     nbvh::DeviceBuffer<uint32_t> d_status; // error word of kernels with bounded waits
-    // cell copy of the coarse hash-grid levels, built for the first query after the parameters changed
+    // cell copy of the coarse hash-grid levels (ensure_cells)
     nbvh::DeviceBuffer<uint4> d_cells;
     nbvh::CellParams cell_levels{};
     size_t n_cells = 0;       // cells of the layout (0: none)
     std::atomic<bool> cells_fresh{false}; // d_cells holds the current parameters' entries
     uint64_t cells_rays = 0;  // rays queried without it since the parameters changed
-    bool cells_off = false;   // never: no memory for it, or Adam steps captured into a graph
+    bool cells_off = false;   // never again: Adam steps captured into a graph change the parameters unseen
     cudaEvent_t ev_params = nullptr; // after the last nbvh_adam_step, on its stream
     std::mutex cells_mu;      // guards the six above (cells_fresh is also read without it)
     uint32_t *h_readback = nullptr; // two page-locked words a call reads its status and loss back into
