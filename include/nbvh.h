@@ -311,6 +311,13 @@ nbvh_status nbvh_set_ignore_neural_blas(nbvh_handle *h, int ignore);
  * It changes no result, only the order in which the classic kernel and the neural query's first
  * pass take the rays. */
 nbvh_status nbvh_set_ray_ordering(nbvh_handle *h, int enable);
+/* Cell copy (no counterpart in the reference): for each cell of the coarsest hash-grid levels the entries
+ * of its 8 corners side by side, which the encoder of batches above 16,384 rays reads instead of
+ * gathering them from the table (2^22 rays: 2.6 ms per query with it, 2.8 without). It is built on the
+ * device once 2^21 rays have been queried in such batches on one set of parameters, and takes as many
+ * levels as max_bytes holds: 201,326,592 (192 MiB) unless set lower here, 0 for no copy. It changes no
+ * result. What is there is freed; no query of the handle may run meanwhile, in a scene or server either. */
+nbvh_status nbvh_set_cell_copy(nbvh_handle *h, uint64_t max_bytes);
 
 /* ---------------------------------------------------------------------------------------------
  * Queries (device buffers, asynchronous on stream)

@@ -422,6 +422,10 @@ class NBVH:
     def set_ray_ordering(self, enable):
         self._check(self.lib.nbvh_set_ray_ordering(self.h, 1 if enable else 0))
 
+    def set_cell_copy(self, max_bytes):
+        """Device memory for the cell copy of the coarse hash-grid levels (0: none)."""
+        self._check(self.lib.nbvh_set_cell_copy(self.h, max_bytes))
+
     def set_ignore_neural_blas(self, ignore):
         self._check(self.lib.nbvh_set_ignore_neural_blas(self.h, int(bool(ignore))))
 

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) k_build_cells(const __grid_constant__ Gri
 
 } // namespace
 
-size_t plan_cells(const GridParams &grid, CellParams &cp)
+size_t plan_cells(const GridParams &grid, CellParams &cp, size_t max_bytes)
 {
     cp = CellParams{};
     if (grid.n_features == 2u && (grid.n_levels & 3u) != 0u)
@@ -119,7 +119,7 @@ size_t plan_cells(const GridParams &grid, CellParams &cp)
         if (!(last >= 0.f && last < 1024.f))
             break;
         const size_t n = (size_t)last + 1u;
-        if ((total + n * n * n) * 16u * grid.n_features > kCellBytes)
+        if ((total + n * n * n) * 16u * grid.n_features > max_bytes)
             break;
         cp.dim[l] = (uint32_t)n;
         total += n * n * n;

@@ -736,7 +736,7 @@ nbvh_status nbvh_create(const nbvh_config *cfg, int device, nbvh_handle **out)
         cuda_check(h->d_loss_sum.resize(1u), "alloc loss");
         compute_layout(h->cfg, h->layout, h->grid);
         apply_device_level_scales(h->cfg, h->layout, h->grid);
-        h->n_cells = plan_cells(h->grid, h->cell_levels);
+        h->n_cells = plan_cells(h->grid, h->cell_levels, h->cells_limit);
         std::vector<float> p(h->layout.n_params);
         init_params(h->cfg, h->layout, p.data());
         upload_params(h, p.data(), true);
@@ -1031,6 +1031,19 @@ extern "C" {
 nbvh_status nbvh_set_ray_ordering(nbvh_handle *h, int enable)
 {
     return guarded(h, [&]() { h->ray_ordering = enable != 0; });
+}
+
+nbvh_status nbvh_set_cell_copy(nbvh_handle *h, uint64_t max_bytes)
+{
+    return guarded(h, [&]() {
+        std::lock_guard<std::mutex> lock(h->cells_mu);
+        h->cells_limit = (size_t)std::min<uint64_t>(max_bytes, kCellBytes);
+        h->n_cells = plan_cells(h->grid, h->cell_levels, h->cells_limit);
+        h->cells_fresh = false;
+        h->cells_rays = 0;
+        h->model_version++; // captured query graphs may hold the copy
+        h->d_cells.release();
+    });
 }
 
 nbvh_status nbvh_query_closest_classic(nbvh_handle *h, const nbvh_ray *d_rays, uint32_t n, nbvh_hit *d_hits,
@@ -2028,7 +2041,7 @@ nbvh_status nbvh_load(nbvh_handle *h, const char *path)
         h->cfg = cfg;
         h->layout = L;
         h->grid = g;
-        h->n_cells = plan_cells(h->grid, h->cell_levels);
+        h->n_cells = plan_cells(h->grid, h->cell_levels, h->cells_limit);
         params_changed(h);
         h->vertices.swap(verts);
         h->indices.swap(idx);

@@ -93,6 +93,7 @@ struct CellParams {
     uint32_t dim[kMaxLevels];
     uint32_t offset[kMaxLevels];
 };
+constexpr size_t kCellBytes = (size_t)192 << 20; // the copy's size at most
 
 // Constants of the neural traversal and decode (NeuralBVHRendererConstants /
 // PathTracingOutputConstants subsets).
@@ -363,6 +364,7 @@ struct nbvh_handle {
     nbvh::DeviceBuffer<uint4> d_cells;
     nbvh::CellParams cell_levels{};
     size_t n_cells = 0;       // cells of the layout (0: none)
+    size_t cells_limit = nbvh::kCellBytes; // nbvh_set_cell_copy
     std::atomic<bool> cells_fresh{false}; // d_cells holds the current parameters' entries
     uint64_t cells_rays = 0;  // rays queried without it since the parameters changed
     bool cells_off = false;   // never again: Adam steps captured into a graph change the parameters unseen
@@ -611,10 +613,9 @@ constexpr uint32_t kTailOnlyRays = 1u << 14; // batches up to this size run the 
 // Cell copy of the coarse levels of a hash grid: for every cell of such a level the entries of its 8
 // corners side by side (corner c at c * F halves), so that a point's lookup on the level is one 16F-byte
 // read instead of 8 entries in 4 to 8 sectors. plan_cells picks the levels (as many of the coarsest as
-// kCellBytes holds) and returns the number of cells; launch_build_cells fills the copy from the
+// max_bytes, at most kCellBytes, holds) and returns the number of cells; launch_build_cells fills the copy from the
 // 16-bit parameters.
-constexpr size_t kCellBytes = (size_t)192 << 20;
-size_t plan_cells(const GridParams &grid, CellParams &cp);
+size_t plan_cells(const GridParams &grid, CellParams &cp, size_t max_bytes);
 cudaError_t launch_build_cells(const __half *params_h, const GridParams &grid, const CellParams &cp,
                                uint32_t n_hidden_layers, uint4 *cells, cudaStream_t s);
 

@@ -1,5 +1,5 @@
 """When the cell copy of the coarse grid levels takes memory: only where a kernel reads it, again after an
-allocation that failed, and no longer once it is given up."""
+allocation that failed, no longer once it is given up, and no more than the caller allows."""
 
 import ctypes as C
 
@@ -101,3 +101,24 @@ def test_copy_given_up_is_freed(built):
         for _ in range(3):
             h.query_closest_neural(rays)
         assert _allocations() == before
+
+
+def test_caller_sets_the_size(built):
+    h, rays = _model()
+    with h:
+        h.set_cell_copy(0)
+        h.query_closest_neural(rays)
+        before = _allocations()
+        ref = h.query_closest_neural(rays)
+        for _ in range(3):
+            assert torch.equal(h.query_closest_neural(rays), ref)
+        assert _allocations() == before
+        free = torch.cuda.mem_get_info()[0]
+        taken = []
+        for limit in (16 << 20, 192 << 20, 1 << 40, 1 << 10, 192 << 20, 0):
+            h.set_cell_copy(limit)
+            for _ in range(3):
+                assert torch.equal(h.query_closest_neural(rays), ref)
+            taken.append(free - torch.cuda.mem_get_info()[0])
+        small, full, more, none, again, off = taken
+        assert 0 < small <= 18 << 20 and small < full <= 194 << 20 and more == again == full and none == off == 0
