@@ -611,7 +611,8 @@ typedef struct nbvh_server nbvh_server;
 typedef struct nbvh_server_config {
     uint32_t n_slots;          /* batches in flight at once (default 4) */
     uint32_t max_batch_rays;   /* rays (or render paths) one batch may hold (default 2^22) */
-    uint64_t hbm_budget_bytes; /* device memory all slots' buffers may take together (default 150 GiB) */
+    uint64_t hbm_budget_bytes; /* device memory all slots' buffers may take together (default 150 GiB); a
+                                  model's cell copy (nbvh_set_cell_copy) is used if it fits beside them */
     uint32_t use_graphs;       /* replay captured CUDA graphs per batch-size bucket (default 1) */
     uint32_t autotune;         /* time the launch-parameter candidates per bucket (default 1) */
     uint32_t query_slots;      /* of the n_slots, how many take query requests only, on streams of the

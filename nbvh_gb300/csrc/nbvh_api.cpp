@@ -2216,26 +2216,29 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
         q.generation++;
 }
 
-void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
+bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
 {
     std::lock_guard<std::mutex> lock(h->cells_mu);
     if (h->cells_off)
         h->d_cells.release();
-    if (h->cells_fresh || h->cells_off || h->n_cells == 0u || h->cfg.bvh.ignore_neural_blas || !uses_cells(n))
-        return;
+    if (h->cells_off || h->n_cells == 0u || h->cfg.bvh.ignore_neural_blas || !uses_cells(n))
+        return false;
+    if (h->cells_fresh)
+        return true;
     if (h->cells_rays + n < kCellsAfterRays) { // a program may train again before its next query
         h->cells_rays += n;
-        return;
+        return false;
     }
     const size_t words = h->n_cells * h->layout.n_features_per_level;
     if (h->d_cells.count < words) {
         if (!may_allocate)
-            return;
-        h->model_version++; // captured graphs hold the address
+            return false;
+        if (h->d_cells.ptr)
+            h->model_version++; // captured graphs hold the address
         if (h->d_cells.resize(words) != cudaSuccess) { // no room now: as many rays on the table alone
             cudaGetLastError();
             h->cells_rays = 0;
-            return;
+            return false;
         }
     }
     if (h->ev_params) // an Adam step on another stream may still be writing the parameters
@@ -2245,6 +2248,7 @@ void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
                "cell copy");
     cuda_check(cudaStreamSynchronize(s), "sync");
     h->cells_fresh = true;
+    return true;
 }
 
 // The neural query itself on explicit per-call buffers (context q, counters): reads only the
@@ -2289,6 +2293,8 @@ uint32_t run_neural_query(const nbvh_handle *h, QueryContext &q, QueryCounters *
     res.cells = h->cells_fresh ? h->d_cells.ptr : nullptr;
     res.cell_levels = h->cell_levels;
     if (tune) {
+        if (tune->table_only)
+            res.cells = nullptr;
         res.visits_per_round = tune->visits_per_round;
         res.encode_blocks_per_sm = tune->encode_blocks_per_sm;
         res.unchecked_steps = tune->unchecked_steps;

@@ -538,6 +538,7 @@ struct StepResources {
     uint16_t *row_keys = nullptr;
     const uint4 *cells = nullptr;  // cell copy of the coarse grid levels (nullptr: the table alone)
     CellParams cell_levels{};
+    bool table_only = false;       // read the table even where the cell copy is up to date
     bool stall = false;            // failure-path tests: the MLP kernels wait on a barrier nothing arrives at
 };
 
@@ -767,13 +768,17 @@ namespace nbvh {
 // memory; no kernel runs).
 void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n);
 // Brings the handle's cell copy up to date on stream s for a query of n rays and waits for it; called
-// before the queries that may use it (one that finds it stale, or not allocated, reads the table
-// instead). It is built once kCellsAfterRays rays have been queried since the parameters changed:
-// building it takes 150 us, which it saves over 2 to 3 million rays (2^22: 2,880 -> 2,700 us, 2^18: 655
-// -> 620), and a program that trains between its frames never pays for it.
+// before the queries that may use it. Returns whether the query reads it; one that finds it stale, or not
+// allocated, reads the table instead. It is built once kCellsAfterRays rays have been queried since the
+// parameters changed: building it takes 150 us, which it saves over 2 to 3 million rays (2^22: 2,880 -> 2,700
+// us, 2^18: 655 -> 620), and a program that trains between its frames never pays for it.
 constexpr uint32_t kCellsAfterRays = 1u << 21;
 constexpr bool uses_cells(uint32_t n) { return n > kTailOnlyRays; }
-void ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate = true);
+bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate = true);
+inline uint64_t cell_copy_bytes(const nbvh_handle *h)
+{
+    return (uint64_t)h->n_cells * h->layout.n_features_per_level * sizeof(uint4);
+}
 
 // The neural query on explicit per-call buffers (context q, counters): reads only the handle's
 // scene, cut and parameters, so several contexts may run it at once on different streams.

@@ -32,6 +32,7 @@
 #include <memory>
 #include <random>
 #include <thread>
+#include <tuple>
 #include <vector>
 
 #include "nbvh_internal.h"
@@ -54,6 +55,7 @@ struct Tuning {
 
 struct Model {
     nbvh_handle *h = nullptr;
+    uint64_t cell_bytes = 0;         // of the budget: what the model's cell copy may take
     std::map<uint32_t, Tuning> tune; // by bucket
 };
 
@@ -76,9 +78,10 @@ struct Work {
 
 struct GraphKey {
     uint32_t model, bucket, depth;
+    bool cells; // reads the model's cell copy
     bool operator<(const GraphKey &o) const
     {
-        return model != o.model ? model < o.model : bucket != o.bucket ? bucket < o.bucket : depth < o.depth;
+        return std::tie(model, bucket, depth, cells) < std::tie(o.model, o.bucket, o.depth, o.cells);
     }
 };
 
@@ -126,6 +129,7 @@ struct nbvh_server {
     nbvh_server_config cfg{};
     int device = 0;
     int num_sms = 0;
+    uint64_t budget_left = 0; // bytes of the HBM budget that neither slots nor cell copies have
     std::vector<Model> models;
     std::vector<std::unique_ptr<Slot>> slots;
     std::mutex mu;
@@ -193,9 +197,10 @@ StepResources tuning_of(const Model &m, uint32_t bucket)
 // pass and the first kGraphSteps steps, ending with a copy of the wave counters to the host. Nothing
 // runs; the kernels' attributes are set beforehand (a captured launch cannot set them). A shape
 // whose capture fails is recorded without a graph and keeps running directly.
-cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t bucket, uint32_t depth)
+cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t bucket, uint32_t depth,
+                             bool cells)
 {
-    const GraphKey key{model_id, bucket, depth};
+    const GraphKey key{model_id, bucket, depth, cells};
     auto g = sl.graphs.find(key);
     if (g != sl.graphs.end())
         return g->second;
@@ -203,6 +208,7 @@ cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint
     StepResources cap = tuning_of(m, bucket);
     cap.unchecked_steps = kGraphSteps;
     cap.capture_only = true;
+    cap.table_only = !cells;
     cudaGraphExec_t exec = nullptr;
     // the captured launches cannot set kernel attributes: set those of every variant first
     cuda_check(configure_query_kernels(), "kernel attributes");
@@ -239,9 +245,12 @@ void slot_query(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t n, uint3
         cuda_check(cudaMemcpyAsync(sl.rays.ptr + n, srv->dead, (size_t)(bucket - n) * sizeof(nbvh_ray),
                                    cudaMemcpyDeviceToDevice, sl.stream),
                    "pad batch");
-    const StepResources tune = tuning_of(m, bucket);
+    StepResources tune = tuning_of(m, bucket);
     nbvh_handle *h = m.h;
-    ensure_cells(h, sl.stream, kCellsAfterRays); // the model may have been trained since its last request
+    // the copy follows the parameters (the model may have been trained since its last request); while it is
+    // stale or not there the batch reads the table, from a graph of its own
+    const bool cells = cell_copy_bytes(h) <= m.cell_bytes && ensure_cells(h, sl.stream, bucket);
+    tune.table_only = !cells;
     // a model whose device arrays were reallocated since its graphs were captured (a new cut, a
     // grown learned cut, a new mesh) drops them; the context is resized for the new cut first
     auto ver = sl.model_versions.find(model_id);
@@ -261,7 +270,7 @@ void slot_query(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t n, uint3
         }
         ver->second = h->model_version;
     }
-    cudaGraphExec_t exec = graphable(srv, h) ? ensure_graph(srv, sl, model_id, bucket, depth) : nullptr;
+    cudaGraphExec_t exec = graphable(srv, h) ? ensure_graph(srv, sl, model_id, bucket, depth, cells) : nullptr;
     if (!exec) {
         run_neural_query(h, sl.q, sl.counters.ptr, sl.rays.ptr, bucket, depth, false, sl.hits.ptr, sl.stream, &tune);
         return;
@@ -523,6 +532,7 @@ void autotune(nbvh_server *srv, uint32_t model_id)
                     t.visits_per_round = v;
                     t.encode_blocks_per_sm = eb;
                     t.stage_cut = stage;
+                    t.table_only = true;
                     run_neural_query(h, sl.q, sl.counters.ptr, sl.rays.ptr, b, 1u, false, sl.hits.ptr, sl.stream, &t);
                     float ms_total = 0.f;
                     for (int rep = 0; rep < 2; rep++) {
@@ -588,6 +598,7 @@ nbvh_status nbvh_server_create(const nbvh_server_config *cfg, int device, nbvh_s
             pow2 <<= 1;
         require(cap >= kMinBucket, NBVH_EINVAL, "HBM budget too small for one minimal batch per slot");
         cap = pow2;
+        srv->budget_left = cfg->hbm_budget_bytes - (uint64_t)cfg->n_slots * cap * kBytesPerRay;
         int least_priority = 0, greatest_priority = 0; // numerically lower = higher priority
         cuda_check(cudaDeviceGetStreamPriorityRange(&least_priority, &greatest_priority), "stream priorities");
         std::vector<nbvh_ray> dead(cap);
@@ -630,6 +641,13 @@ nbvh_status nbvh_server_add_model(nbvh_server *srv, nbvh_handle *h, uint32_t *mo
         }
         Model m;
         m.h = h;
+        for (const Model &o : srv->models) // the handle's copy is counted once
+            if (o.h == h)
+                m.cell_bytes = o.cell_bytes;
+        if (m.cell_bytes == 0u && cell_copy_bytes(h) <= srv->budget_left) {
+            m.cell_bytes = cell_copy_bytes(h);
+            srv->budget_left -= m.cell_bytes;
+        }
         srv->models.push_back(m);
         const uint32_t id = (uint32_t)srv->models.size() - 1u;
         // size every slot's query context for this model now, so serving never allocates; a context
@@ -644,7 +662,6 @@ nbvh_status nbvh_server_add_model(nbvh_server *srv, nbvh_handle *h, uint32_t *mo
                 sl->graphs.clear();
             }
         }
-        ensure_cells(h, srv->slots[0]->stream, kCellsAfterRays);
         if (srv->cfg.autotune) {
             autotune(srv, id);
         } else { // one direct query sets the kernels' attributes before any capture
@@ -658,7 +675,7 @@ nbvh_status nbvh_server_add_model(nbvh_server *srv, nbvh_handle *h, uint32_t *mo
             for (auto &sl : srv->slots)
                 for (uint32_t b = kMinBucket; b <= sl->capacity; b <<= 1)
                     for (uint32_t depth = 1; depth <= 2; depth++)
-                        ensure_graph(srv, *sl, id, b, depth);
+                        ensure_graph(srv, *sl, id, b, depth, false);
         for (auto &sl : srv->slots)
             sl->model_versions[id] = h->model_version;
         *model_id = id;
