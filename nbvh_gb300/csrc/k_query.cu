@@ -20,7 +20,7 @@
 // Splitting the step lets each phase run at the occupancy it needs: the gathers of K3 with 32
 // warps per SM, the MLP with its accumulators in tensor memory, the divergent traversal with the
 // cut read through L1 (or staged in shared memory: StepResources::stage_cut). Every kernel reads the
-// list length from device memory; the host reads it once, after the tail kernel (one 16-byte copy).
+// list length from device memory; the host reads one status word, after the tail kernel.
 #include <type_traits>
 
 #include "device_math.cuh"
@@ -1425,7 +1425,6 @@ __global__ void __launch_bounds__(kTailThreads, SMEM_CUT ? 1 : 2) k_wave_tail(co
 }
 
 constexpr size_t kSmemLimit = (size_t)kMaxDynamicSmem;
-constexpr uint32_t kStepsPerCheck = 4;
 
 template <bool SMEM_CUT, bool BF16, bool FP8>
 cudaError_t launch_tail_variant(const WaveArgs &a, uint32_t it, int num_sms, bool configure, size_t smem,
@@ -1460,10 +1459,11 @@ cudaError_t launch_tail(const WaveArgs &a, uint32_t it, int num_sms, bool config
                     : launch_tail_variant<false, false, false>(a, it, num_sms, configure, smem, s);
 }
 
-// The kernels of steps [it0, it1): sort, K3, K4, K2 per step, no host synchronisation.
+// The kernels of the first `steps` steps: sort, K3, K4, K2 per step, or the tail kernel; no host
+// synchronisation.
 template <bool SMEM_CUT>
-cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem, int num_sms, uint32_t it0,
-                          uint32_t it1, cudaStream_t s, uint32_t &launches)
+cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem, int num_sms, uint32_t steps,
+                          cudaStream_t s, uint32_t &launches)
 {
     cudaError_t e = cudaSuccess;
     const uint32_t F = a.grid.n_features;
@@ -1472,10 +1472,9 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
                                     : kEncodeBlocksPerSm;
     const uint32_t enc_blocks = (uint32_t)num_sms * enc_per_sm;
     const uint32_t dec_blocks = (uint32_t)num_sms * (SMEM_CUT ? 1u : 2u);
-    for (uint32_t it = it0; it < it1; it++) {
+    for (uint32_t it = 0; it < steps; it++) {
         if (it == a.tail_at) {
-            // the rest of the query in one launch; in a captured graph the list counters are cleared
-            // after it, so that the copy the graph ends with reads an empty list
+            // the rest of the query in one launch
             if (a.perm) {
                 k_wave_sort<<<(uint32_t)num_sms, kSortThreads, sort_smem_bytes(a.n_sort_nodes), s>>>(a, it);
                 e = cudaGetLastError();
@@ -1484,8 +1483,6 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
                 launches++;
             }
             e = launch_tail(a, it, num_sms, !r.capture_only, r.stage_cut, s);
-            if (e == cudaSuccess && r.capture_only)
-                e = cudaMemsetAsync(a.wave_counts, 0, 3u * sizeof(uint32_t), s);
             if (e != cudaSuccess)
                 return e;
             launches++;
@@ -1544,14 +1541,10 @@ cudaError_t enqueue_steps(const WaveArgs &a, const StepResources &r, size_t dec_
     return cudaSuccess;
 }
 
-// Copies the wave counters to the host words and waits for them; 1 if the list of step `it` is
-// empty (the query is done), 0 if not, or an error (cudaErrorTimeout if the MLP's bounded wait
-// gave up).
-cudaError_t check_done(const WaveArgs &a, const StepResources &r, uint32_t it, cudaStream_t s, bool &done)
+// Waits for the copy of the counters; cudaErrorTimeout if a bounded wait of the MLP gave up.
+cudaError_t wait_steps(const StepResources &r, cudaStream_t s)
 {
-    cudaError_t e = cudaMemcpyAsync(r.h_words, a.wave_counts, 4u * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess)
-        return e;
+    cudaError_t e;
     if (r.ev) {
         e = cudaEventRecord(r.ev, s);
         if (e == cudaSuccess)
@@ -1561,22 +1554,16 @@ cudaError_t check_done(const WaveArgs &a, const StepResources &r, uint32_t it, c
     }
     if (e != cudaSuccess)
         return e;
-    if (r.h_words[3] != 0u)
-        return cudaErrorTimeout;
-    done = r.h_words[it % 3u] == 0u;
-    return cudaSuccess;
+    return r.h_words[3] != 0u ? cudaErrorTimeout : cudaSuccess;
 }
 
-// The step loop from step `from` (after `unchecked` steps launched without a host check when from
-// is 0): the steps up to and with the tail kernel, which answers every ray left, then one host
-// check; where no tail kernel comes (a step limit below it, a resumed query) batches of
-// kStepsPerCheck steps, the host reading the list length after each. The loop ends when a list comes
-// out empty or at the step cap (each ray at most max_traversal_steps + 1 segments) plus the final
-// capping step. With capture_only the unchecked steps and the copy of the counters are only
-// enqueued (for stream capture) and nothing waits.
+// The steps of a query: up to and with the tail kernel, which answers every ray left, or to the step cap
+// (each ray at most max_traversal_steps + 1 segments, plus the final capping step) where that comes
+// first; then the host waits. With capture_only the steps and the copy of the counters are only enqueued
+// (for stream capture) and nothing waits.
 template <bool SMEM_CUT>
 cudaError_t run_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem, int num_sms, uint32_t max_steps,
-                      uint32_t from, cudaStream_t s, uint32_t &launches)
+                      cudaStream_t s, uint32_t &launches)
 {
     cudaError_t e = cudaSuccess;
     if (!r.capture_only) { // kernel attributes are set outside stream capture (an earlier run set them)
@@ -1586,34 +1573,13 @@ cudaError_t run_steps(const WaveArgs &a, const StepResources &r, size_t dec_smem
         if (e != cudaSuccess)
             return e;
     }
-    const uint32_t limit = max_steps + 2u;
-    uint32_t it = from;
-    if (from == 0u && r.unchecked_steps > 0u) {
-        const uint32_t u = r.unchecked_steps < limit ? r.unchecked_steps : limit;
-        e = enqueue_steps<SMEM_CUT>(a, r, dec_smem, num_sms, 0u, u, s, launches);
-        if (e != cudaSuccess)
-            return e;
-        it = u;
-        if (r.capture_only)
-            return cudaMemcpyAsync(r.h_words, a.wave_counts, 4u * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        bool done = false;
-        e = check_done(a, r, it, s, done);
-        if (e != cudaSuccess || done || it > a.tail_at)
-            return e;
-    }
-    while (it < limit) {
-        const uint32_t want = it <= a.tail_at ? a.tail_at + 1u - it : kStepsPerCheck;
-        const uint32_t batch = (limit - it) < want ? (limit - it) : want;
-        e = enqueue_steps<SMEM_CUT>(a, r, dec_smem, num_sms, it, it + batch, s, launches);
-        if (e != cudaSuccess)
-            return e;
-        it += batch;
-        bool done = false;
-        e = check_done(a, r, it, s, done);
-        if (e != cudaSuccess || done || it > a.tail_at)
-            return e;
-    }
-    return cudaSuccess;
+    const uint32_t steps = a.tail_at > 1u && max_steps < a.tail_at - 1u ? max_steps + 2u : a.tail_at + 1u;
+    e = enqueue_steps<SMEM_CUT>(a, r, dec_smem, num_sms, steps, s, launches);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(r.h_words, a.wave_counts, 4u * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess || r.capture_only)
+        return e;
+    return wait_steps(r, s);
 }
 
 } // namespace
@@ -1741,10 +1707,6 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     a.late_from = res.drain_host ? res.drain_step + 1u : 0xFFFFFFFFu;
     const size_t smem_cut = (size_t)n_cut_nodes * 56u;
     const bool use_smem_cut = res.stage_cut && smem_cut <= kSmemLimit;
-    if (res.resume_from > 0u) // continue a query whose first steps ran from a captured graph
-        return use_smem_cut
-                   ? run_steps<true>(a, res, smem_cut, num_sms, nc.max_traversal_steps, res.resume_from, s, *launches)
-                   : run_steps<false>(a, res, 0, num_sms, nc.max_traversal_steps, res.resume_from, s, *launches);
     // words 0-2: rotating list lengths; 3: the MLP's error word; 4-6: rotating work counters of
     // the decode kernel; 7: work counter of the first pass
     const uint32_t sort_words = sort ? 2u * a.n_sort_nodes : 0u;
@@ -1785,8 +1747,8 @@ cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds,
     if (e != cudaSuccess)
         return e;
     if (use_smem_cut)
-        return run_steps<true>(a, res, smem_cut, num_sms, nc.max_traversal_steps, 0u, s, *launches);
-    return run_steps<false>(a, res, 0, num_sms, nc.max_traversal_steps, 0u, s, *launches);
+        return run_steps<true>(a, res, smem_cut, num_sms, nc.max_traversal_steps, s, *launches);
+    return run_steps<false>(a, res, 0, num_sms, nc.max_traversal_steps, s, *launches);
 }
 
 namespace {

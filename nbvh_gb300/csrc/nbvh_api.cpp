@@ -2297,9 +2297,7 @@ uint32_t run_neural_query(const nbvh_handle *h, QueryContext &q, QueryCounters *
             res.cells = nullptr;
         res.visits_per_round = tune->visits_per_round;
         res.encode_blocks_per_sm = tune->encode_blocks_per_sm;
-        res.unchecked_steps = tune->unchecked_steps;
         res.capture_only = tune->capture_only;
-        res.resume_from = tune->resume_from;
         res.drain_host = tune->drain_host;
         res.drain_stream = tune->drain_stream;
         res.drain_snap = tune->drain_snap;

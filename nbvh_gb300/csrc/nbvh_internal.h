@@ -504,12 +504,10 @@ struct StepResources {
     TensorMapBytes feature_map;
     uint32_t *h_words;
     cudaEvent_t ev;
-    // launch parameters (0 = default) and the graph-capture split of the step loop
+    // launch parameters (0 = default)
     uint32_t visits_per_round = 0;     // node visits per traversal round between lane refills
     uint32_t encode_blocks_per_sm = 0; // blocks of 256 encoder threads per SM
-    uint32_t unchecked_steps = 0;      // steps launched before the first host check
-    bool capture_only = false;         // enqueue the unchecked steps and a counter copy, then return
-    uint32_t resume_from = 0;          // > 0: skip the first pass and continue the checked loop here
+    bool capture_only = false;         // enqueue the steps and a copy of the counters, then return
     // early host copy of the records (page-locked destination, device address): taken on
     // drain_stream after the decode of step drain_step; rays finishing later go to late_list
     nbvh_neural_hit *drain_host = nullptr;
@@ -573,9 +571,8 @@ constexpr size_t kNoallocBytes = 2u * kNoallocListBytes + kNoallocFeatureBytes +
 // device and cached. Fails with cudaErrorInvalidDevice for device ids beyond the cache.
 cudaError_t noalloc_scratch(int device, NoallocScratch *out);
 
-// Wavefront neural query (k_query.cu): first-leaf pass, then batches of K3 -> K4 -> K2 steps,
-// the list length checked by the host after each batch. Returns when the loop has finished;
-// cudaErrorTimeout if a bounded wait inside the tensor-core MLP gave up.
+// Wavefront neural query (k_query.cu): first-leaf pass, K3 -> K4 -> K2 steps, tail kernel. Returns when
+// it is done; cudaErrorTimeout if a bounded wait inside the tensor-core MLP gave up.
 cudaError_t launch_wave_query(const float4 *dilated_nodes, const float4 *bounds, uint32_t n_cut_nodes,
                               const uint8_t *non_neural, const __half *params_h, const GridParams &grid,
                               const NeuralConsts &nc, uint32_t n_hidden_layers, const nbvh_ray *rays, uint32_t n,

@@ -16,9 +16,8 @@
 //    scheduler starts its blocks first as resident ones finish. While the lane runs a batch, the
 //    render slots hold back their next bounce query (for at most kYieldMs), so the lane's kernels
 //    meet only the render work already on the device.
-//  * Graphs. A query batch is padded to a power-of-two bucket; the first part of its query (the
-//    first-leaf pass and the first steps) is captured once per (slot, model, bucket) as a CUDA graph
-//    and replayed; the host then checks the list length and finishes any remaining steps directly.
+//  * Graphs. A query batch is padded to a power-of-two bucket; its query is captured once per (slot,
+//    model, bucket) as a CUDA graph and replayed.
 //  * Autotuning. When a model is added, each bucket's launch parameters (node visits per traversal
 //    round, encoder blocks per SM) are chosen by timing the candidates on rays through the model's
 //    scene box.
@@ -44,7 +43,6 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr uint32_t kMinBucket = 1u << 12;
-constexpr uint32_t kGraphSteps = 8;          // steps inside the captured graph
 constexpr uint64_t kBytesPerRay = 1024;      // query + path buffers per ray of slot capacity (upper bound)
 constexpr int kYieldMs = 20;                 // longest a render bounce waits for the query lane
 
@@ -193,9 +191,8 @@ StepResources tuning_of(const Model &m, uint32_t bucket)
     return t;
 }
 
-// Captures (once) the graph of a padded batch of `bucket` rays in the slot's buffers: the first-leaf
-// pass and the first kGraphSteps steps, ending with a copy of the wave counters to the host. Nothing
-// runs; the kernels' attributes are set beforehand (a captured launch cannot set them). A shape
+// Captures (once) the graph of a padded batch of `bucket` rays in the slot's buffers: the whole query,
+// ending with a copy of the wave counters to the host. Nothing runs; the kernels' attributes are set beforehand (a captured launch cannot set them). A shape
 // whose capture fails is recorded without a graph and keeps running directly.
 cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t bucket, uint32_t depth,
                              bool cells)
@@ -206,7 +203,6 @@ cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint
         return g->second;
     const Model &m = srv->models[model_id];
     StepResources cap = tuning_of(m, bucket);
-    cap.unchecked_steps = kGraphSteps;
     cap.capture_only = true;
     cap.table_only = !cells;
     cudaGraphExec_t exec = nullptr;
@@ -235,8 +231,8 @@ cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint
     return exec;
 }
 
-// Runs the neural query of a batch of n rays already in the slot's ray buffer: padded to its
-// bucket, the captured graph replayed (when graphs are on), then the host-checked remainder.
+// Runs the neural query of a batch of n rays already in the slot's ray buffer, padded to its bucket: the
+// captured graph replayed, or directly when graphs are off.
 void slot_query(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t n, uint32_t depth)
 {
     const Model &m = srv->models[model_id];
@@ -283,11 +279,6 @@ void slot_query(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t n, uint3
     cuda_check(cudaStreamSynchronize(sl.stream), "graph sync");
     if (sl.q.h_words[3] != 0u)
         fail(NBVH_ETIMEOUT, "tensor-core MLP: a bounded wait gave up");
-    if (sl.q.h_words[kGraphSteps % 3u] == 0u)
-        return; // the list of the first step after the graph is empty: done
-    StepResources rest = tune;
-    rest.resume_from = kGraphSteps;
-    run_neural_query(h, sl.q, sl.counters.ptr, sl.rays.ptr, bucket, depth, false, sl.hits.ptr, sl.stream, &rest);
 }
 
 // The path tracer's per-bounce query on a slot: the bounce's rays are copied into the slot's ray
