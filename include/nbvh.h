@@ -744,14 +744,13 @@ nbvh_status nbvh_debug_device_level_scales(const nbvh_config *cfg, int device, f
  * trace: a renderer whose GPU memory is reserved up front and must not grow mid-frame, or a host
  * thread that may not take the device-wide synchronisation an allocation can cause. The ordinary
  * query grows per-handle buffers to the largest batch seen; this one allocates nothing. Its
- * scratch (the per-ray traversal state, the network inputs and outputs of a step, the node order,
- * the fallback list and the counters: about 660 bytes per ray, 10.8 MB in all) is one fixed buffer
+ * scratch (the per-ray traversal state, the fallback list and the counters: 180 bytes per ray, 2.9 MB
+ * in all; batches of this size need no buffers between steps) is one fixed buffer
  * of NBVH_NOALLOC_MAX_RAYS rays compiled into the library, one copy per device, created when the
  * library's device code is loaded.
  *  - n must be at most NBVH_NOALLOC_MAX_RAYS; a larger n returns NBVH_EINVAL and launches nothing.
  *    Split larger batches into several calls.
- *  - The call cannot be captured into a CUDA graph: it reads the list lengths back to the host
- *    between steps and synchronises its stream before it returns.
+ *  - The call cannot be captured into a CUDA graph: it synchronises its stream before it returns.
  *  - The first call on each device loads the library's device code there if nothing has yet
  *    (setup); a first call with n = 0 does only that, so a caller can take the setup's latency
  *    before its first frame. Every call looks the buffer's address up again (no allocation), so

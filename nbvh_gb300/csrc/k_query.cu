@@ -1809,27 +1809,15 @@ cudaError_t noalloc_scratch(int device, NoallocScratch *out)
         return e;
     unsigned char *p = static_cast<unsigned char *>(addr);
     const size_t n = kNoallocRays;
-    for (int k = 0; k < 2; k++) {
-        WaveList &L = out->lists[k];
-        L.od0 = reinterpret_cast<float4 *>(p);
-        L.od1 = L.od0 + n;
-        L.nv = L.od1 + n;
-        L.ar = L.nv + n;
-        L.meta = reinterpret_cast<uint4 *>(L.ar + n);
-        L.stack = reinterpret_cast<uint32_t *>(L.meta + n);
-        L.capacity = (uint32_t)n;
-        p += kNoallocListBytes;
-    }
-    out->features = reinterpret_cast<__half *>(p);
-    p += kNoallocFeatureBytes;
-    out->outputs = reinterpret_cast<float *>(p);
-    p += kNoallocOutputBytes;
-    out->wpacked = reinterpret_cast<__half *>(p);
-    p += kNoallocWeightBytes;
-    out->perm = reinterpret_cast<uint32_t *>(p);
-    out->node_bins = out->perm + n;
-    out->node_cursor = out->node_bins + 2u * kMaxSortNodes;
-    p += kNoallocSortBytes;
+    WaveList &L = out->list;
+    L.od0 = reinterpret_cast<float4 *>(p);
+    L.od1 = L.od0 + n;
+    L.nv = L.od1 + n;
+    L.ar = L.nv + n;
+    L.meta = reinterpret_cast<uint4 *>(L.ar + n);
+    L.stack = reinterpret_cast<uint32_t *>(L.meta + n);
+    L.capacity = (uint32_t)n;
+    p += kNoallocListBytes;
     out->fallback_list = reinterpret_cast<uint32_t *>(p);
     p += n * 4u;
     out->counters = reinterpret_cast<QueryCounters *>(p);

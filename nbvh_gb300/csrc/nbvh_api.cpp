@@ -583,28 +583,13 @@ void neural_query_noalloc(nbvh_handle *h, const nbvh_ray *d_rays, uint32_t n, ui
     } else {
         const NeuralConsts nc = make_neural_consts(h, depth, false);
         uint32_t host_words[4] = {0, 0, 0, 0}, launches = 0;
-        StepResources res;
-        res.features = sc.features;
-        res.outputs = sc.outputs;
-        res.wpacked = sc.wpacked;
-        res.perm = sc.perm;
-        res.node_bins = sc.node_bins;
-        res.node_cursor = sc.node_cursor;
+        const WaveList lists[2] = {sc.list, WaveList{}};
+        StepResources res{}; // the first pass and the tail kernel need no buffers but the list
         res.h_words = host_words;
-        res.ev = nullptr;
-        res.wait_ns = h->wait_limit_ns;
-        res.stall = h->debug_stall;
-        res.sort_key = h->n_sort_bins ? h->d_sort_key.ptr : nullptr;
-        res.n_sort_bins = h->n_sort_bins;
-        ensure_cells(h, s, n, false);
-        res.cells = h->cells_fresh ? h->d_cells.ptr : nullptr;
-        res.cell_levels = h->cell_levels;
-        cuda_check(make_feature_map(sc.features, h->layout.n_inputs, (uint32_t)kNoallocRays, &res.feature_map),
-                   "feature map");
         cuda_check(launch_wave_query(h->d_neural_dilated.ptr, h->d_neural_bounds.ptr,
                                      (uint32_t)h->neural_nodes.size(), h->any_non_neural ? h->d_non_neural.ptr : nullptr,
                                      h->d_params_h.ptr, h->grid, nc, (uint32_t)h->cfg.network.n_hidden_layers, d_rays,
-                                     n, d_hits, sc.counters, sc.fallback_list, sc.lists, sc.wave_counts, res,
+                                     n, d_hits, sc.counters, sc.fallback_list, lists, sc.wave_counts, res,
                                      mlp_prec(h), h->num_sms, s, &launches),
                    "neural query");
         if (h->any_non_neural || h->cfg.fallback_margin > 0.f)
@@ -2216,7 +2201,7 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
         q.generation++;
 }
 
-bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
+bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n)
 {
     std::lock_guard<std::mutex> lock(h->cells_mu);
     if (h->cells_off)
@@ -2231,8 +2216,6 @@ bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate)
     }
     const size_t words = h->n_cells * h->layout.n_features_per_level;
     if (h->d_cells.count < words) {
-        if (!may_allocate)
-            return false;
         if (h->d_cells.ptr)
             h->model_version++; // captured graphs hold the address
         if (h->d_cells.resize(words) != cudaSuccess) { // no room now: as many rays on the table alone

@@ -541,34 +541,22 @@ struct StepResources {
 };
 
 // Scratch of the allocation-free neural query: one static device buffer per device holding, for
-// NBVH_NOALLOC_MAX_RAYS rays, both wave lists, the feature rows and outputs of a step, the packed
-// weights, the node-sort buffers, the fallback list, the counters and the wave counters. Every region starts on a
+// NBVH_NOALLOC_MAX_RAYS rays, the list between the first pass and the tail kernel (which alone answer
+// batches of that size), the fallback list, the counters and the wave counters. Every region starts on a
 // 256-byte boundary.
 struct NoallocScratch {
-    WaveList lists[2];
-    __half *features;
-    float *outputs;
-    __half *wpacked;
-    uint32_t *perm;
-    uint32_t *node_bins;
-    uint32_t *node_cursor;
+    WaveList list;
     uint32_t *fallback_list;
     QueryCounters *counters;
     uint32_t *wave_counts;
 };
+constexpr uint32_t kTailOnlyRays = 1u << 14; // batches up to this size run the tail kernel alone (k_query.cu)
 constexpr size_t kNoallocRays = NBVH_NOALLOC_MAX_RAYS;
 static_assert(kNoallocRays % 64u == 0u, "regions must stay 256-byte aligned");
+static_assert(kNoallocRays <= kTailOnlyRays, "no wavefront step: no second list, features or outputs");
 constexpr size_t kNoallocListBytes = kNoallocRays * (4u * sizeof(float4) + sizeof(uint4) + kNeuralStackSize * 4u);
-constexpr size_t kNoallocFeatureBytes = kNoallocRays * kMaxInputs * 2u;
-constexpr size_t kNoallocOutputBytes = kNoallocRays * kOutputs * 4u;
-constexpr size_t kNoallocWeightBytes = // W0 at most 64 x 128, at most 7 more 64 x 64, output 16 x 64
-    ((kNeurons * kMaxInputs + (kMaxHiddenLayers - 1u) * kNeurons * kNeurons + kOutputsPadded * kNeurons) * 2u + 255u) &
-    ~size_t(255);
-constexpr size_t kNoallocSortBytes = kNoallocRays * 4u + 4u * kMaxSortNodes * 4u; // perm, bins, cursors
-constexpr size_t kNoallocBytes = 2u * kNoallocListBytes + kNoallocFeatureBytes + kNoallocOutputBytes +
-                                 kNoallocWeightBytes + kNoallocSortBytes + kNoallocRays * 4u + 256u + 256u;
-// The buffer's address on `device` (which must be current): looked up on the first call for that
-// device and cached. Fails with cudaErrorInvalidDevice for device ids beyond the cache.
+constexpr size_t kNoallocBytes = kNoallocListBytes + kNoallocRays * 4u + 256u + 256u;
+// The buffer's address on `device` (which must be current), looked up on every call.
 cudaError_t noalloc_scratch(int device, NoallocScratch *out);
 
 // Wavefront neural query (k_query.cu): first-leaf pass, K3 -> K4 -> K2 steps, tail kernel. Returns when
@@ -605,8 +593,6 @@ cudaError_t launch_segments(const float4 *dilated_nodes, const float4 *bounds, c
 cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, uint32_t n_hidden_layers,
                                const float *positions, uint32_t n, __half *features, bool bf16, int num_sms,
                                cudaStream_t s);
-
-constexpr uint32_t kTailOnlyRays = 1u << 14; // batches up to this size run the tail kernel alone (k_query.cu)
 
 // Cell copy of the coarse levels of a hash grid: for every cell of such a level the entries of its 8
 // corners side by side (corner c at c * F halves), so that a point's lookup on the level is one 16F-byte
@@ -771,7 +757,7 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n);
 // us, 2^18: 655 -> 620), and a program that trains between its frames never pays for it.
 constexpr uint32_t kCellsAfterRays = 1u << 21;
 constexpr bool uses_cells(uint32_t n) { return n > kTailOnlyRays; }
-bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n, bool may_allocate = true);
+bool ensure_cells(nbvh_handle *h, cudaStream_t s, uint32_t n);
 inline uint64_t cell_copy_bytes(const nbvh_handle *h)
 {
     return (uint64_t)h->n_cells * h->layout.n_features_per_level * sizeof(uint4);
