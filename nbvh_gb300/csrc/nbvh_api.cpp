@@ -1000,10 +1000,10 @@ const uint32_t *classic_order(nbvh_handle *h, uint32_t n)
 {
     if (!h->ray_ordering || n < kRaySortMin)
         return nullptr;
-    if (h->d_classic_order.count < n) {
+    if (h->d_classic_order.count < n)
         cuda_check(h->d_classic_order.resize(n), "alloc ray order");
+    if (h->d_classic_keys.count < n)
         cuda_check(h->d_classic_keys.resize(n), "alloc ray bins");
-    }
     if (h->d_classic_bins.count < kRayBinWords)
         cuda_check(h->d_classic_bins.resize(kRayBinWords), "alloc ray bin counts");
     return h->d_classic_order.ptr;
@@ -2167,10 +2167,10 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
             q.h_words[k] = 0;
     }
     const size_t cut = h->neural_nodes.size();
-    if (q.node_bins.count < 2u * kSubBins * cut) { // room for the octant sub-bins of every node
+    if (q.node_bins.count < 2u * kSubBins * cut) // room for the octant sub-bins of every node
         cuda_check(q.node_bins.resize(2u * kSubBins * cut), "alloc node counts");
+    if (q.node_cursor.count < 2u * kSubBins * cut)
         cuda_check(q.node_cursor.resize(2u * kSubBins * cut), "alloc node cursors");
-    }
     const uint32_t wb = packed_weight_bytes(h->layout.n_inputs, (uint32_t)h->cfg.network.n_hidden_layers);
     if (q.wpacked.count < wb / 2u)
         cuda_check(q.wpacked.resize(wb / 2u), "alloc packed weights");
@@ -2179,6 +2179,7 @@ void grow_query_context(const nbvh_handle *h, QueryContext &q, uint32_t n)
     if (!q.ev)
         cuda_check(cudaEventCreateWithFlags(&q.ev, cudaEventDisableTiming), "event");
     if (q.capacity < n || q.features.count < (size_t)n * h->layout.n_inputs) {
+        q.capacity = 0; // until every buffer is there again
         for (int k = 0; k < 2; k++) {
             cuda_check(q.od0[k].resize(n), "alloc wave state");
             cuda_check(q.od1[k].resize(n), "alloc wave state");
@@ -2327,7 +2328,8 @@ uint64_t render_path_core(const nbvh_handle *h, QueryContext &q, QueryCounters *
     const uint64_t n64 = (uint64_t)cam.width * cam.height * req->spp;
     require(n64 <= (1ull << 26), NBVH_EINVAL, "width * height * spp exceeds 2^26 paths");
     const uint32_t n = (uint32_t)n64;
-    if (pb.thr.count < n) {
+    if (pb.hits.count < n) {
+        pb.hits.release(); // the last one allocated: its size stands for all
         cuda_check(pb.thr.resize(n), "alloc path throughput");
         cuda_check(pb.rad.resize(n), "alloc path radiance");
         for (int k = 0; k < 2; k++) {

@@ -94,6 +94,7 @@ void ensure_object_capacity(nbvh_scene *sc, size_t m)
 {
     if (sc->obj_capacity >= m)
         return;
+    sc->obj_capacity = 0; // until every buffer is there again
     cuda_check(sc->obj_rays.resize(m), "alloc object rays");
     cuda_check(sc->obj_ids.resize(m), "alloc object ids");
     cuda_check(sc->obj_scale.resize(m), "alloc object scales");
@@ -117,10 +118,10 @@ void ensure_scene_buffers(nbvh_scene *sc, uint32_t n)
 ModelContext &context_of(nbvh_scene *sc, nbvh_handle *model, uint32_t n)
 {
     auto &slot = sc->contexts[model];
-    if (!slot) {
+    if (!slot)
         slot.reset(new ModelContext());
+    if (slot->counters.count < 1u)
         cuda_check(slot->counters.resize(1u), "alloc counters");
-    }
     grow_query_context(model, slot->q, n);
     return *slot;
 }
