@@ -1255,8 +1255,10 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
                               __half *features, __half *dfeat, __half *wpacked, float *wpart, float *grad,
                               float out_scale, float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
-                              uint64_t wait_ns, bool stall, const cudaEvent_t *marks)
+                              uint64_t wait_ns, bool stall, const cudaEvent_t *marks, uint32_t *launches)
 {
+    if (launches)
+        *launches = 0;
     if (n == 0)
         return cudaSuccess;
     cudaError_t e = marks ? cudaEventRecord(marks[0], s) : cudaSuccess;
@@ -1276,6 +1278,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
             return e;
         order = words;
     }
+    uint32_t count = order ? 5u : 3u; // the order, encoding, packing and scatter
     e = encode_rows(grid, table, positions, n, features, bf16, num_sms, s, order);
     if (e == cudaSuccess)
         e = launch_pack_weights(params_h, n_in, H, wpacked, s, clear ? status : nullptr,
@@ -1309,6 +1312,7 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
         kernel<<<blocks, kTcThreads, p.smem, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return e;
+        count++;
     }
     if (marks && (e = cudaEventRecord(marks[2], s)) != cudaSuccess)
         return e;
@@ -1317,6 +1321,8 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
              : scatter_rows<false>(grid, ws, positions, dfeat, n, grad + n_network_params, out_scale, s);
     if (e == cudaSuccess && marks)
         e = cudaEventRecord(marks[3], s);
+    if (launches)
+        *launches = count;
     return e;
 }
 

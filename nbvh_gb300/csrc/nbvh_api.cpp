@@ -1068,7 +1068,7 @@ nbvh_status nbvh_query_any_classic(nbvh_handle *h, const nbvh_ray *d_rays, uint3
         cuda_check(launch_classic(h->d_nodes.ptr, h->d_tris.ptr, d_rays, n, d_hits, true, order, h->classic_fast_div, s),
                    "classic");
         cuda_check(cudaEventRecord(h->ev1, s), "event");
-        h->last_launches = 1;
+        h->last_launches = order ? 3u : 1u;
         h->last_rays = n;
     });
 }
@@ -1472,20 +1472,23 @@ TrainCull train_cull(const nbvh_handle *h)
 }
 
 // forward + loss + backward of one batch: the gradient times the loss scale times out_scale into grad,
-// the loss into *loss_slot (added; `clear`: it and the status word start from zero)
-void batch_gradients(nbvh_handle *h, const float *d_pos, const float *d_tgt, uint32_t n, cudaStream_t s, float *grad,
+// the loss into *loss_slot (added; `clear`: it and the status word start from zero). Returns the number of
+// kernels launched.
+uint32_t batch_gradients(nbvh_handle *h, const float *d_pos, const float *d_tgt, uint32_t n, cudaStream_t s, float *grad,
                      float out_scale, float *loss_slot, bool clear, const cudaEvent_t *marks = nullptr)
 {
     ensure_train_workspace(h, n);
     const uint32_t H = (uint32_t)h->cfg.network.n_hidden_layers;
     cuda_check(cudaMemsetAsync(grad, 0, (size_t)h->layout.n_params * sizeof(float), s), "zero grad");
+    uint32_t launches = 0;
     cuda_check(launch_train_step(h->d_params_h.ptr, h->grid, H, make_loss_consts(h->cfg, n), d_pos, d_tgt, n,
                                  h->d_train_feat.ptr, h->d_train_dfeat.ptr, h->d_train_wpacked.ptr,
                                  h->d_train_wpart.ptr, grad, out_scale,
                                  loss_slot, clear, h->d_train_loss.ptr, h->d_status.ptr, mlp_bf16(h),
                                  h->cfg.network.precision == NBVH_PRECISION_FP8, h->num_sms, s, h->wait_limit_ns,
-                                 h->debug_stall, marks),
+                                 h->debug_stall, marks, &launches),
                "forward/backward");
+    return launches;
 }
 
 // Whether the kernels may add the gradient straight into the caller's buffer: it holds 16-byte
@@ -1517,8 +1520,8 @@ nbvh_status nbvh_compute_gradients(nbvh_handle *h, const float *d_positions, con
         const bool direct = direct_gradients(h, d_gradients, d_positions, d_targets, n);
         int exponent = 0;
         const bool fold = direct && std::frexp(scale, &exponent) == 0.5f;
-        batch_gradients(h, d_positions, d_targets, n, s, direct ? d_gradients : h->d_grad.ptr, fold ? 1.0f / scale : 1.0f,
-                        h->d_loss_sum.ptr, true);
+        const uint32_t launches = batch_gradients(h, d_positions, d_targets, n, s, direct ? d_gradients : h->d_grad.ptr,
+                                                  fold ? 1.0f / scale : 1.0f, h->d_loss_sum.ptr, true);
         if (!direct)
             cuda_check(cudaMemcpyAsync(d_gradients, h->d_grad.ptr, (size_t)h->layout.n_params * sizeof(float),
                                        cudaMemcpyDeviceToDevice, s),
@@ -1530,7 +1533,7 @@ nbvh_status nbvh_compute_gradients(nbvh_handle *h, const float *d_positions, con
         require(status == 0u, NBVH_ETIMEOUT, "tensor-core training kernel: a bounded wait gave up");
         if (h_loss)
             *h_loss = loss;
-        h->last_launches = 4;
+        h->last_launches = launches + (fold ? 0u : 1u);
     });
 }
 
@@ -1601,6 +1604,7 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
         const NeuralConsts nc = make_neural_consts(h, 1u, false);
         const uint32_t first = h->training_step;
         float lr_t = 0.f;
+        uint32_t launches = 0;
         cuda_check(cudaEventRecord(h->ev0, s), "event");
         for (uint32_t i = 0; i < steps; i++) {
             NodeSurvival survival{nullptr, nullptr, 1.0f, 0.0f, 0u};
@@ -1617,8 +1621,8 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
                                                h->d_train_nodes.ptr, learned_lod, &survival, h->d_sample_state.ptr,
                                                h->classic_fast_div, train_cull(h), h->num_sms, s),
                        "training samples");
-            batch_gradients(h, h->d_train_pos.ptr, h->d_train_tgt.ptr, n, s, h->d_grad.ptr, 1.0f,
-                            h->d_loss_sum.ptr + i, false, prof ? h->kprof->train_ev + 1 : nullptr);
+            launches += 3u + batch_gradients(h, h->d_train_pos.ptr, h->d_train_tgt.ptr, n, s, h->d_grad.ptr, 1.0f,
+                                             h->d_loss_sum.ptr + i, false, prof ? h->kprof->train_ev + 1 : nullptr);
             lr_t = adam_step_size(c, h->training_step);
             cuda_check(launch_adam(h->d_params.ptr, h->d_params_h.ptr, h->d_adam_m.ptr, h->d_adam_v.ptr, h->d_grad.ptr,
                                    h->layout.n_params, lr_t, c.optimizer.beta1, c.optimizer.beta2, c.optimizer.epsilon,
@@ -1646,7 +1650,7 @@ nbvh_status nbvh_run_optimisation(nbvh_handle *h, uint32_t steps, nbvh_train_sta
         float ms = 0.f;
         cuda_check(cudaEventElapsedTime(&ms, h->ev0, h->ev1), "elapsed");
         h->last_kernel_ms = ms;
-        h->last_launches = 7u * steps;
+        h->last_launches = launches; // of the steps, without a tree-cut session's
         if (stats) {
             double sum = 0.0;
             for (uint32_t i = 0; i < steps; i++)

@@ -690,9 +690,10 @@ cudaError_t launch_train_step(const __half *params_h, const GridParams &grid, ui
                               const LossConsts &lc, const float *positions, const float *targets, uint32_t n,
                               __half *features, __half *dfeat, __half *wpacked, float *wpart, float *grad,
                               float out_scale, float *loss_sum, bool clear, float *sample_loss, uint32_t *status, bool bf16, bool fp8, int num_sms, cudaStream_t s,
-                              uint64_t wait_ns = 0, bool stall = false, const cudaEvent_t *marks = nullptr);
+                              uint64_t wait_ns = 0, bool stall = false, const cudaEvent_t *marks = nullptr,
+                              uint32_t *launches = nullptr);
 // (marks, when given: 4 events recorded before the encoding, before and after the tensor-core
-// passes, and after the grid scatter)
+// passes, and after the grid scatter; launches: the kernels launched)
 
 // ---- learned tree cut (k_tree_cut.cu) ----
 // Copies the records of the late-listed rays from src (device) to dst (page-locked host).
