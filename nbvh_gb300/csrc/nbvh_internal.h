@@ -31,6 +31,7 @@ inline void require(bool cond, nbvh_status s, const char *msg)
 inline void cuda_check(cudaError_t e, const char *what)
 {
     if (e != cudaSuccess) {
+        cudaGetLastError(); // this call reports it; the next launch's check must not
         if (e == cudaErrorMemoryAllocation)
             fail(NBVH_ENOMEM, std::string(what) + ": " + cudaGetErrorString(e));
         if (e == cudaErrorTimeout)

@@ -95,3 +95,17 @@ def test_every_failing_allocation_of_a_scene(built):
             if not any(status):
                 break
     assert not any(status) and failures >= 20
+
+
+def test_error_is_reported_once(built):
+    """A call that fails in the CUDA runtime (no query was timed yet) leaves nothing for the next one's check of
+    its launches."""
+    h, s = handle(kind="sphere4k", seed=1)
+    rays = torch.from_numpy(scenes.uniform_rays(SMALL, s["bbox"][:3], s["bbox"][3:], seed=2)).cuda()
+    with h:
+        with pytest.raises(nb.NBVHError) as e:
+            h.last_kernel_time()
+        assert e.value.status == abi.NBVH_EDEVICE
+        first = h.query_closest_neural(rays)
+        assert torch.equal(h.query_closest_neural(rays), first)
+        assert h.last_kernel_time()[0] > 0.0
