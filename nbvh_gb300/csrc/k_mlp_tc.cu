@@ -304,6 +304,8 @@ __global__ void __launch_bounds__(kMaxGroups * kGroupThreads, 1) k_mlp_tc(const 
     }
     if (!ok) {
         // a wait ran out: record it, give copies and MMAs still in flight one more bounded wait
+        if (tid == 0u)
+            tc::mbar_wait(bar_w, 0u);
         if (issuer) {
             atomicOr(a.status, 1u);
             if (load_pending)

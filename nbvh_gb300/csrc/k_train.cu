@@ -848,6 +848,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
     if (!ok) {
         // a wait ran out: record it, give copies and MMAs still in flight one more bounded wait
         tc::copy_async_wait();
+        if (issuer)
+            tc::mbar_wait(bar_w, 0u);
         for (uint32_t i = threadIdx.x; i < a.n_network; i += kTcThreads) // no gradient of this CTA
             a.wpart[(size_t)blockIdx.x * a.n_network + i] = 0.f;
         if (mma_warp && tc::elect_one()) {
