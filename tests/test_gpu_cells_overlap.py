@@ -16,17 +16,50 @@ from nbvh_gb300 import scenes
 pytestmark = pytest.mark.gpu
 
 
-def test_copy_built_during_training_is_dropped(built):
+def _model(n):
     cfg = nb.default_config(batch_size=1 << 16, **{"hashgrid.log2_hashmap_size": 15})
     h, s = handle(cfg, kind="sphere4k", seed=1)
-    n = 1 << 20
-    rays = torch.from_numpy(scenes.uniform_rays(n, s["bbox"][:3], s["bbox"][3:], seed=2)).cuda()
+    rng = np.random.default_rng(7)
+    p = h.params()
+    nn = h.layout.n_network_params
+    p[nn:] = rng.uniform(-0.5, 0.5, p.size - nn).astype(np.float32)
+    h.set_params(p)
+    return h, s, torch.from_numpy(scenes.uniform_rays(n, s["bbox"][:3], s["bbox"][3:], seed=2)).cuda()
+
+
+def test_copy_waits_for_an_adam_step_on_another_stream(built):
+    """The step is still behind other work on its stream when a query of 2^21 rays on this one finds the copy
+    due: the build waits for it, and so does the query after the build."""
+    h, s, rays = _model(1 << 21)
     with h:
-        rng = np.random.default_rng(7)
-        p = h.params()
-        nn = h.layout.n_network_params
-        p[nn:] = rng.uniform(-0.5, 0.5, p.size - nn).astype(np.float32)
-        h.set_params(p)
+        g = torch.rand(h.layout.n_params, device="cuda", generator=torch.Generator("cuda").manual_seed(3)) - 0.5
+        a = torch.rand((4096, 4096), device="cuda")
+        b = a @ a
+        before = h.query_closest_neural(rays)
+        other = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            for _ in range(40):
+                torch.mm(a, a, out=b)
+        h.adam_step(g, other)
+        pending = not other.query()
+        got = h.query_closest_neural(rays)
+        assert pending
+        torch.cuda.synchronize()
+        with nb.NBVH(h.cfg) as f:
+            f.set_mesh(s["v"], s["f"])
+            f.build_classic()
+            f.build_neural_cut()
+            f.set_params(h.params())
+            f.set_cell_copy(0)
+            ref = f.query_closest_neural(rays)
+        assert torch.equal(got, ref) and not torch.equal(got, before)
+
+
+def test_copy_built_during_training_is_dropped(built):
+    n = 1 << 20
+    h, s, rays = _model(n)
+    with h:
         scene = nb.Scene()
         scene.add_instance(h)
         scene.query_closest(rays[:1024])  # the scene's buffers
