@@ -587,8 +587,9 @@ def run_ours(args):
                                     "gathers + 256 B feature row + 52 B list state) x %d segments per launch"
                                     % (ENCODE_BYTES_PER_SEGMENT,
                                        sum(p.encoded_segments for p in enc_prof) // max(1, enc_launches)),
-                     "note": "the 24 MB table is L2-resident: the gathers are served by L2 (DRAM traffic is "
-                             "below the algorithmic bytes); the kernel is bound by the L1 miss path"},
+                     "note": "8 of 16 levels are read from the 192 MB cell copy, the others from the 24 MB table; "
+                             "both against an L2 of 129 MB: DRAM traffic is a fifth of the algorithmic bytes; the "
+                             "kernel is bound by the L1 (data pipe and request path to L2)"},
         "e2e": {"value": world * N_RAYS / (e2e_ms * 1e-3) / 1e6, "unit": "Mrays/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": N_RAYS * 32, "d2h_bytes_per_step": N_RAYS * 48},
         "gpu_launches": args.steps * (neural_launches + classic_launches),
@@ -1048,8 +1049,9 @@ def run_train_roofline(nb, scenes, peaks, steps=50, warmup=5):
                            "algorithmic": "3 x 43,008 FLOP per row (forward, data and weight gradients)"},
                 "adam": {"kernel": "k_adam", "bound": "hbm", "achieved": adam_gbs, "peak": hbm, "unit": "GB/s",
                          "frac": adam_gbs / hbm, "algorithmic": "30 B per parameter x %d parameters" % L.n_params},
-                "grid_scatter": {"atomics_per_s": gathers / (p.train_scatter_ms * 1e-3),
-                                 "algorithmic": "one 8-byte vector atomic per (row, point, level, corner)"}}
+                "grid_scatter": {"corners_per_s": gathers / (p.train_scatter_ms * 1e-3),
+                                 "algorithmic": "(row, point, level, corner) contributions; the kernel merges those "
+                                                "of a row that meet in a cell before its atomics"}}
     finally:
         h.close()
 

@@ -39,10 +39,18 @@ constexpr uint32_t kFirstThreads = 256;
 constexpr uint32_t kSortThreads = 1024;
 // Lists shorter than kSortMinRows are walked in list order: the sort would cost more than the locality it buys.
 // Batches below kSortMinRays have no list sorted: besides the sorts' launches, which every step has whatever its
-// list, the first pass and the decode then count no rows per bin. us per call with lists sorted from 2^16 rows on /
-// not at all: 131,072 uniform rays 333 / 317, 262,144 459 / 432, a 512 x 512 frame 580 / 545, a 960 x 540 path
-// 1,864 / 1,785, 524,288 uniform rays 654 / 650. Larger batches gain from it: 2^20 rays 947 sorted, 963 with lists
-// below 2^19 left as they are; of 2^16, 2^17 and 2^18 none is better for them (2^22 rays 2,622, 2,613, 2,616).
+// list, the first pass and the decode then count no rows per bin. us per call with lists sorted from 2^17 rows on /
+// not at all, with the encoder's cell copy and without it (u: uniform rays, s: rays that start on the surface,
+// which list almost every row; r: the reference's 3 points x 8 levels, without octant bins):
+//   copy     u 262,144  452 / 431   u 393,216  529 / 507   u 524,287  628 / 607   u 2^20  940 / 925   u 2^22  2,563 / 2,680
+//            s 262,144  579 / 580   s 393,216  743 / 755   s 524,287  920 / 945   s 2^20  1,558 / 1,654
+//   none     u 262,144  475 / 455   u 393,216  567 / 546   u 524,287  666 / 661   u 2^20  1,006 / 1,018   u 2^22  2,789 / 3,039
+//            s 262,144  629 / 654   s 393,216  811 / 859   s 524,287  1,001 / 1,088   s 2^20  1,723 / 1,888
+//   none, r  u 262,144  276 / 257   u 393,216  325 / 308   u 524,287  381 / 365   s 393,216  524 / 531   s 524,287  627 / 653
+//   frames and paths, none: 512 x 512 608 / 588, 720 x 720 867 / 834, 960 x 540 path 1,920 / 1,871
+// Without the copy surface rays would gain from sorting already at 200,000 (4 to 8% at 262,144 to 524,287) and
+// uniform rays, frames and paths lose 1 to 7% up to the line: neither state has a better one for all. Lists of 2^16
+// or 2^15 rows and more sorted: within 1% of 2^17.
 constexpr uint32_t kSortMinRays = 1u << 19;
 constexpr uint32_t kSortMinRows = 1u << 17;
 // Rows with at least this many (point, level) pairs to encode are sorted by octant within a leaf.
@@ -604,8 +612,9 @@ __global__ void __launch_bounds__(kFirstThreads, 4) k_wave_first(const __grid_co
 // negative mint, then encoded into the dilated scene box. The point is computed once for all its
 // levels, so the kernel's instructions go to the gathers and their interpolation; it holds no
 // MLP state; its 4 blocks of 256 threads per SM keep many gathers in flight to hide their latency.
-// The L1 bounds it: it looks up one cache line per cycle, and a (point, level) of the table costs 6
-// lookups (4 pairs of x corners, half of them split). Levels in the cell copy cost one 32-byte read:
+// The L1 bounds it (ncu, 329,000 segments: its data pipe 73%, its request path to L2 69%, L2 57%, DRAM 10%,
+// issue 43%): a (point, level) of the table costs 4 gathers of x corner pairs, half of them split into two, and no
+// two lanes of a warp share a sector on the fine levels. Levels in the cell copy cost one 32-byte read:
 // 1,453 -> 1,250 us per 2^22-ray query with the copy of the 8 coarsest levels (192 MB; dense levels
 // alone, 11 MB: 1,390; 9 levels, 520 MB: no more), 489 -> 455 for 2^20 rays with 5 of the reference's 8
 // levels. Reading the quad of entries where both corners lie in it was slower (1,435 us: the warp then

@@ -361,7 +361,7 @@ __device__ __forceinline__ void composite_loss(const LossConsts &lc, uint32_t ch
 // features (LPS levels) per 16-byte store (K3 forward). `split`: the point's levels are spread over
 // L / LPS threads instead, one store each; batches too small to fill the GPU otherwise are bound by
 // the latency of one thread's gathers, level after level (3,001 rows: 37 -> 15 us). Large batches are
-// bound by the L1's misses to L2 (ncu: L1 88%, L2 68%); 4-byte stores, sixteen partial sectors a
+// bound by the L1 (ncu, in place order: its data pipe 70%, its request path to L2 65%, L2 53%); 4-byte stores, sixteen partial sectors a
 // point, were the rest of 289 us per 2^18 rows, 222 now; large training batches come in an order that
 // brings neighbours together (kRowOrderMin).
 // ---------------------------------------------------------------------------------------------
@@ -898,8 +898,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_train_tc(const __grid_constan
 // the odd lane the upper ones, and go through the row's points; points in the same cell are summed
 // in registers and leave as one set of atomics.
 //
-// The L2 bounds this kernel: it takes about 2e11 32-byte sectors of atomics a second, whatever part
-// of the sector they touch. The points of a row lie on a short segment, so on the coarser levels most
+// The L2 bounds this kernel: it takes 2e11 32-byte sectors of atomics a second, whatever part of the sector they
+// touch (ncu, 2^18 rows at the start of training: 6.72e7 sectors in 327 us, its busiest slice 90% of the time). The points of a row lie on a short segment, so on the coarser levels most
 // share a cell (45 sets of corners instead of 64 for the 64 (point, level) pairs of a row). And the
 // entries of x and x + 1 lie in one sector 3 times in 4 (2 features; tcnn's hash multiplies x by 1), so
 // the two lanes' atomics of one instruction merge into one. Warps are 16 rows of one level: the
