@@ -370,7 +370,7 @@ struct nbvh_handle {
     uint64_t cells_rays = 0;  // rays queried without it since the parameters changed
     bool cells_off = false;   // never again: Adam steps captured into a graph change the parameters unseen
     cudaEvent_t ev_params = nullptr; // after the last nbvh_adam_step, on its stream
-    std::mutex cells_mu;      // guards the six above (cells_fresh is also read without it)
+    std::mutex cells_mu;      // guards the copy and its state (queries read cells_fresh and the plan without it)
     uint32_t *h_readback = nullptr; // two page-locked words a call reads its status and loss back into
     nbvh::DeviceBuffer<float> d_adam_m, d_adam_v;
     nbvh::DeviceBuffer<float> d_grad;
@@ -598,8 +598,8 @@ cudaError_t launch_encode_rows(const __half *params_h, const GridParams &grid, u
 // Cell copy of the coarse levels of a hash grid: for every cell of such a level the entries of its 8
 // corners side by side (corner c at c * F halves), so that a point's lookup on the level is one 16F-byte
 // read instead of 8 entries in 4 to 8 sectors. plan_cells picks the levels (as many of the coarsest as
-// max_bytes, at most kCellBytes, holds) and returns the number of cells; launch_build_cells fills the copy from the
-// 16-bit parameters.
+// max_bytes, at most kCellBytes, holds; none where the encoder reads the table alone) and returns the number
+// of cells; launch_build_cells fills the copy from the 16-bit parameters.
 size_t plan_cells(const GridParams &grid, CellParams &cp, size_t max_bytes);
 cudaError_t launch_build_cells(const __half *params_h, const GridParams &grid, const CellParams &cp,
                                uint32_t n_hidden_layers, uint4 *cells, cudaStream_t s);

@@ -192,7 +192,8 @@ StepResources tuning_of(const Model &m, uint32_t bucket)
 }
 
 // Captures (once) the graph of a padded batch of `bucket` rays in the slot's buffers: the whole query,
-// ending with a copy of the wave counters to the host. Nothing runs; the kernels' attributes are set beforehand (a captured launch cannot set them). A shape
+// ending with a copy of the wave counters to the host. Nothing runs; the kernels' attributes are set
+// beforehand (a captured launch cannot set them). A shape
 // whose capture fails is recorded without a graph and keeps running directly.
 cudaGraphExec_t ensure_graph(nbvh_server *srv, Slot &sl, uint32_t model_id, uint32_t bucket, uint32_t depth,
                              bool cells)
